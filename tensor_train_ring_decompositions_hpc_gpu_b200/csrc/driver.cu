@@ -11,6 +11,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <cmath>
 #include <string>
 #include <vector>
 
@@ -980,8 +981,7 @@ int run_chain(tt_ctx* c, const float* x_in, Plan P, const tt_opts& o, float* con
         TT_TRY(pass.run(TT_PASS_SKETCH, fl_pass, by_pass, [&] {
           return launch_sketch(cur, m, cols, B.omega, ksa, 1, cols, B.yd, engine, ws, c->dstat, s);
         }));
-        TT_TRY(launch_f64_to_f32_cols(B.yd, m, m, ksa, B.yf, m, ksa, s));
-        TT_TRY(launch_cholqr2(B.yf, m, ksa, 1, m, nullptr, ws, c->dstat, s));
+        TT_TRY(launch_cholqr2(B.yd, B.yf, m, ksa, m, nullptr, ws, s));
         for (int it = 0; it < pwa; ++it) {
           // Z = A^T Q written column-major (cols x ksa), the layout the sketch reads W in
           TT_TRY(pass.run(TT_PASS_PROJECT, fl_pass, by_pass, [&] {
@@ -991,13 +991,12 @@ int run_chain(tt_ctx* c, const float* x_in, Plan P, const tt_opts& o, float* con
           // Adaptive ranks need the basis beyond the FP32 Gram's resolution (graded spectra
           // down to delta / ||A|| ~ 1e-4): the pass forms its Gram with FP64 products there.
           TT_TRY(pass.run(TT_PASS_OTHER, 4.0 * cols * ksa * ksa, 12.0 * cols * ksa, [&] {
-            return launch_orth_power(B.bt, cols, ksa, 1, cols, ws, c->dstat, s, adaptive);
+            return launch_orth_power(B.bt, cols, ksa, cols, ws, s, adaptive);
           }));
           TT_TRY(pass.run(TT_PASS_SKETCH, fl_pass, by_pass, [&] {
             return launch_sketch(cur, m, cols, B.bt, ksa, 1, cols, B.yd, engine, ws, c->dstat, s);
           }));
-          TT_TRY(launch_f64_to_f32_cols(B.yd, m, m, ksa, B.yf, m, ksa, s));
-          TT_TRY(launch_cholqr2(B.yf, m, ksa, 1, m, nullptr, ws, c->dstat, s));
+          TT_TRY(launch_cholqr2(B.yd, B.yf, m, ksa, m, nullptr, ws, s));
         }
         // B^T = A^T Q (cols x ksa, row-major) = B (ksa x cols, column-major).  Adaptive ranks
         // take ||B||^2 as the captured energy, which must hold ~1e-8 relative.  Tensor-core
@@ -1340,39 +1339,75 @@ extern "C" int tt_rel_error(tt_ctx* c, const float* x, int d, const int* n, cons
     return TT_ERR_SHAPE;
   }
   TT_CUDA(cudaSetDevice(c->device));
-  long long N = 1;
-  for (int k = 1; k < d; ++k) N *= n[k];
-  // merged right part M_k sizes: r_{k-1} * (n_k ... n_d) * r_d
-  // M_k (cores k..d-1 merged) holds r[k] * n[k] * ... * n[d-1] * r[d] floats.
-  long long maxm = 0;
-  {
-    long long rest = r[d];
-    for (int k = d - 1; k >= 1; --k) {
-      rest *= n[k];
-      maxm = std::max(maxm, (long long)r[k] * rest);
+  const long long rr0 = ring ? r[0] : 1;
+  if (((double)rr0 * n[0] * r[1] + 32.0 * rr0 * r[1]) * sizeof(float) > 200.0 * 1024) {
+    set_error(TT_ERR_UNSUPPORTED, "reconstruction check: first core too large");
+    return TT_ERR_UNSUPPORTED;
+  }
+  // Left part of a split after core k (k cores): (r0, P_k, r_k); right part: (r_k, N_k, r_d).  Any
+  // split gives the same product; its cost is the final contraction (2 |X| r0 r_k, in tiles of 128
+  // x 128) plus the merges of both sides, least where both sides are small.  Scratch: two buffers
+  // a side, at most what merging everything right of core 1 takes.
+  std::vector<double> P((size_t)d + 1, 1.0);
+  for (int k = 0; k < d; ++k) P[(size_t)k + 1] = P[(size_t)k] * n[k];
+  const double most = [&] {
+    double m = 0.0;
+    for (int k = d - 1; k >= 1; --k) m = std::max(m, (double)r[k] * (P[(size_t)d] / P[(size_t)k]) * r[d]);
+    return m;
+  }();
+  int cut = 1;
+  double best = -1.0;
+  for (int k = 1; k < d; ++k) {
+    const double Nk = P[(size_t)d] / P[(size_t)k];
+    const double tiles = std::ceil(P[(size_t)k] / 128.0) * std::ceil(Nk / 128.0);
+    double cost = tiles * 16384.0 * rr0 * r[k], lmax = 0.0, rmax = 0.0;
+    for (int j = 2; j <= k; ++j) {
+      cost += (double)rr0 * P[(size_t)j] * r[j - 1] * r[j];
+      lmax = std::max(lmax, (double)rr0 * P[(size_t)j] * r[j]);
+    }
+    for (int j = d - 2; j >= k; --j) {
+      const double out = (double)r[j] * (P[(size_t)d] / P[(size_t)j]) * r[d];
+      cost += out * r[j + 1];
+      rmax = std::max(rmax, out);
+    }
+    if (k > 1 && lmax + rmax > most) continue;
+    if (best < 0.0 || cost < best) {
+      best = cost;
+      cut = k;
     }
   }
-  TT_TRY(tt_ctx_reserve(c, sizeof(float) * (size_t)maxm * 2 + 4096 + (1 << 20)));
+  auto left_elems = [&](int k) { return (size_t)rr0 * (size_t)P[(size_t)k] * (size_t)r[k]; };
+  auto right_elems = [&](int k) { return (size_t)r[k] * (size_t)(P[(size_t)d] / P[(size_t)k]) * (size_t)r[d]; };
+  size_t lmax = 1, rmax = 1;
+  for (int k = 2; k <= cut; ++k) lmax = std::max(lmax, left_elems(k));
+  for (int k = d - 2; k >= cut; --k) rmax = std::max(rmax, right_elems(k));
+  TT_TRY(tt_ctx_reserve(c, sizeof(float) * 2 * (lmax + rmax) + 4096 + (1 << 20)));
   Arena a{c->arena, c->cap, 0};
-  float* buf[2] = {a.take<float>(maxm), a.take<float>(maxm)};
+  float* lbuf[2] = {a.take<float>(lmax), a.take<float>(lmax)};
+  float* rbuf[2] = {a.take<float>(rmax), a.take<float>(rmax)};
   double* acc = a.take<double>(2);
-  if (!buf[1] || !acc) {
+  if (!lbuf[1] || !rbuf[1] || !acc) {
     set_error(TT_ERR_NOMEM, "error workspace");
     return TT_ERR_NOMEM;
   }
   cudaStream_t s = c->stream;
-  const float* mk = cores[d - 1];
-  long long cols = (long long)n[d - 1] * r[d];
-  int sl = 0;
-  for (int k = d - 2; k >= 1; --k) {
-    // M_k = G_k (r_{k-1} n_k x r_k) * M_{k+1} (r_k x cols)
-    TT_TRY(launch_gemm_nn(cores[k], (long long)r[k] * n[k], r[k + 1], mk, cols, buf[sl], s));
-    mk = buf[sl];
-    sl ^= 1;
-    cols *= n[k];
+  const float* lf = cores[0];
+  for (int k = 2; k <= cut; ++k) {
+    // (r0, P_k, r_k) = (r0 P_{k-1} x r_{k-1}) * (r_{k-1} x n_{k-1} r_k)
+    TT_TRY(launch_gemm_nn(lf, rr0 * (long long)P[(size_t)k - 1], r[k - 1], cores[k - 1], (long long)n[k - 1] * r[k],
+                          lbuf[k & 1], s));
+    lf = lbuf[k & 1];
+  }
+  const float* rf = cores[d - 1];
+  for (int k = d - 2; k >= cut; --k) {
+    // (r_k, N_k, r_d) = (r_k n_k x r_{k+1}) * (r_{k+1} x N_{k+1} r_d)
+    TT_TRY(launch_gemm_nn(cores[k], (long long)r[k] * n[k], r[k + 1], rf,
+                          (long long)(P[(size_t)d] / P[(size_t)k + 1]) * r[d], rbuf[k & 1], s));
+    rf = rbuf[k & 1];
   }
   TT_CUDA(cudaMemsetAsync(acc, 0, 2 * sizeof(double), s));
-  TT_TRY(launch_recon_err(x, n[0], N, cores[0], ring ? r[0] : 1, r[1], mk, acc, s));
+  TT_TRY(launch_recon_err(x, (long long)P[(size_t)cut], (long long)(P[(size_t)d] / P[(size_t)cut]), lf, rf, (int)rr0,
+                          r[cut], acc, s));
   double h[2] = {0, 0};
   TT_CUDA(cudaMemcpyAsync(h, acc, sizeof(h), cudaMemcpyDeviceToHost, s));
   TT_CUDA(cudaStreamSynchronize(s));
@@ -1659,7 +1694,7 @@ extern "C" int tt_k_cholqr2(tt_ctx* c, float* y, long long n, int N, long long l
   Arena ws;
   TT_TRY(ws_for(c, gram_ws_bytes(n, N) + 8 * TT_MAX_SMALL * TT_MAX_SMALL * sizeof(double), ws));
   TT_CUDA(cudaMemsetAsync(c->dstat, 0, sizeof(DevStatus), c->stream));
-  TT_TRY(launch_cholqr2(y, n, N, 1, ld, r, ws, c->dstat, c->stream));
+  TT_TRY(launch_cholqr2(nullptr, y, n, N, ld, r, ws, c->stream));
   return check_status(c);
 }
 

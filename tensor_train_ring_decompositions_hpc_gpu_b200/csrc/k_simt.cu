@@ -1,5 +1,5 @@
 // CUDA-core kernels: the plain-FP32 GEMM engine and every small linear-algebra kernel of the
-// TT/TR-SVD chain (Gaussian test matrix, Gram matrices, CholeskyQR2, Jacobi eigen-solver,
+// TT/TR-SVD chain (Gaussian test matrix, Gram matrices, Jacobi eigen-solver,
 // bond permute, core folding, reconstruction error).
 #include <float.h>
 #include <stdlib.h>
@@ -103,10 +103,15 @@ int launch_gaussian(float* out, long long rows, int cols, long long ld, unsigned
 // ---------------------------------------------------------------------------------------
 // Plain-FP32 sketch  Y = A * W  (split over the long dimension n, FP64 reduction of splits)
 // ---------------------------------------------------------------------------------------
-// Asynchronous global -> shared copies (cp.async): 16-byte, and 4-byte with zero fill when
+// Asynchronous global -> shared copies (cp.async): 16-byte, and 16- or 4-byte with zero fill when
 // `valid` is false (no byte is read then).
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async16z(void* dst, const void* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(valid ? 16 : 0)
                : "memory");
 }
 __device__ __forceinline__ void cp_async4(void* dst, const void* src, bool valid) {
@@ -1581,623 +1586,7 @@ int launch_gram(const float* x, long long nvec, int M, long long vs, long long e
   return TT_OK;
 }
 
-// ---------------------------------------------------------------------------------------
-// CholeskyQR2: FP64 Cholesky + triangular inverse on chip, FP32 apply
-// ---------------------------------------------------------------------------------------
-// One block: W (N x N, FP64) -> R (upper, FP64) and R^-1 (FP64).  Pivots below
-// rel_tol * max diag mark a dependent column: its row of R and column of R^-1 are zero.
-// Cholesky right-looking with one barrier per column; in the trailing update thread
-// (row group g, column j) loads all its rows before storing any; the pivot's reciprocal square
-// root is the only special function per column.  R^-1 is formed column-parallel with no barrier
-// in between: thread j back-substitutes R x = e_j (x_i = -(sum_{k>i} r_ik x_k) / r_ii), four
-// partial sums per dot product.  On-chip matrices use an odd row stride (N | 1 doubles), so the
-// threads of a warp, each in a different row or column, read distinct banks.
-constexpr int chol_ld(int N) { return N | 1; }
-__global__ void __launch_bounds__(256) k_chol_inv(const double* __restrict__ w, int N,
-                                                  double* __restrict__ r_out,
-                                                  double* __restrict__ rinv, double rel_tol,
-                                                  int ri_smem, DevStatus* st) {
-  extern __shared__ double sm[];
-  const int L = chol_ld(N);
-  double* A = sm;                                // N x L (row-major), upper part becomes R
-  double* Ri = ri_smem ? sm + N * L : rinv;      // R^-1 column-major: stride L on chip, N in memory
-  const int LR = ri_smem ? L : N;
-  int* dead = reinterpret_cast<int*>(sm + (ri_smem ? 2 : 1) * N * L);
-  __shared__ double dinv[128];
-  __shared__ double dmax_s;
-  const int tid = threadIdx.x, NT = blockDim.x;
-  for (int idx = tid; idx < N * N; idx += NT) {
-    const int j = idx / N, i = idx - (idx / N) * N;  // w column-major: coalesced reads
-    A[i * L + j] = w[idx];
-  }
-  __syncthreads();
-  if (tid < 32) {
-    double dm = 0.0;
-    for (int i = tid; i < N; i += 32) dm = fmax(dm, A[i * L + i]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) dm = fmax(dm, __shfl_xor_sync(0xffffffffu, dm, o));
-    if (tid == 0) dmax_s = dm;
-  }
-  __syncthreads();
-  const double dmax = dmax_s, tol = rel_tol * dmax;
-  // column j = k + 1 + (tid % CW), rows from k + 1 + tid / CW in steps of RG
-  const int CW = N <= 32 ? 32 : N <= 64 ? 64 : 128;
-  const int RG = NT / CW;
-  for (int k = 0; k < N; ++k) {
-    const double d = A[k * L + k];
-    const bool live = d > tol && dmax > 0.0;
-    const double rs = live ? rsqrt(d) : 0.0;  // 1 / r_kk
-    if (live) {
-      const double inv = rs * rs;
-      const int j = k + 1 + (tid % CW);
-      if (j < N) {
-        const double wkj = A[k * L + j] * inv;
-        const int i0 = k + 1 + tid / CW;
-        constexpr int U = 8;
-        for (int ib = i0; ib <= j; ib += U * RG) {
-          double wk[U], wij[U];
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            const int i = ib + u * RG;
-            if (i <= j) {
-              wk[u] = A[k * L + i];
-              wij[u] = A[i * L + j];
-            }
-          }
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            const int i = ib + u * RG;
-            if (i <= j) A[i * L + j] = fma(-wk[u], wkj, wij[u]);
-          }
-        }
-      }
-    }
-    __syncthreads();
-    // row k of R: A[k][c] / r_kk for c > k, r_kk = d / sqrt(d) (after the update that read it)
-    for (int c = k + tid; c < N; c += NT) A[k * L + c] = live ? A[k * L + c] * rs : 0.0;
-    if (tid == 0) {
-      dead[k] = live ? 0 : 1;
-      dinv[k] = rs;
-    }
-    __syncthreads();
-  }
-  // R out (column-major), zero below the diagonal; dead rows are zero.
-  if (r_out) {
-    for (int idx = tid; idx < N * N; idx += NT) {
-      const int i = idx % N, j = idx / N;
-      r_out[idx] = (j >= i) ? A[i * L + j] : 0.0;
-    }
-  }
-  // R^-1, column j by thread j: x_j = 1 / r_jj, x_i = -(sum_{k=i+1..j} r_ik x_k) / r_ii.
-  for (int j = tid; j < N; j += NT) {
-    double* x = Ri + (long long)LR * j;
-    for (int i = j + 1; i < N; ++i) x[i] = 0.0;
-    if (dead[j]) {
-      for (int i = 0; i <= j; ++i) x[i] = 0.0;
-      continue;
-    }
-    x[j] = dinv[j];
-    for (int i = j - 1; i >= 0; --i) {
-      const double* ar = A + i * L;
-      double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-      int kk = i + 1;
-      for (; kk + 3 <= j; kk += 4) {
-        s0 = fma(ar[kk], x[kk], s0);
-        s1 = fma(ar[kk + 1], x[kk + 1], s1);
-        s2 = fma(ar[kk + 2], x[kk + 2], s2);
-        s3 = fma(ar[kk + 3], x[kk + 3], s3);
-      }
-      for (; kk <= j; ++kk) s0 = fma(ar[kk], x[kk], s0);
-      x[i] = -((s0 + s1) + (s2 + s3)) * dinv[i];
-    }
-  }
-  if (ri_smem) {
-    __syncthreads();
-    for (int idx = tid; idx < N * N; idx += NT) {
-      const int i = idx % N, j = idx / N;
-      rinv[idx] = Ri[i + L * j];
-    }
-  }
-  (void)st;
-}
-
-// Y (n x N) <- Y * T, T = R^-1 upper (FP64 in global, staged as FP32 once per block).  Blocks
-// loop over tiles of 128 rows, one row per thread, outputs produced 32 columns at a time and
-// written over the tile in shared memory.
-template <int NP>
-__global__ void __launch_bounds__(128) k_apply_rinv(float* __restrict__ y, long long n, int N,
-                                                    long long vs, long long es,
-                                                    const double* __restrict__ t) {
-  extern __shared__ float sm_apply[];
-  float* ts = sm_apply;                 // NP x NP, ts[k*NP + c]
-  float* ys = ts + NP * NP;             // 128 x (NP+1): the tile, overwritten by the result
-  constexpr int LD = NP + 1;
-  const int tid = threadIdx.x;
-  for (int idx = tid; idx < NP * NP; idx += 128) {
-    const int k = idx % NP, c = idx / NP;
-    ts[k * NP + c] = (k < N && c < N) ? (float)t[k + (long long)N * c] : 0.f;
-  }
-  // Output chunk width divides NP (NP is a multiple of 16), so cb + c < NP always.
-  constexpr int CB = (NP % 32 == 0) ? 32 : 16;
-  static_assert(NP % CB == 0, "chunk width must divide the padded width");
-  const long long ntile = (n + 127) / 128;
-  // column-major rows read / written as 16-byte runs of 4 rows
-  const bool v4 = vs == 1 && es != 1 && (es & 3) == 0 && ((reinterpret_cast<uintptr_t>(y) & 15) == 0);
-  for (long long tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
-    const long long j0 = tile * 128;
-    __syncthreads();  // ts ready / the previous tile's stores done
-    if (es == 1) {
-      for (int f = tid; f < 128 * NP; f += 128) {
-        const int c = f % NP, r = f / NP;
-        const long long j = j0 + r;
-        ys[r * LD + c] = (j < n && c < N) ? y[j * vs + c] : 0.f;
-      }
-    } else if (v4) {
-      // 4 consecutive rows of a column per 16-byte load; a warp covers 8 row groups x 4 columns
-      for (int f = tid; f < 32 * NP; f += 128) {
-        const int r4 = (f & 7) + 8 * ((f >> 5) & 3), c = ((f >> 3) & 3) + 4 * (f >> 7);
-        const long long j = j0 + 4 * r4;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (c < N) {
-          if (j + 3 < n) {
-            v = *reinterpret_cast<const float4*>(y + j + (long long)c * es);
-          } else {
-            const float* src = y + (long long)c * es;
-            if (j < n) v.x = src[j];
-            if (j + 1 < n) v.y = src[j + 1];
-            if (j + 2 < n) v.z = src[j + 2];
-          }
-        }
-        ys[(4 * r4) * LD + c] = v.x;
-        ys[(4 * r4 + 1) * LD + c] = v.y;
-        ys[(4 * r4 + 2) * LD + c] = v.z;
-        ys[(4 * r4 + 3) * LD + c] = v.w;
-      }
-    } else {
-      for (int f = tid; f < 128 * NP; f += 128) {
-        const int r = f % 128, c = f / 128;
-        const long long j = j0 + r;
-        ys[r * LD + c] = (j < n && c < N) ? y[j * vs + (long long)c * es] : 0.f;
-      }
-    }
-    __syncthreads();
-    // Row tid in place: T is upper triangular, so output columns cb.. need inputs k < cb + CB
-    // only; chunks run from the last one down and overwrite inputs no later chunk reads.
-    for (int cb = NP - CB; cb >= 0; cb -= CB) {
-      float outv[CB];
-#pragma unroll
-      for (int c = 0; c < CB; ++c) outv[c] = 0.f;
-      for (int k = 0; k < cb + CB; ++k) {
-        const float yk = ys[tid * LD + k];
-#pragma unroll
-        for (int c = 0; c < CB; ++c) outv[c] = fmaf(yk, ts[k * NP + cb + c], outv[c]);
-      }
-#pragma unroll
-      for (int c = 0; c < CB; ++c) ys[tid * LD + cb + c] = outv[c];
-    }
-    __syncthreads();
-    if (es == 1) {
-      for (int f = tid; f < 128 * NP; f += 128) {
-        const int c = f % NP, r = f / NP;
-        const long long j = j0 + r;
-        if (j < n && c < N) y[j * vs + c] = ys[r * LD + c];
-      }
-    } else if (v4) {
-      for (int f = tid; f < 32 * NP; f += 128) {
-        const int r4 = (f & 7) + 8 * ((f >> 5) & 3), c = ((f >> 3) & 3) + 4 * (f >> 7);
-        const long long j = j0 + 4 * r4;
-        if (c >= N || j >= n) continue;
-        const float4 v = make_float4(ys[(4 * r4) * LD + c], ys[(4 * r4 + 1) * LD + c], ys[(4 * r4 + 2) * LD + c],
-                                     ys[(4 * r4 + 3) * LD + c]);
-        float* dst = y + (long long)c * es;
-        if (j + 3 < n) {
-          *reinterpret_cast<float4*>(dst + j) = v;
-        } else {
-          dst[j] = v.x;
-          if (j + 1 < n) dst[j + 1] = v.y;
-          if (j + 2 < n) dst[j + 2] = v.z;
-        }
-      }
-    } else {
-      for (int f = tid; f < 128 * NP; f += 128) {
-        const int r = f % 128, c = f / 128;
-        const long long j = j0 + r;
-        if (j < n && c < N) y[j * vs + (long long)c * es] = ys[r * LD + c];
-      }
-    }
-  }
-}
-
-// R = R2 * R1 (upper triangular, FP64).
-__global__ void k_mul_upper(const double* __restrict__ r2, const double* __restrict__ r1, int N,
-                            double* __restrict__ r) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= N * N) return;
-  const int i = idx % N, j = idx / N;
-  double acc = 0.0;
-  for (int k = i; k <= j; ++k) acc += r2[i + (long long)N * k] * r1[k + (long long)N * j];
-  r[idx] = (j >= i) ? acc : 0.0;
-}
-
-// Cluster helpers: rank in the cluster, cluster size, cluster-wide barrier (release / acquire),
-// and an FP64 load from the same shared-memory offset in another CTA of the cluster.
-__device__ __forceinline__ unsigned cl_rank() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ unsigned cl_size() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cl_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ double ld_peer_f64(const double* p, unsigned rank) {
-  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
-  unsigned ra;
-  double v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
-  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(ra) : "memory");
-  return v;
-}
-
-// CholeskyQR2 of an n x N sketch (N <= 64) in one launch: a cluster of up to 8 CTAs, each
-// holding `rpc` consecutive rows in shared memory (64 < N <= 80: one CTA of 256 threads, the
-// Gram summed straight into W, no R output).  Y is staged row-major with a padded
-// stride S (S/4 odd, so the float4 row accesses of neighbouring threads fall in distinct
-// banks); per pass:
-//   each CTA's partial Gram Y_c^T Y_c in FP64 (4x4 register tiles over the upper tile
-//   triangle, row groups reduced through shared memory), summed over the cluster through
-//   distributed shared memory in rank order (every CTA gets the same bits, so the redundant
-//   factorisations agree), right-looking Cholesky in FP64 (one barrier per column, dead
-//   pivots below rel_tol * max diag), then Q = Y R^-1 by forward substitution, one row per
-//   thread in FP32 registers against an FP32 copy of R (column-major, diagonal stored as
-//   1/r_cc).
-// Optional R output (column-major) = R2 * R1, written by rank 0.  Each pass has its own partial
-// buffer, so a CTA that runs ahead never overwrites a partial a peer is still reading; the
-// final cluster barrier keeps every CTA's shared memory alive until the peers are done.
-template <int NP>
-__global__ void __launch_bounds__(NP > 64 ? 256 : 512) k_cholqr2_small(float* __restrict__ y, int n, int N,
-                                                                      long long vs, long long es, int S,
-                                                                      int rpc, double* __restrict__ r,
-                                                                      double rel_tol) {
-  constexpr int NT = NP > 64 ? 256 : 512;  // the wide rows of the substitution need the registers
-  extern __shared__ __align__(16) unsigned char sm_cq[];
-  const unsigned crank = cl_rank(), csize = cl_size();
-  const int row0 = (int)crank * rpc;
-  const int nl = max(0, min(rpc, n - row0));                         // rows of this CTA
-  const int WN = (N * N + 1) & ~1;
-  float* Ys = reinterpret_cast<float*>(sm_cq);                       // rpc x S
-  double* Wp = reinterpret_cast<double*>(Ys + (size_t)rpc * S);      // 2 x N x N partials
-  double* W = NP > 64 ? Wp : Wp + 2 * WN;                            // N x N row-major
-  float* Rf = reinterpret_cast<float*>(W + WN);                      // NP x NP, Rf[c*NP+k] = R[k][c]
-  float* invd = Rf + NP * NP;                                        // NP
-  double* R1 = reinterpret_cast<double*>(invd + NP);                 // N x N (only with r)
-  const int tid = threadIdx.x;
-  const int TTa = (N + 3) >> 2;
-  const int ngrp = S >> 2;
-  for (int f = tid; f < nl * ngrp; f += NT) {
-    const int i = f % nl, q4 = f / nl;
-    const long long gi = row0 + i;
-    float v[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int c = 4 * q4 + e;
-      v[e] = (c < N) ? y[gi * vs + (long long)c * es] : 0.f;
-    }
-    *reinterpret_cast<float4*>(&Ys[(size_t)i * S + 4 * q4]) = make_float4(v[0], v[1], v[2], v[3]);
-  }
-  // Tile assignment for the Gram: tile t of the TTa x TTa upper triangle, row group g.
-  const int nt = TTa * (TTa + 1) / 2;
-  const int groups = min(32, max(1, NT / nt));
-  const int t = tid % nt, g = tid / nt;
-  const bool act = g < groups;
-  int ta = 0, rem = act ? t : 0;
-  while (rem >= TTa - ta) {
-    rem -= TTa - ta;
-    ++ta;
-  }
-  const int tb = ta + rem;
-  for (int pass = 0; pass < 2; ++pass) {
-    double* Wq = NP > 64 ? W : Wp + pass * WN;
-    __syncthreads();
-    double acc[16];
-#pragma unroll
-    for (int e = 0; e < 16; ++e) acc[e] = 0.0;
-    if (act) {
-      for (int v = g; v < nl; v += groups) {
-        const float4 xa = *reinterpret_cast<const float4*>(&Ys[(size_t)v * S + 4 * ta]);
-        const float4 xb = *reinterpret_cast<const float4*>(&Ys[(size_t)v * S + 4 * tb]);
-        const double av[4] = {xa.x, xa.y, xa.z, xa.w};
-        const double bv[4] = {xb.x, xb.y, xb.z, xb.w};
-#pragma unroll
-        for (int p = 0; p < 4; ++p)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) acc[p * 4 + q] = fma(av[p], bv[q], acc[p * 4 + q]);
-      }
-    }
-    for (int gg = 0; gg < groups; ++gg) {
-      if (act && g == gg) {
-#pragma unroll
-        for (int p = 0; p < 4; ++p)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int i = 4 * ta + p, j = 4 * tb + q;
-            if (i < N && j < N) Wq[i * N + j] = (gg == 0 ? 0.0 : Wq[i * N + j]) + acc[p * 4 + q];
-          }
-      }
-      __syncthreads();
-    }
-    // Sum the partials over the cluster (upper triangle), in rank order.
-    cl_sync();
-    for (int idx = tid; idx < N * N; idx += NT) {
-      const int i = idx / N, j = idx - (idx / N) * N;
-      if (i > j) continue;
-      double a = Wq[idx];
-      if (csize > 1) {
-        a = 0.0;
-        for (unsigned q = 0; q < csize; ++q) a += ld_peer_f64(Wq + idx, q);
-      }
-      W[idx] = a;
-    }
-    __syncthreads();
-    double dmax = 0.0;
-    for (int k = 0; k < N; ++k) dmax = fmax(dmax, W[k * N + k]);
-    const double tol = rel_tol * dmax;
-    __syncthreads();  // every thread has read the diagonal before the first update changes it
-    for (int k = 0; k < N; ++k) {
-      const double d = W[k * N + k];
-      if (d > tol && dmax > 0.0) {
-        // trailing update of the upper triangle: thread (row group tid / CW, column tid % CW);
-        // a thread's rows in chunks of 8, each chunk loaded before any of it is stored
-        constexpr int CW = NP > 64 ? 128 : 64, RG = NT / CW;
-        const double inv = 1.0 / d;
-        const int j = k + 1 + (tid % CW);
-        if (j < N) {
-          const double wkj = W[k * N + j] * inv;
-          for (int i0 = k + 1 + tid / CW; i0 <= j; i0 += 8 * RG) {
-            double wk[8], wij[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-              const int i = i0 + RG * u;
-              if (i <= j) {
-                wk[u] = W[k * N + i];
-                wij[u] = W[i * N + j];
-              }
-            }
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-              const int i = i0 + RG * u;
-              if (i <= j) W[i * N + j] = fma(-wk[u], wkj, wij[u]);
-            }
-          }
-        }
-      }
-      __syncthreads();
-    }
-    // R[k][c] = W[k][c] / sqrt(W[k][k]) on live rows (c >= k); dead rows are zero.
-    for (int idx = tid; idx < NP * NP; idx += NT) {
-      const int c = idx / NP, k = idx % NP;
-      float v = 0.f;
-      if (c < N && k < c) {
-        const double d = W[k * N + k];
-        if (d > tol && dmax > 0.0) v = (float)(W[k * N + c] / sqrt(d));
-      }
-      Rf[idx] = v;
-    }
-    for (int c = tid; c < NP; c += NT) {
-      float v = 0.f;
-      if (c < N) {
-        const double d = W[c * N + c];
-        if (d > tol && dmax > 0.0) v = (float)(1.0 / sqrt(d));
-      }
-      invd[c] = v;
-    }
-    if (r) {
-      for (int idx = tid; idx < N * N; idx += NT) {
-        const int k = idx % N, c = idx / N;  // column-major (k, c)
-        const double dk = W[k * N + k];
-        const bool live = dk > tol && dmax > 0.0;
-        if (pass == 0) {
-          R1[idx] = (live && c >= k) ? W[k * N + c] / sqrt(dk) : 0.0;
-        } else {
-          double a = 0.0;
-          if (live && c >= k) {
-            const double sk = 1.0 / sqrt(dk);
-            for (int j = k; j <= c; ++j) a += W[k * N + j] * sk * R1[j + N * c];
-          }
-          if (crank == 0) r[idx] = a;
-        }
-      }
-    }
-    __syncthreads();
-    // Forward substitution q R = y, one row per thread.
-    for (int i = tid; i < nl; i += NT) {
-      float q[NP];
-#pragma unroll
-      for (int j4 = 0; j4 < NP / 4; ++j4) {
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (j4 < TTa) v = *reinterpret_cast<const float4*>(&Ys[(size_t)i * S + 4 * j4]);
-        q[4 * j4] = v.x;
-        q[4 * j4 + 1] = v.y;
-        q[4 * j4 + 2] = v.z;
-        q[4 * j4 + 3] = v.w;
-      }
-#pragma unroll
-      for (int c = 0; c < NP; ++c) {
-        // four independent partial sums (one per float4 lane) shorten the dependency chain
-        float a0 = q[c], a1 = 0.f, a2 = 0.f, a3 = 0.f;
-#pragma unroll
-        for (int k4 = 0; k4 < (c + 3) / 4; ++k4) {
-          const float4 rr = *reinterpret_cast<const float4*>(&Rf[c * NP + 4 * k4]);
-          a0 = fmaf(-q[4 * k4], rr.x, a0);
-          a1 = fmaf(-q[4 * k4 + 1], rr.y, a1);
-          a2 = fmaf(-q[4 * k4 + 2], rr.z, a2);
-          a3 = fmaf(-q[4 * k4 + 3], rr.w, a3);
-        }
-        q[c] = ((a0 + a1) + (a2 + a3)) * invd[c];
-      }
-      if (pass == 0) {
-#pragma unroll
-        for (int j4 = 0; j4 < NP / 4; ++j4)
-          if (j4 < TTa)
-            *reinterpret_cast<float4*>(&Ys[(size_t)i * S + 4 * j4]) =
-                make_float4(q[4 * j4], q[4 * j4 + 1], q[4 * j4 + 2], q[4 * j4 + 3]);
-      } else {
-        const long long gi = row0 + i;
-#pragma unroll
-        for (int c = 0; c < NP; ++c)
-          if (c < N) y[gi * vs + (long long)c * es] = q[c];
-      }
-    }
-  }
-  cl_sync();  // peers may still be reading this CTA's second partial
-}
-
 static int max_optin_smem() { return dev_smem_max(); }
-
-// Cluster shape and shared-memory bytes of k_cholqr2_small: the fewest CTAs (at most 8) with
-// at least 128 rows each that fit in shared memory; 0 when the sketch does not fit.
-static size_t cholqr2_small_smem(long long n, int N, bool want_r, int* S_out, int* cl_out, int* rpc_out) {
-  if (N < 1 || N > 80 || n < 1 || n > (1LL << 20)) return 0;
-  if (N > 64 && want_r) return 0;  // the one-CTA wide variant forms no R
-  const int NP = N <= 16 ? 16 : N <= 32 ? 32 : N <= 48 ? 48 : N <= 64 ? 64 : 80;
-  int S = 4 * ((N + 3) / 4);
-  if (((S / 4) & 1) == 0) S += 4;
-  const size_t WN = ((size_t)N * N + 1) & ~(size_t)1;
-  const size_t fixed = (NP > 64 ? 1 : 3) * WN * 8 + (size_t)NP * NP * 4 + NP * 4 + (want_r ? (size_t)N * N * 8 : 0);
-  const int cl_max = NP > 64 ? 1 : 8;
-  for (int cl = (int)std::min<long long>(cl_max, std::max<long long>(1, (n + 127) / 128)); cl <= cl_max; ++cl) {
-    const long long rpc = (n + cl - 1) / cl;
-    const size_t bytes = (size_t)rpc * S * 4 + fixed;
-    if (bytes <= (size_t)max_optin_smem()) {
-      *S_out = S;
-      *cl_out = cl;
-      *rpc_out = (int)rpc;
-      return bytes;
-    }
-  }
-  return 0;
-}
-
-static int cholqr_passes(float* y, long long n, int N, long long vs, long long es, double* r, Arena& ws,
-                         DevStatus* st, cudaStream_t s, int passes, bool acc64);
-
-int launch_cholqr2(float* y, long long n, int N, long long vs, long long es, double* r,
-                   Arena& ws, DevStatus* st, cudaStream_t s) {
-  return cholqr_passes(y, n, N, vs, es, r, ws, st, s, 2, true);
-}
-
-// One CholeskyQR pass: the orthonormalisation between power iterations, which only has to keep
-// the basis well conditioned (the sketch that follows is orthonormalised by CholeskyQR2).  The
-// Gram is FP32-accumulated (FP64 across chunks of vectors), or FP64 per product with acc64: a
-// basis whose columns span a graded spectrum (condition kappa) then comes out with
-// orthogonality ~kappa * 2^-24, still well conditioned, where the FP32 Gram (condition
-// kappa^2) would lose the small directions.
-int launch_orth_power(float* y, long long n, int N, long long vs, long long es, Arena& ws, DevStatus* st,
-                      cudaStream_t s, bool acc64) {
-  return cholqr_passes(y, n, N, vs, es, nullptr, ws, st, s, 1, acc64);
-}
-
-static int cholqr_passes(float* y, long long n, int N, long long vs, long long es, double* r, Arena& ws,
-                         DevStatus* st, cudaStream_t s, int passes, bool acc64) {
-  if (N <= 0 || n <= 0) return TT_OK;
-  if (N > TT_MAX_SMALL) {
-    set_error(TT_ERR_UNSUPPORTED, "cholqr2 width %d > %d", N, TT_MAX_SMALL);
-    return TT_ERR_UNSUPPORTED;
-  }
-  int S = 0, cl = 1, rpc = 0;
-  const size_t sshm = cholqr2_small_smem(n, N, r != nullptr, &S, &cl, &rpc);
-  if (sshm > 0) {
-    {
-      const int mx = max_optin_smem();
-      smem_optin_k(k_cholqr2_small<16>, mx);
-      smem_optin_k(k_cholqr2_small<32>, mx);
-      smem_optin_k(k_cholqr2_small<48>, mx);
-      smem_optin_k(k_cholqr2_small<64>, mx);
-      smem_optin_k(k_cholqr2_small<80>, mx);
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(cl, 1, 1);
-    cfg.blockDim = dim3(N > 64 ? 256 : 512, 1, 1);
-    cfg.dynamicSmemBytes = sshm;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = cl;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    const int nn = (int)n;
-    const double tol = 1e-12;
-    cudaError_t e;
-    if (N <= 16)
-      e = cudaLaunchKernelEx(&cfg, k_cholqr2_small<16>, y, nn, N, vs, es, S, rpc, r, tol);
-    else if (N <= 32)
-      e = cudaLaunchKernelEx(&cfg, k_cholqr2_small<32>, y, nn, N, vs, es, S, rpc, r, tol);
-    else if (N <= 48)
-      e = cudaLaunchKernelEx(&cfg, k_cholqr2_small<48>, y, nn, N, vs, es, S, rpc, r, tol);
-    else if (N <= 64)
-      e = cudaLaunchKernelEx(&cfg, k_cholqr2_small<64>, y, nn, N, vs, es, S, rpc, r, tol);
-    else
-      e = cudaLaunchKernelEx(&cfg, k_cholqr2_small<80>, y, nn, N, vs, es, S, rpc, r, tol);
-    if (e == cudaSuccess) {
-      count_launch();
-      TT_LAUNCH_CHECK();
-      return TT_OK;
-    }
-    // A cluster that cannot be placed (its CTAs' shared memory on one GPC) falls through to the
-    // multi-launch path below.
-    (void)cudaGetLastError();
-  }
-  const size_t mk = ws.mark();
-  double* w = ws.take<double>((size_t)N * N);
-  double* rinv = ws.take<double>((size_t)N * N);
-  double* r1 = ws.take<double>((size_t)N * N);
-  double* r2 = ws.take<double>((size_t)N * N);
-  if (!w || !rinv || !r1 || !r2) {
-    set_error(TT_ERR_NOMEM, "cholqr2 workspace");
-    return TT_ERR_NOMEM;
-  }
-  const int NP = N <= 16 ? 16 : N <= 32 ? 32 : N <= 48 ? 48 : N <= 64 ? 64 : 128;
-  const int ri_smem = 2 * (size_t)N * chol_ld(N) * sizeof(double) + N * sizeof(int) + 16 <= 200 * 1024;
-  const size_t shm = (size_t)(ri_smem ? 2 : 1) * N * chol_ld(N) * sizeof(double) + N * sizeof(int) + 16;
-  smem_optin_k(k_chol_inv, 200 * 1024);
-  smem_optin_k(k_apply_rinv<16>, 200 * 1024);
-  smem_optin_k(k_apply_rinv<32>, 200 * 1024);
-  smem_optin_k(k_apply_rinv<48>, 200 * 1024);
-  smem_optin_k(k_apply_rinv<64>, 200 * 1024);
-  smem_optin_k(k_apply_rinv<128>, 200 * 1024);
-  for (int pass = 0; pass < passes; ++pass) {
-    TT_TRY(launch_gram(y, n, N, vs, es, w, acc64, ws, s));
-    k_chol_inv<<<1, 256, shm, s>>>(w, N, pass == 0 ? r1 : r2, rinv, 1e-12, ri_smem, st);
-    count_launch();
-    TT_LAUNCH_CHECK();
-    const size_t ashm = ((size_t)NP * NP + 128 * (size_t)(NP + 1)) * sizeof(float);
-    // persistent blocks (R^-1 staged once per block), as many as fit on the SMs
-    const int per_sm = std::max(1, std::min(8, (int)((200u * 1024u) / (ashm + 1024))));
-    const int grid = (int)std::min<long long>(ceil_div_ll(n, 128), (long long)per_sm * num_sms());
-    switch (NP) {
-      case 16: k_apply_rinv<16><<<grid, 128, ashm, s>>>(y, n, N, vs, es, rinv); break;
-      case 32: k_apply_rinv<32><<<grid, 128, ashm, s>>>(y, n, N, vs, es, rinv); break;
-      case 48: k_apply_rinv<48><<<grid, 128, ashm, s>>>(y, n, N, vs, es, rinv); break;
-      case 64: k_apply_rinv<64><<<grid, 128, ashm, s>>>(y, n, N, vs, es, rinv); break;
-      default: k_apply_rinv<128><<<grid, 128, ashm, s>>>(y, n, N, vs, es, rinv); break;
-    }
-    count_launch();
-    TT_LAUNCH_CHECK();
-  }
-  if (r && passes == 2) {
-    k_mul_upper<<<ceil_div(N * N, 256), 256, 0, s>>>(r2, r1, N, r);
-    count_launch();
-    TT_LAUNCH_CHECK();
-  }
-  ws.reset(mk);
-  return TT_OK;
-}
 
 // ---------------------------------------------------------------------------------------
 // Symmetric eigen-decomposition: parallel cyclic Jacobi (round-robin pairs), FP64
@@ -3118,6 +2507,7 @@ __global__ void __launch_bounds__(256) k_gemm_nn(const float* __restrict__ a, lo
     __syncthreads();
     if (i < M) {
       const int kmax = (K - k0 < 64) ? K - k0 : 64;
+#pragma unroll 8  // loads of A in flight: a merge of small cores is all latency
       for (int kk = 0; kk < kmax; ++kk) {
         const float av = a[i + M * (long long)(k0 + kk)];
 #pragma unroll
@@ -3151,37 +2541,149 @@ int launch_gemm_nn(const float* a, long long M, int K, const float* b, long long
   return TT_OK;
 }
 
-// err^2 += sum_{i,J} (X[i + n1 J] - sum_{a,b} G1[a + r0 i + r0 n1 b] M[b + r1 J + r1 N a])^2
-__global__ void __launch_bounds__(256) k_recon_err(const float* __restrict__ x, int n1, long long N,
-                                                   const float* __restrict__ g1, int r0, int r1,
-                                                   const float* __restrict__ mrg, double* acc) {
-  extern __shared__ float smem[];
-  float* gs = smem;                     // r0*n1*r1
-  const int q = r0 * r1;
-  const int JT = 32;
-  float* ms = gs + r0 * n1 * r1;        // JT x q: ms[jj*q + (a + r0 b)]
+// err^2 += sum_{i,J} (X[i + P J] - sum_{a,b} L[a + r0 (i + P b)] R[b + rk (J + N a)])^2, and ||X||^2.
+//
+// A GEMM over q = r0 rk whose 128 x 128 result tile is compared with X in registers and never
+// written.  Bound by the FP32 FMAs (2 q per element of X; 0.93 ms for a 32^6 tensor at q = 32) next
+// to one read of X (0.66 ms).  256 threads of 8 x 8 entries: 4 shared-memory loads of 16 bytes feed
+// 32 paired FMAs, the 32-deep K chunks of both factors double-buffered by cp.async.  Difference and
+// sums are FP64; two blocks per SM, so one block's X loads and conversions run beside the other's
+// FMAs.  (The kernel this one replaces took two shared-memory loads per FMA, and a merged factor as
+// large as X besides: 18.0 ms for the 32^6 check at ranks 32, 2.4 ms now.)
+constexpr int RE_T = 128, RE_KC = 32, RE_LD = RE_T + 4;
+constexpr size_t RE_SMEM = (size_t)2 * 2 * RE_KC * RE_LD * sizeof(float);
+
+template <bool RING>
+__global__ void __launch_bounds__(256, 2) k_recon_err(const float* __restrict__ x, long long P, long long N,
+                                                      const float* __restrict__ lf, const float* __restrict__ rf,
+                                                      int r0, int rk, double* acc) {
+  extern __shared__ __align__(16) float sm_re[];
+  float* const ls = sm_re;                       // [2][KC][LD] rows i
+  float* const rs = sm_re + 2 * RE_KC * RE_LD;   // [2][KC][LD] columns J
   __shared__ double sh[32];
-  for (int f = threadIdx.x; f < r0 * n1 * r1; f += blockDim.x) gs[f] = g1[f];
-  double d2 = 0.0, x2 = 0.0;
-  for (long long J0 = (long long)blockIdx.x * JT; J0 < N; J0 += (long long)gridDim.x * JT) {
-    __syncthreads();
-    for (int f = threadIdx.x; f < JT * q; f += blockDim.x) {
-      const int b = f % r1, jj = (f / r1) % JT, a = f / (r1 * JT);
-      const long long J = J0 + jj;
-      ms[jj * q + a + r0 * b] = (J < N) ? mrg[b + (long long)r1 * J + (long long)r1 * N * a] : 0.f;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int q = r0 * rk, nk = (q + RE_KC - 1) / RE_KC;
+  const long long pt = (P + RE_T - 1) / RE_T, nt = (N + RE_T - 1) / RE_T, ntiles = pt * nt;
+  const long long my = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;  // tiles of this block
+  const long long stages = my * nk;
+  const bool lv = r0 == 1 && (P & 3) == 0 && (reinterpret_cast<uintptr_t>(lf) & 15) == 0;
+  const bool xv = (P & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  // stage st: K chunk st % nk of this block's tile st / nk, into buffer st & 1
+  auto load = [&](long long st) {
+    const long long t = blockIdx.x + (st / nk) * gridDim.x;
+    const int k0 = (int)(st % nk) * RE_KC;
+    const long long i0 = (t % pt) * RE_T, j0 = (t / pt) * RE_T;
+    float* const l = ls + (st & 1) * RE_KC * RE_LD;
+    float* const r = rs + (st & 1) * RE_KC * RE_LD;
+    if (lv) {
+      const int kk = tid >> 5, i4 = 4 * (tid & 31);
+      const float* src = lf + (i0 + i4) + P * (k0 + kk);
+      const bool in = i0 + i4 < P;  // P % 4 == 0: four rows or none
+#pragma unroll
+      for (int u = 0; u < RE_KC / 8; ++u) {
+        const bool ok = in && k0 + kk + 8 * u < q;
+        cp_async16z(l + (kk + 8 * u) * RE_LD + i4, ok ? src + 8 * u * P : lf, ok);
+      }
+    } else {
+#pragma unroll 4
+      for (int u = 0; u < RE_KC * RE_T / 256; ++u) {
+        const int f = tid + 256 * u, kk = f >> 7, i = f & 127;
+        const int c = k0 + kk, b = RING ? c / r0 : c, a = RING ? c - b * r0 : 0;
+        const bool ok = c < q && i0 + i < P;
+        cp_async4(l + kk * RE_LD + i, ok ? lf + a + r0 * ((i0 + i) + P * b) : lf, ok);
+      }
     }
-    __syncthreads();
-    for (int f = threadIdx.x; f < JT * n1; f += blockDim.x) {
-      const int i = f % n1, jj = f / n1;
-      const long long J = J0 + jj;
-      if (J >= N) continue;
-      float s = 0.f;
-      for (int a = 0; a < r0; ++a)
-        for (int b = 0; b < r1; ++b) s = fmaf(gs[a + r0 * i + r0 * n1 * b], ms[jj * q + a + r0 * b], s);
-      const double xv = x[i + (long long)n1 * J];
-      const double dv = xv - (double)s;
-      d2 += dv * dv;
-      x2 += xv * xv;
+    // consecutive lanes take consecutive contraction indices: for a train R's columns are contiguous
+    const int kk = tid & 31, c = k0 + kk, b = RING ? c / r0 : c, a = RING ? c - b * r0 : 0;
+    const float* src = rf + b + rk * ((j0 + (tid >> 5)) + N * a);
+    const int nj = c < q ? (int)min((long long)RE_T, N - j0) : 0;
+#pragma unroll
+    for (int u = 0; u < RE_T / 8; ++u) {
+      const int j = (tid >> 5) + 8 * u;
+      cp_async4(r + kk * RE_LD + j, j < nj ? src + (long long)(8 * rk) * u : rf, j < nj);
+    }
+  };
+  uint64_t s2[4][8];  // rows (i, i + 1) of four row pairs x 8 columns
+  double d2 = 0.0, x2 = 0.0;
+  if (stages > 0) load(0);
+  cp_async_commit();
+  for (long long st = 0; st < stages; ++st) {
+    cp_async_wait<0>();
+    __syncthreads();  // stage st landed for every thread; buffer (st + 1) & 1 is no longer read
+    if (st + 1 < stages) load(st + 1);
+    cp_async_commit();
+    const int kc = (int)(st % nk);
+    const long long t = blockIdx.x + (st / nk) * gridDim.x;
+    const long long ib = (t % pt) * RE_T, jb = (t / pt) * RE_T;
+    const bool whole = xv && ib + RE_T <= P && jb + RE_T <= N;
+    if (kc == 0) {
+      if (whole) {  // the tile of X into L2 while its products are formed: 512 lines, 2 per thread
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(x + ib + 32 * (tid & 3) + P * (jb + (tid >> 2) + 64 * u)));
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int c = 0; c < 8; ++c) s2[e][c] = 0ull;
+    }
+    const float* l = ls + (st & 1) * RE_KC * RE_LD + 4 * tx;
+    const float* r = rs + (st & 1) * RE_KC * RE_LD + 4 * ty;
+    const int kmax = min(RE_KC, q - kc * RE_KC);
+#pragma unroll 4
+    for (int kk = 0; kk < kmax; ++kk) {
+      const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(l + kk * RE_LD);
+      const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(l + kk * RE_LD + 64);
+      const float4 b0 = *reinterpret_cast<const float4*>(r + kk * RE_LD);
+      const float4 b1 = *reinterpret_cast<const float4*>(r + kk * RE_LD + 64);
+      const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const uint64_t bd = f2_dup(b[c]);
+        ffma2(s2[0][c], a0.x, bd);
+        ffma2(s2[1][c], a0.y, bd);
+        ffma2(s2[2][c], a1.x, bd);
+        ffma2(s2[3][c], a1.y, bd);
+      }
+    }
+    if (kc + 1 < nk) continue;
+    const long long i0 = ib + 4 * tx, j0 = jb + 4 * ty;
+    auto add = [&](float xe, float se) {
+      const double xd = xe, dv = xd - (double)se;
+      d2 = fma(dv, dv, d2);
+      x2 = fma(xd, xd, x2);
+    };
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const long long i = i0 + 64 * h;
+      if (whole) {
+        // 8 loads in flight (a load at a time, each waited for, took 4.1 ms instead of 2.4)
+        float4 v[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          v[c] = __ldcs(reinterpret_cast<const float4*>(x + i + P * (j0 + (c & 3) + (c & 4) * 16)));
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          float s0, s1, s3, s4;
+          f2_unpack(s2[2 * h][c], s0, s1);
+          f2_unpack(s2[2 * h + 1][c], s3, s4);
+          add(v[c].x, s0);
+          add(v[c].y, s1);
+          add(v[c].z, s3);
+          add(v[c].w, s4);
+        }
+      } else {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const long long j = j0 + (c & 3) + (c & 4) * 16;
+          float sr[4];
+          f2_unpack(s2[2 * h][c], sr[0], sr[1]);
+          f2_unpack(s2[2 * h + 1][c], sr[2], sr[3]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (j < N && i + e < P) add(x[i + e + P * j], sr[e]);
+        }
+      }
     }
   }
   d2 = block_sum(d2, sh);
@@ -3192,16 +2694,16 @@ __global__ void __launch_bounds__(256) k_recon_err(const float* __restrict__ x, 
   }
 }
 
-int launch_recon_err(const float* x, int n1, long long N, const float* g1, int r0, int r1,
-                     const float* mrg, double* acc, cudaStream_t s) {
-  const size_t shm = ((size_t)r0 * n1 * r1 + 32 * (size_t)r0 * r1) * sizeof(float);
-  if (shm > 200 * 1024) {
-    set_error(TT_ERR_UNSUPPORTED, "reconstruction check: first core too large");
-    return TT_ERR_UNSUPPORTED;
-  }
-  TT_TRY(smem_optin_k(k_recon_err, 200 * 1024));
-  const int grid = (int)std::min<long long>(ceil_div_ll(N, 32), 8LL * num_sms());
-  k_recon_err<<<grid, 256, shm, s>>>(x, n1, N, g1, r0, r1, mrg, acc);
+int launch_recon_err(const float* x, long long P, long long N, const float* lf, const float* rf, int r0, int rk,
+                     double* acc, cudaStream_t s) {
+  TT_TRY(smem_optin_k(k_recon_err<false>, RE_SMEM));
+  TT_TRY(smem_optin_k(k_recon_err<true>, RE_SMEM));
+  const long long tiles = ceil_div_ll(P, RE_T) * ceil_div_ll(N, RE_T);
+  const int grid = (int)std::min<long long>(tiles, 2LL * num_sms());
+  if (r0 == 1)
+    k_recon_err<false><<<grid, 256, RE_SMEM, s>>>(x, P, N, lf, rf, r0, rk, acc);
+  else
+    k_recon_err<true><<<grid, 256, RE_SMEM, s>>>(x, P, N, lf, rf, r0, rk, acc);
   count_launch();
   TT_LAUNCH_CHECK();
   return TT_OK;
