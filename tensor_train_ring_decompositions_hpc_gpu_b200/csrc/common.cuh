@@ -73,6 +73,11 @@ __device__ __forceinline__ uint64_t f2_dup(float a) {
   asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
   return r;
 }
+__device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
 __device__ __forceinline__ void f2_unpack(uint64_t v, float& lo, float& hi) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }

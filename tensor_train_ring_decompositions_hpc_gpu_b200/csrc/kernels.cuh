@@ -56,14 +56,13 @@ int launch_project(const float* a, long long m, long long n, const float* q, int
 int launch_gram(const float* x, long long nvec, int M, long long vs, long long es, double* w,
                 bool acc64, Arena& ws, cudaStream_t s);
 
-// CholeskyQR2 on a tall FP32 matrix, element (j, c) at y[j*vs + c*es], n x N.
-// Writes R (N x N, FP64, upper) when r != nullptr.
-int launch_cholqr2(float* y, long long n, int N, long long vs, long long es, double* r,
-                   Arena& ws, DevStatus* st, cudaStream_t s);
+// CholeskyQR2 on a tall FP32 matrix (n x N, column-major, ld), in place; y64 (or null): the matrix
+// in FP64 (ld = n), taken instead of y's contents.  Writes R (N x N, FP64, upper) when r != nullptr.
+int launch_cholqr2(const double* y64, float* y, long long n, int N, long long ld, double* r, Arena& ws,
+                   cudaStream_t s);
 // One CholeskyQR pass (between power iterations): FP32-accumulated Gram, or FP64 products with
 // acc64 (graded spectra, whose small directions lie below the FP32 Gram's resolution).
-int launch_orth_power(float* y, long long n, int N, long long vs, long long es, Arena& ws, DevStatus* st,
-                      cudaStream_t s, bool acc64 = false);
+int launch_orth_power(float* y, long long n, int N, long long ld, Arena& ws, cudaStream_t s, bool acc64 = false);
 
 // Arena bytes launch_syev takes for N > 64 (the rotation log); 0 for N <= 64.
 size_t syev_ws_bytes(int N, int max_sweeps);
@@ -124,10 +123,11 @@ int launch_diff_norm(const float* x, const float* y, long long count, double* ac
 int launch_gemm_nn(const float* a, long long M, int K, const float* b, long long N, float* c,
                    cudaStream_t s);
 
-// Fused reconstruction check of a ring/train: acc += sum_J ||X[:, J] - sum_a G1[a] M[:, J, a]||^2
-// and ||X||^2, where G1 is (r0, n1, r1) and M is (r1, N, r0).
-int launch_recon_err(const float* x, int n1, long long N, const float* g1, int r0, int r1,
-                     const float* mrg, double* acc, cudaStream_t s);
+// Fused reconstruction check of a ring/train: acc += ||X - X^||^2 and ||X||^2, X (P x N) and
+// X^[i, J] = sum_{a,b} L[a, i, b] R[b, J, a] with the merged left cores L (r0, P, rk) and the merged
+// right cores R (rk, N, r0).
+int launch_recon_err(const float* x, long long P, long long N, const float* lf, const float* rf, int r0, int rk,
+                     double* acc, cudaStream_t s);
 
 // Learned predictor (mlp.cu).  Features from the descending probe eigenvalues mu
 // (TT_PROBE_COLS of them); network inference; training (mode 0: Adam steps on Philox-drawn

@@ -1,0 +1,63 @@
+"""Edge sizes of the FP32 / FP64 kernels: tile remainders, one-element sides, unaligned rows, and the
+switch points of the launch rules, against NumPy in FP64."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+U32 = 2.0 ** -24  # unit roundoff of FP32
+
+
+def _ttr():
+    import tensor_train_ring_decompositions_hpc_gpu_b200 as ttr
+    return ttr
+
+
+def _dev(x, dev, dtype=np.float32):
+    import torch
+    return torch.from_numpy(np.asfortranarray(x, dtype=dtype)).to(dev)
+
+
+@pytest.mark.parametrize("ring,n,ranks", [
+    (False, (5, 3), (1, 3, 1)),
+    (False, (128, 128), (1, 32, 1)),              # one tile, one K chunk
+    (False, (129, 127), (1, 33, 1)),              # remainders on every side
+    (False, (4, 1, 260, 7), (1, 2, 2, 5, 1)),
+    (False, (12, 12, 12, 12, 12), (1, 7, 40, 65, 9, 1)),
+    (False, (6, 20, 20, 22), (1, 6, 64, 16, 1)),
+    (True, (7, 6, 5), (3, 2, 4, 3)),
+    (True, (16, 9, 17, 8), (4, 3, 11, 2, 4)),
+    (True, (130, 3, 131), (2, 5, 6, 2)),
+])
+def test_rel_error_edges(gpu, ring, n, ranks):
+    """Every merged entry is a chain of FP32 FMAs (one contraction per bond): relative errors of
+    (sum of the bond sizes + order) u of the absolute sums, taken as 4x the sums themselves."""
+    rng = np.random.default_rng(sum(n))
+    d = len(n)
+    cores = [rng.standard_normal((ranks[k], n[k], ranks[k + 1])).astype(np.float32) for k in range(d)]
+    full = (oracle.tr_full if ring else oracle.tt_full)([c.astype(np.float64) for c in cores])
+    x = (full + 1e-2 * np.linalg.norm(full) / np.sqrt(full.size) * rng.standard_normal(n)).astype(np.float32)
+    got = _ttr().rel_error(_dev(x, gpu), [_dev(c, gpu) for c in cores], ring=ring)
+    q = ranks[0] if ring else 1
+    assert abs(got - oracle.rel_error(x, full)) <= 4 * (sum(ranks) * q + d) * U32
+
+
+@pytest.mark.parametrize("n,N", [(1, 1), (3, 3), (8, 8), (64, 9), (65, 17), (129, 40), (511, 33), (640, 127),
+                                 (1471, 128), (60000, 129 - 1), (4097, 65)])
+def test_cholqr2_edges(gpu, n, N):
+    """Panel, row-chunk and cluster remainders; (60000, 128) takes the multi-launch path.  Two passes
+    over a matrix of condition < 1e3: orthogonality is the FP32 rounding of Q's entries, u sqrt(n) per
+    inner product of unit columns at worst, N^2 of them; Q R reproduces Y to the same."""
+    import torch
+    g = torch.Generator(device="cpu").manual_seed(n + N)
+    y = torch.randn((N, n), generator=g).to(gpu).t()
+    q, r = _ttr().cholqr2(y)
+    qd, rd, yd = q.double().cpu().numpy(), r.cpu().numpy(), y.double().cpu().numpy()
+    tol = 4 * U32 * N * max(1.0, np.sqrt(N))
+    assert np.linalg.norm(qd.T @ qd - np.eye(N)) <= tol
+    assert np.linalg.norm(qd @ rd - yd) <= tol * np.linalg.norm(yd)
+    assert np.allclose(np.tril(rd, -1), 0.0) and np.all(np.diag(rd) > 0.0)
+    q2, _ = _ttr().cholqr2(y, want_r=False)
+    assert torch.equal(q, q2)  # R is a by-product: Q is the same with and without it
