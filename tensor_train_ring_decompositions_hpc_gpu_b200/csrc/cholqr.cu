@@ -505,7 +505,7 @@ __global__ void k_mul_upper(const double* __restrict__ r2, const double* __restr
 constexpr double kCqTol = 1e-12;  // pivots below this share of the largest diagonal: dependent columns
 
 int cholqr_passes(const double* y64, float* y, long long n, int N, long long ld, double* r, Arena& ws,
-                  cudaStream_t s, int passes, bool acc64) {
+                  cudaStream_t s, int passes) {
   if (N <= 0 || n <= 0) return TT_OK;
   if (N > TT_MAX_SMALL) {
     set_error(TT_ERR_UNSUPPORTED, "cholqr2 width %d > %d", N, TT_MAX_SMALL);
@@ -568,7 +568,7 @@ int cholqr_passes(const double* y64, float* y, long long n, int N, long long ld,
   const int per_sm = std::max(1, std::min(8, (int)((size_t)dev_smem_max() / (asm_ + 1024))));
   const int grid = (int)std::min<long long>(ceil_div_ll(n, CQ_T), (long long)per_sm * dev_sms());
   for (int pass = 0; pass < passes; ++pass) {
-    TT_TRY(launch_gram(y, n, N, 1, ld, w, acc64, ws, s));
+    TT_TRY(launch_gram(y, n, N, 1, ld, w, ws, s));
     k_chol_inv<<<1, CQ_T, csm, s>>>(w, N, kCqTol, tf, !r ? nullptr : pass == 0 ? r1 : r2);
     count_launch();
     TT_LAUNCH_CHECK();
@@ -589,17 +589,15 @@ int cholqr_passes(const double* y64, float* y, long long n, int N, long long ld,
 
 int launch_cholqr2(const double* y64, float* y, long long n, int N, long long ld, double* r, Arena& ws,
                    cudaStream_t s) {
-  return cholqr_passes(y64, y, n, N, ld, r, ws, s, 2, true);
+  return cholqr_passes(y64, y, n, N, ld, r, ws, s, 2);
 }
 
 // One CholeskyQR pass: the orthonormalisation between power iterations, which only has to keep
-// the basis well conditioned (the sketch that follows is orthonormalised by CholeskyQR2).  Where the
-// Gram is a launch of its own it is FP32-accumulated (FP64 across chunks of vectors), or FP64 per
-// product with acc64: a basis whose columns span a graded spectrum (condition kappa) then comes out
-// with orthogonality ~kappa * 2^-24, still well conditioned, where the FP32 Gram (condition
-// kappa^2) would lose the small directions.  A basis that fits one launch gets both passes there.
-int launch_orth_power(float* y, long long n, int N, long long ld, Arena& ws, cudaStream_t s, bool acc64) {
-  return cholqr_passes(nullptr, y, n, N, ld, nullptr, ws, s, 1, acc64);
+// the basis well conditioned (the sketch that follows is orthonormalised by CholeskyQR2): a basis whose
+// columns span a graded spectrum (condition kappa) comes out with orthogonality ~kappa * 2^-24.  A
+// basis that fits one launch gets both passes there.
+int launch_orth_power(float* y, long long n, int N, long long ld, Arena& ws, cudaStream_t s) {
+  return cholqr_passes(nullptr, y, n, N, ld, nullptr, ws, s, 1);
 }
 
 }  // namespace ttr

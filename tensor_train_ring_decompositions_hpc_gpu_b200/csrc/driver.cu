@@ -703,23 +703,23 @@ int run_chain(tt_ctx* c, const float* x_in, Plan P, const tt_opts& o, float* con
     }
     return TT_OK;
   };
-  // Gram of the rows of an unfolding with m <= 128 rows (the exact step).  Up to 32 rows: the
-  // exact CUDA-core kernel in every form (FP32 products, FP64 sums), whose result resolves
-  // eigenvalues down to ~1e-9 of the largest; the tensor cores' truncating FP32 accumulation
-  // would bias the small ones.  Wider: tensor cores when allowed, else the FP32 engine.
-  // `precise` (adaptive ranks: energies to ~1e-8 relative) keeps short unfoldings, whose few
-  // partial sums do not average the FP32 rounding out, on FP64 products.
+  // Gram of the rows of an unfolding with m <= 128 rows (the exact step).  Up to 32 rows: the exact
+  // CUDA-core kernels in every form (FP32 products, FP64 sums), whose result
+  // resolves eigenvalues down to ~1e-9 of the largest; the tensor cores' truncating FP32 accumulation
+  // would bias the small ones.  `precise` (adaptive ranks: energies to ~1e-8 relative) keeps short
+  // unfoldings, whose few partial sums do not average the FP32 rounding out, on FP64 products.  Wider:
+  // tensor cores when allowed, else FP64 products.
   auto gram_rows = [&](const float* a, long long mm, long long nc, double* w, int eng, bool precise) -> int {
-    const bool long_unf = nc >= (1LL << 16);
-    if (mm <= 32 && (!precise || long_unf)) {
-      const int rc = launch_gram32x(a, nc, (int)mm, w, ws, c->dstat, s);
+    if (mm <= 32 && (!precise || nc >= (1LL << 16))) {
+      int rc = launch_gram32x(a, nc, (int)mm, w, ws, c->dstat, s);
+      if (rc == TT_ERR_UNSUPPORTED) rc = launch_gram32u(a, nc, (int)mm, w, ws, s);
       if (rc != TT_ERR_UNSUPPORTED) return rc;
     }
-    if (eng == TT_GEMM_TC && !precise) {
+    if (eng == TT_GEMM_TC && !precise && mm > 32) {
       const int rc = launch_gram_tc(a, mm, nc, w, ws, c->dstat, s);
       if (rc != TT_ERR_UNSUPPORTED) return rc;
     }
-    return launch_gram(a, nc, (int)mm, mm, 1, w, precise && nc < (1LL << 22), ws, s);
+    return launch_gram(a, nc, (int)mm, mm, 1, w, ws, s);
   };
   int npasses = 0, natt = 0, nfall = 0;  // bulk passes, EDrSVD attempts, learned fallbacks
   std::vector<int> step_ks((size_t)nsteps, 0), step_pw((size_t)nsteps, 0), step_att((size_t)nsteps, 0);
@@ -894,7 +894,7 @@ int run_chain(tt_ctx* c, const float* x_in, Plan P, const tt_opts& o, float* con
                                 s);
         }));
         TT_TRY(pass.run(TT_PASS_OTHER, 2.0 * cols * b * b, 4.0 * cols * b,
-                        [&] { return launch_gram(B.bt, cols, b, b, 1, B.w, true, ws, s); }));
+                        [&] { return launch_gram(B.bt, cols, b, b, 1, B.w, ws, s); }));
         TT_TRY(launch_syev(B.w, b, B.evals, B.evecs, max_sweeps, ws, c->dstat, s));
         k_store_sigma<<<1, 64, 0, s>>>(B.evals, std::min(b, TT_STATS_MAX_SIGMA), sigdst);
         count_launch();
@@ -944,7 +944,7 @@ int run_chain(tt_ctx* c, const float* x_in, Plan P, const tt_opts& o, float* con
       npasses += 2;
       // W = A^T A over the rows of A (vectors = rows i, components = columns)
       TT_TRY(pass.run(TT_PASS_GRAM, 2.0 * m * cols * cols, 4.0 * m * cols,
-                      [&] { return launch_gram(cur, m, (int)cols, 1, m, B.w, true, ws, s); }));
+                      [&] { return launch_gram(cur, m, (int)cols, 1, m, B.w, ws, s); }));
       TT_TRY(launch_syev(B.w, (int)cols, B.evals, B.evecs, max_sweeps, ws, c->dstat, s));
       k_store_sigma<<<1, 64, 0, s>>>(B.evals, (int)std::min<long long>(cols, TT_STATS_MAX_SIGMA), sigdst);
       count_launch();
@@ -988,10 +988,8 @@ int run_chain(tt_ctx* c, const float* x_in, Plan P, const tt_opts& o, float* con
             return launch_project(cur, m, cols, B.yf, ksa, m, B.bt, cols, OUT_COLMAJOR, 1, 1, engine, ws, c->dstat,
                                   s);
           }));
-          // Adaptive ranks need the basis beyond the FP32 Gram's resolution (graded spectra
-          // down to delta / ||A|| ~ 1e-4): the pass forms its Gram with FP64 products there.
           TT_TRY(pass.run(TT_PASS_OTHER, 4.0 * cols * ksa * ksa, 12.0 * cols * ksa, [&] {
-            return launch_orth_power(B.bt, cols, ksa, cols, ws, s, adaptive);
+            return launch_orth_power(B.bt, cols, ksa, cols, ws, s);
           }));
           TT_TRY(pass.run(TT_PASS_SKETCH, fl_pass, by_pass, [&] {
             return launch_sketch(cur, m, cols, B.bt, ksa, 1, cols, B.yd, engine, ws, c->dstat, s);
@@ -1017,7 +1015,7 @@ int run_chain(tt_ctx* c, const float* x_in, Plan P, const tt_opts& o, float* con
             const int rc = launch_gram_tc(B.bt, ksa, cols, B.w, ws, c->dstat, s);
             if (rc != TT_ERR_UNSUPPORTED) return rc;
           }
-          return launch_gram(B.bt, cols, ksa, ksa, 1, B.w, true, ws, s);
+          return launch_gram(B.bt, cols, ksa, ksa, 1, B.w, ws, s);
         }));
         // Fixed ranks keep the first re <= 16 eigenpairs of a wide sketch's Gram: above 64 the
         // subspace solver's 32 Ritz pairs (the eigenvalues beyond them are reported as 0).
@@ -1092,7 +1090,7 @@ int run_chain(tt_ctx* c, const float* x_in, Plan P, const tt_opts& o, float* con
                           }));
           ++npasses;
           TT_TRY(launch_f64_to_f32_cols(B.y0, m, m, TT_PROBE_COLS, B.yf, m, TT_PROBE_COLS, s));
-          TT_TRY(launch_gram(B.yf, m, TT_PROBE_COLS, 1, m, B.w, true, ws, s));
+          TT_TRY(launch_gram(B.yf, m, TT_PROBE_COLS, 1, m, B.w, ws, s));
           TT_TRY(launch_syev(B.w, TT_PROBE_COLS, B.evals, B.evecs, max_sweeps, ws, c->dstat, s));
           const double tol = energy > 0.0 ? std::sqrt(delta2 / energy) : 1.0;
           TT_TRY(launch_probe_features(B.evals, energy, tol, m, cols, feat, s));
@@ -1567,7 +1565,7 @@ extern "C" int tt_probe_features(tt_ctx* c, const float* a, long long m, long lo
   TT_TRY(launch_gaussian(om, n, P, n, seed, stream_id, s));
   TT_TRY(launch_sketch(a, m, n, om, P, 1, n, yd, engine, ws, c->dstat, s));
   TT_TRY(launch_f64_to_f32_cols(yd, m, m, P, yf, m, P, s));
-  TT_TRY(launch_gram(yf, m, P, 1, m, w, true, ws, s));
+  TT_TRY(launch_gram(yf, m, P, 1, m, w, ws, s));
   TT_TRY(launch_syev(w, P, ev, vec, 40, ws, c->dstat, s));
   TT_TRY(launch_probe_features(ev, energy, tol, m, n, features, s));
   return check_status(c);
@@ -1661,7 +1659,7 @@ extern "C" int tt_k_gram_rows(tt_ctx* c, const float* a, long long m, long long 
   if (gemm != TT_GEMM_TC && m <= 32) rc = launch_gram32x(a, n, (int)m, w, ws, c->dstat, c->stream);
   if (rc == TT_ERR_UNSUPPORTED && gemm != TT_GEMM_FP32 && tc_available())
     rc = launch_gram_tc(a, m, n, w, ws, c->dstat, c->stream);
-  if (rc == TT_ERR_UNSUPPORTED) rc = launch_gram(a, n, (int)m, m, 1, w, false, ws, c->stream);
+  if (rc == TT_ERR_UNSUPPORTED) rc = launch_gram(a, n, (int)m, m, 1, w, ws, c->stream);
   TT_TRY(rc);
   return check_status(c);
 }
@@ -1678,7 +1676,7 @@ extern "C" int tt_k_gram_tall(tt_ctx* c, const float* z, long long n, int N, lon
   TT_CUDA(cudaSetDevice(c->device));
   Arena ws;
   TT_TRY(ws_for(c, gram_ws_bytes(n, N), ws));
-  TT_TRY(launch_gram(z, n, N, rs, cs, w, true, ws, c->stream));
+  TT_TRY(launch_gram(z, n, N, rs, cs, w, ws, c->stream));
   TT_CUDA(cudaStreamSynchronize(c->stream));
   return TT_OK;
 }

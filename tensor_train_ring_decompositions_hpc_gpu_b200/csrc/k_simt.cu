@@ -1,5 +1,5 @@
 // CUDA-core kernels: the plain-FP32 GEMM engine and every small linear-algebra kernel of the
-// TT/TR-SVD chain (Gaussian test matrix, Gram matrices, Jacobi eigen-solver,
+// TT/TR-SVD chain (Gaussian test matrix, Jacobi eigen-solver,
 // bond permute, core folding, reconstruction error).
 #include <float.h>
 #include <stdlib.h>
@@ -17,7 +17,6 @@ namespace ttr {
 thread_local int g_kernel_launches = 0;
 
 static int num_sms() { return dev_sms(); }
-static int max_optin_smem();
 
 // ---------------------------------------------------------------------------------------
 // Philox4x32-10 Gaussian generator (replaces curandGenerateNormal, TT3O:585-587)
@@ -103,28 +102,6 @@ int launch_gaussian(float* out, long long rows, int cols, long long ld, unsigned
 // ---------------------------------------------------------------------------------------
 // Plain-FP32 sketch  Y = A * W  (split over the long dimension n, FP64 reduction of splits)
 // ---------------------------------------------------------------------------------------
-// Asynchronous global -> shared copies (cp.async): 16-byte, and 16- or 4-byte with zero fill when
-// `valid` is false (no byte is read then).
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async16z(void* dst, const void* src, bool valid) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-               "l"(src), "r"(valid ? 16 : 0)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async4(void* dst, const void* src, bool valid) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-               "l"(src), "r"(valid ? 4 : 0)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int PENDING>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
-}
-
 // 32 x RI rows of A per block (RI per thread) x NT sketch columns (NT / 8 per thread); narrow
 // sketches (NT <= 24) take RI = 16 rows per thread, so that each shared-memory load feeds more
 // FMAs.  The long dimension runs in chunks of JC columns of A (32 KB of A per chunk) streamed
@@ -765,828 +742,6 @@ int launch_project(const float* a, long long m, long long n, const float* q, int
   ws.reset(mk);
   return TT_OK;
 }
-
-// ---------------------------------------------------------------------------------------
-// Gram  W = sum_j x_j x_j^T  (M <= 128), symmetric 4x4 register tiles, FP64 across blocks
-// ---------------------------------------------------------------------------------------
-template <int MP, bool ACC64>
-__global__ void __launch_bounds__(256) k_gram(const float* __restrict__ x, long long nvec, int M,
-                                              long long vs, long long es, long long vchunk,
-                                              double* __restrict__ part) {
-  constexpr int VC = 32;
-  constexpr int TT = MP / 4;
-  constexpr int NTILE = TT * (TT + 1) / 2;
-  constexpr int GROUPS = NTILE >= 256 ? 1 : 256 / NTILE;
-  constexpr int TPT = NTILE >= 256 ? (NTILE + 255) / 256 : 1;
-  __shared__ __align__(16) float xs[VC][MP];
-  __shared__ double red[GROUPS > 1 ? MP * MP : 1];
-  const int tid = threadIdx.x;
-  const long long vb = (long long)blockIdx.x * vchunk;
-  const long long ve = (vb + vchunk < nvec) ? vb + vchunk : nvec;
-
-  int ta[TPT], tb[TPT];
-  bool act[TPT];
-  int g = 0;
-#pragma unroll
-  for (int u = 0; u < TPT; ++u) {
-    int t = (GROUPS > 1) ? (tid % NTILE) : (tid + 256 * u);
-    if (GROUPS > 1) g = tid / NTILE;
-    act[u] = (GROUPS > 1) ? (g < GROUPS) : (t < NTILE);
-    int aa = 0, rem = act[u] ? t : 0;
-    while (rem >= TT - aa) {
-      rem -= TT - aa;
-      ++aa;
-    }
-    ta[u] = aa;
-    tb[u] = aa + rem;
-  }
-  float acc[TPT][16];
-  double accd[TPT][16];
-#pragma unroll
-  for (int u = 0; u < TPT; ++u)
-#pragma unroll
-    for (int e = 0; e < 16; ++e) {
-      acc[u][e] = 0.f;
-      accd[u][e] = 0.0;
-    }
-  int chunk = 0;
-  for (long long v0 = vb; v0 < ve; v0 += VC, ++chunk) {
-    if (es == 1) {
-      for (int f = tid; f < VC * MP; f += 256) {
-        const int c = f % MP, v = f / MP;
-        const long long j = v0 + v;
-        xs[v][c] = (j < ve && c < M) ? x[j * vs + c] : 0.f;
-      }
-    } else {
-      for (int f = tid; f < VC * MP; f += 256) {
-        const int v = f % VC, c = f / VC;
-        const long long j = v0 + v;
-        xs[v][c] = (j < ve && c < M) ? x[j * vs + (long long)c * es] : 0.f;
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < TPT; ++u) {
-      if (!act[u]) continue;
-      for (int v = g; v < VC; v += GROUPS) {
-        const float4 xa = *reinterpret_cast<const float4*>(&xs[v][ta[u] * 4]);
-        const float4 xb = *reinterpret_cast<const float4*>(&xs[v][tb[u] * 4]);
-        const float av[4] = {xa.x, xa.y, xa.z, xa.w};
-        const float bv[4] = {xb.x, xb.y, xb.z, xb.w};
-        if (ACC64) {
-#pragma unroll
-          for (int p = 0; p < 4; ++p)
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-              accd[u][p * 4 + r] = fma((double)av[p], (double)bv[r], accd[u][p * 4 + r]);
-        } else {
-#pragma unroll
-          for (int p = 0; p < 4; ++p)
-#pragma unroll
-            for (int r = 0; r < 4; ++r) acc[u][p * 4 + r] = fmaf(av[p], bv[r], acc[u][p * 4 + r]);
-        }
-      }
-    }
-    if (!ACC64 && (chunk & 31) == 31) {
-#pragma unroll
-      for (int u = 0; u < TPT; ++u)
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          accd[u][e] += (double)acc[u][e];
-          acc[u][e] = 0.f;
-        }
-    }
-    __syncthreads();
-  }
-  if (!ACC64) {
-#pragma unroll
-    for (int u = 0; u < TPT; ++u)
-#pragma unroll
-      for (int e = 0; e < 16; ++e) accd[u][e] += (double)acc[u][e];
-  }
-  double* dst = part + (long long)blockIdx.x * MP * MP;
-  if (GROUPS > 1) {
-    for (int gg = 0; gg < GROUPS; ++gg) {
-      if (g == gg && act[0]) {
-#pragma unroll
-        for (int p = 0; p < 4; ++p)
-#pragma unroll
-          for (int r = 0; r < 4; ++r) {
-            const int idx = (ta[0] * 4 + p) * MP + tb[0] * 4 + r;
-            red[idx] = (gg == 0) ? accd[0][p * 4 + r] : red[idx] + accd[0][p * 4 + r];
-          }
-      }
-      __syncthreads();
-    }
-    if (g == 0 && act[0]) {
-#pragma unroll
-      for (int p = 0; p < 4; ++p)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const int idx = (ta[0] * 4 + p) * MP + tb[0] * 4 + r;
-          dst[idx] = red[idx];
-        }
-    }
-  } else {
-#pragma unroll
-    for (int u = 0; u < TPT; ++u) {
-      if (!act[u]) continue;
-#pragma unroll
-      for (int p = 0; p < 4; ++p)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) dst[(ta[u] * 4 + p) * MP + tb[u] * 4 + r] = accd[u][p * 4 + r];
-    }
-  }
-}
-
-// W = sum over the per-block partials (upper tiles of size T stored, the lower half mirrored):
-// one warp per entry, lanes stride over the blocks, fixed-order shuffle tree (deterministic).
-__global__ void k_gram_reduce(const double* __restrict__ part, int nblk, int MP, int M, int T,
-                              double* __restrict__ w) {
-  const int idx = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (idx >= M * M) return;
-  const int aI = idx % M, bI = idx / M;
-  const int src = (aI / T <= bI / T) ? aI * MP + bI : bI * MP + aI;
-  double sacc = 0.0;
-  for (int k = lane; k < nblk; k += 32) sacc += part[(long long)k * MP * MP + src];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) sacc += __shfl_xor_sync(0xffffffffu, sacc, o);
-  if (lane == 0) w[aI + (long long)M * bI] = sacc;
-}
-
-static void launch_gram_reduce(const double* part, int nblk, int MP, int M, int T, double* w, cudaStream_t s) {
-  const long long threads = 32LL * M * M;
-  k_gram_reduce<<<(int)ceil_div_ll(threads, 256), 256, 0, s>>>(part, nblk, MP, M, T, w);
-}
-
-// ---------------------------------------------------------------------------------------
-// Gram of many short vectors  W = sum_j x_j x_j^T  (17 <= M <= 64 components), two layouts:
-//  * contiguous (COL = false): x_j = x + j M, M % 4 == 0, x 16-byte aligned -- the Gram of a
-//    long unfolding with few rows (columns contiguous) and of a row-major factor B^T.  A stage
-//    of VC vectors is one contiguous block, copied with 16-byte cp.async;
-//  * column-major (COL = true): component c of x_j at x[j + c ld] -- a tall n x M matrix (the
-//    power-iteration basis Z).  Each component's VC values are copied with 16-byte cp.async
-//    into a row of the stage, chunks swizzled for conflict-free column reads (gv_col_at).
-// Stages are NS deep.  Each warp computes a 32 x 32 block of W: lane (p, q) = (lane / 8,
-// lane % 8) holds rows 8p..8p+7 x columns 4q..4q+3, 12 loaded values per vector for 32 FMAs.
-// MP = 32 has one such block (12 warps split the vectors), MP = 64 the three upper blocks
-// (4 warps each); one block of 384 threads per SM.  Rows and columns >= M read neighbouring
-// words; those entries are never written out.  FP32 products accumulate over VFLUSH vectors
-// per lane (round-to-nearest FMA, unbiased) and are then added into FP64; ACC64 accumulates
-// every product in FP64 instead.
-// ---------------------------------------------------------------------------------------
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(gmem) : "memory");
-}
-
-constexpr int GV_VC = 192;  // vectors per stage
-constexpr int GV_NS = 4;    // stages in flight
-constexpr int GV_VFLUSH = 64;
-
-// Column-major stages: component c's values of the stage's vectors occupy row c (stride
-// GV_VC floats) with 4-vector chunks XOR-swizzled by the key (c >> 2) & 7, so the 16-byte copies
-// stay aligned and the reads of the rows 8p + i (i fixed) and 4q + j (j fixed) of one vector hit
-// distinct banks.  Element (c, v) of the stage sits at gv_col_at(c, v).
-__device__ __forceinline__ int gv_col_key(int c) { return ((c >> 2) & 7) << 2; }
-__device__ __forceinline__ int gv_col_at(int c, int v) { return c * GV_VC + (v ^ gv_col_key(c)); }
-
-// Copy vectors [v0, v0 + nv) of the column-major n x M matrix x (column stride ld) into a
-// column-major stage: 16-byte copies of 4 vectors when the layout allows them, 4-byte ones
-// otherwise.
-template <int NT>
-__device__ __forceinline__ void gv_load_col(float* dst, const float* __restrict__ x, long long v0, int nv, int M,
-                                            long long ld, int tid) {
-  const bool v16 = ((ld & 3) == 0) && ((v0 & 3) == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
-  const int n4 = v16 ? nv >> 2 : 0;  // whole 4-vector chunks per component
-  if (n4 > 0) {
-    const int tot = n4 * M;
-    const float inv = 1.0f / (float)n4;  // exact quotients: c < 64, far inside the 0.5 / n4 margin
-    for (int f = tid; f < tot; f += NT) {
-      const int c = (int)(((float)f + 0.5f) * inv), g = f - c * n4;
-      cp_async16(dst + gv_col_at(c, 4 * g), x + (v0 + 4 * g) + (long long)c * ld);
-    }
-  }
-  const int rest = nv - 4 * n4;  // remaining vectors, 4-byte copies
-  if (rest > 0) {
-    const int tot = rest * M;
-    const float inv = 1.0f / (float)rest;
-    for (int f = tid; f < tot; f += NT) {
-      const int c = (int)(((float)f + 0.5f) * inv), v = 4 * n4 + (f - c * rest);
-      cp_async4(dst + gv_col_at(c, v), x + (v0 + v) + (long long)c * ld);
-    }
-  }
-}
-
-template <int MP>
-struct GramVecShape {
-  static constexpr int WB = MP == 32 ? 1 : 3;    // 32 x 32 warp blocks (upper triangle)
-  static constexpr int WPB = MP == 32 ? 12 : 4;  // warps per warp block
-  static constexpr int NT = 32 * WB * WPB;       // 384
-};
-
-// FP64 products of row-major vectors convert each stage to FP64 once, in shared memory, next to
-// two FP32 stages (the conversion is the scarce unit: F2F runs at a fraction of the FP64 FMA
-// rate, and converting per use costs every lane 12 conversions per 32 products).
-static size_t gram_vec_smem(int MP, int M, bool col, bool acc64 = false) {
-  const size_t stage = col ? (size_t)MP * GV_VC : (size_t)GV_VC * M + MP;
-  const size_t red = (size_t)12 * 1024 * 2;  // per-warp 32 x 32 FP64 blocks, in floats
-  if (acc64 && !col) return std::max(stage * 2 + ((size_t)GV_VC * M + MP) * 2, red) * sizeof(float);
-  return std::max(stage * GV_NS, red) * sizeof(float);
-}
-
-template <int MP, bool ACC64, bool COL>
-__global__ void __launch_bounds__(GramVecShape<MP>::NT, 1) k_gram_vec(const float* __restrict__ x, long long nvec,
-                                                                    int M, long long ld, long long vchunk,
-                                                                    double* __restrict__ part) {
-  using S = GramVecShape<MP>;
-  constexpr bool CONV = ACC64 && !COL;    // stages converted to FP64 once
-  constexpr int NS = CONV ? 2 : GV_NS;    // FP32 stages
-  extern __shared__ __align__(16) float sm_gv[];
-  // floats per stage buffer: COL, MP component rows; otherwise VC vectors + MP words of slack
-  const int stage_f = COL ? MP * GV_VC : GV_VC * M + MP;
-  // CONV: VC x M doubles + MP of slack (rows >= M of the last vector read past its end)
-  double* dbuf = reinterpret_cast<double*>(sm_gv + NS * stage_f);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wb = warp % S::WB, ph = warp / S::WB;
-  const int r0 = (wb == 2 ? 32 : 0) + 8 * (lane >> 3);
-  const int c0 = (wb == 0 ? 0 : 32) + 4 * (lane & 7);
-  const long long vb = (long long)blockIdx.x * vchunk;
-  const long long ve = (vb + vchunk < nvec) ? vb + vchunk : nvec;
-  const long long nst = vb < ve ? (ve - vb + GV_VC - 1) / GV_VC : 0;
-
-  auto load = [&](long long st) {
-    const long long v0 = vb + st * GV_VC;
-    const int nv = (int)((ve - v0 < GV_VC) ? ve - v0 : GV_VC);
-    float* dst = sm_gv + (int)(st % NS) * stage_f;
-    if (COL) {
-      gv_load_col<S::NT>(dst, x, v0, nv, M, ld, tid);
-    } else {
-      const int n16 = nv * M / 4;
-      const float* src = x + v0 * M;
-      for (int f = tid; f < n16; f += S::NT) cp_async16(dst + 4 * f, src + 4 * f);
-    }
-  };
-
-  float acc[8][4];
-  double accd[8][4];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      acc[i][j] = 0.f;
-      accd[i][j] = 0.0;
-    }
-  int since = 0;
-#pragma unroll
-  for (int st = 0; st < NS - 1; ++st) {
-    if (st < nst) load(st);
-    cp_async_commit();
-  }
-  for (long long it = 0; it < nst; ++it) {
-    cp_async_wait<NS - 2>();
-    __syncthreads();  // stage `it` landed for every thread; stage it - 1 fully consumed
-    if (it + NS - 1 < nst) load(it + NS - 1);
-    cp_async_commit();
-    const float* buf = sm_gv + (int)(it % NS) * stage_f;
-    const long long v0 = vb + it * GV_VC;
-    const int nv = (int)((ve - v0 < GV_VC) ? ve - v0 : GV_VC);
-    if (CONV) {
-      // the stage in FP64, once (the previous stage's readers are past the barrier above)
-      for (int f = tid; f < nv * M; f += S::NT) dbuf[f] = (double)buf[f];
-      __syncthreads();
-      for (int v = ph; v < nv; v += S::WPB) {
-        const double* col = dbuf + v * M;
-        double av[8], bv[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const double2 t2 = *reinterpret_cast<const double2*>(col + r0 + 2 * i);
-          av[2 * i] = t2.x;
-          av[2 * i + 1] = t2.y;
-        }
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const double2 t2 = *reinterpret_cast<const double2*>(col + c0 + 2 * j);
-          bv[2 * j] = t2.x;
-          bv[2 * j + 1] = t2.y;
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) accd[i][j] = fma(av[i], bv[j], accd[i][j]);
-      }
-      continue;
-    }
-    for (int v = ph; v < nv; v += S::WPB) {
-      float av[8], bv[4];
-      if (COL) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) av[i] = buf[gv_col_at(r0 + i, v)];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) bv[j] = buf[gv_col_at(c0 + j, v)];
-      } else {
-        const float* col = buf + v * M;
-        const float4 a0 = *reinterpret_cast<const float4*>(col + r0);
-        const float4 a1 = *reinterpret_cast<const float4*>(col + r0 + 4);
-        const float4 b = *reinterpret_cast<const float4*>(col + c0);
-        av[0] = a0.x; av[1] = a0.y; av[2] = a0.z; av[3] = a0.w;
-        av[4] = a1.x; av[5] = a1.y; av[6] = a1.z; av[7] = a1.w;
-        bv[0] = b.x; bv[1] = b.y; bv[2] = b.z; bv[3] = b.w;
-      }
-      if (ACC64) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) accd[i][j] = fma((double)av[i], (double)bv[j], accd[i][j]);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-        if (++since == GV_VFLUSH) {
-          since = 0;
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              accd[i][j] += (double)acc[i][j];
-              acc[i][j] = 0.f;
-            }
-        }
-      }
-    }
-  }
-  cp_async_wait<0>();
-  __syncthreads();  // stage buffers free: reused for the cross-warp sum
-  if (!ACC64) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) accd[i][j] += (double)acc[i][j];
-  }
-  double* red = reinterpret_cast<double*>(sm_gv);  // [warp][32][32]
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) red[warp * 1024 + (8 * (lane >> 3) + i) * 32 + 4 * (lane & 7) + j] = accd[i][j];
-  __syncthreads();
-  double* dst = part + (long long)blockIdx.x * MP * MP;
-  for (int e = tid; e < S::WB * 1024; e += S::NT) {
-    const int b = e >> 10, rr = (e >> 5) & 31, cc = e & 31;
-    double t = 0.0;
-    for (int p = 0; p < S::WPB; ++p) t += red[(p * S::WB + b) * 1024 + rr * 32 + cc];
-    const int R = (b == 2 ? 32 : 0) + rr, Cc = (b == 0 ? 0 : 32) + cc;
-    dst[R * MP + Cc] = t;
-  }
-}
-
-static int gram_mp(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 48 ? 48 : M <= 64 ? 64 : 128; }
-
-static void gram_plan(long long nvec, int* nblk, long long* vchunk) {
-  const int target = 4 * num_sms();
-  long long vc = ceil_div_ll(nvec, target);
-  // at least 64 vectors per block: a few thousand vectors (the last unfoldings' Grams) still
-  // spread over tens of blocks instead of one
-  if (vc < 64) vc = 64;
-  vc = ceil_div_ll(vc, 32) * 32;
-  *vchunk = vc;
-  *nblk = (int)std::max<long long>(1, ceil_div_ll(nvec, vc));
-}
-
-// Symmetric variant for 17 <= M <= 32 components, either layout (the exact step's Gram of a long
-// unfolding with few rows; the power basis Z at widths up to 32): the upper triangle of 8 x 8
-// tiles of the 32 x 32 result (10 tiles)
-// times 3 vectors is 30 lanes of a warp, so a vector costs 640 FMAs instead of 1024 and a lane
-// loads 16 values per 64 FMAs.  8 warps of 3 vectors take 24 vectors per step of a stage.
-// FP32 products: the per-lane FP64 sums live in shared memory (row stride 65 doubles) next to
-// the stages, which keeps the registers to the FP32 tile; FP64 products: in registers.
-constexpr int GS_NT = 256;
-constexpr int GS_LD = 65;
-static size_t gram_sym_smem(int M, bool acc64, bool col) {
-  const size_t stages = (col ? (size_t)32 * GV_VC : (size_t)GV_VC * M + 32) * GV_NS * sizeof(float);
-  const size_t red = (size_t)GS_NT * GS_LD * sizeof(double);
-  return acc64 ? std::max(stages, red) : stages + red;
-}
-
-template <bool ACC64, bool COL>
-__global__ void __launch_bounds__(GS_NT, 1) k_gram_sym32(const float* __restrict__ x, long long nvec, int M,
-                                                        long long ld, long long vchunk, double* __restrict__ part) {
-  extern __shared__ __align__(16) float sm_gs[];
-  const int stage_f = COL ? 32 * GV_VC : GV_VC * M + 32;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int t = lane % 10, u = lane / 10;  // tile, vector of the triple (u == 3: idle lanes)
-  const int p = t < 4 ? 0 : t < 7 ? 1 : t < 9 ? 2 : 3;
-  const int q = t < 4 ? t : t < 7 ? t - 3 : t < 9 ? t - 5 : 3;
-  const long long vb = (long long)blockIdx.x * vchunk;
-  const long long ve = (vb + vchunk < nvec) ? vb + vchunk : nvec;
-  const long long nst = vb < ve ? (ve - vb + GV_VC - 1) / GV_VC : 0;
-  auto load = [&](long long st) {
-    const long long v0 = vb + st * GV_VC;
-    const int nv = (int)((ve - v0 < GV_VC) ? ve - v0 : GV_VC);
-    float* dst = sm_gs + (int)(st % GV_NS) * stage_f;
-    if (COL) {
-      gv_load_col<GS_NT>(dst, x, v0, nv, M, ld, tid);
-    } else {
-      const int n16 = nv * M / 4;
-      const float* src = x + v0 * M;
-      for (int f = tid; f < n16; f += GS_NT) cp_async16(dst + 4 * f, src + 4 * f);
-    }
-  };
-  // FP64 sums: registers (ACC64) or this thread's row of the shared block after the stages
-  double* sacc = reinterpret_cast<double*>(sm_gs + GV_NS * stage_f + ((GV_NS * stage_f) & 1)) + tid * GS_LD;
-  float acc[8][8];
-  double accd[ACC64 ? 8 : 1][ACC64 ? 8 : 1];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      acc[i][j] = 0.f;
-      if (ACC64) accd[ACC64 ? i : 0][ACC64 ? j : 0] = 0.0;
-    }
-  if (!ACC64)
-    for (int e = 0; e < 64; ++e) sacc[e] = 0.0;
-  auto flush = [&]() {
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        sacc[i * 8 + j] += (double)acc[i][j];
-        acc[i][j] = 0.f;
-      }
-  };
-  int since = 0;
-#pragma unroll
-  for (int st = 0; st < GV_NS - 1; ++st) {
-    if (st < nst) load(st);
-    cp_async_commit();
-  }
-  for (long long it = 0; it < nst; ++it) {
-    cp_async_wait<GV_NS - 2>();
-    __syncthreads();
-    if (it + GV_NS - 1 < nst) load(it + GV_NS - 1);
-    cp_async_commit();
-    const float* buf = sm_gs + (int)(it % GV_NS) * stage_f;
-    const long long v0 = vb + it * GV_VC;
-    const int nv = (int)((ve - v0 < GV_VC) ? ve - v0 : GV_VC);
-    if (u < 3) {
-      for (int v = 3 * warp + u; v < nv; v += 24) {
-        float av[8], bv[8];
-        if (COL) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            av[i] = buf[gv_col_at(8 * p + i, v)];
-            bv[i] = buf[gv_col_at(8 * q + i, v)];
-          }
-        } else {
-          const float* col = buf + v * M;
-          const float4 a0 = *reinterpret_cast<const float4*>(col + 8 * p);
-          const float4 a1 = *reinterpret_cast<const float4*>(col + 8 * p + 4);
-          const float4 b0 = *reinterpret_cast<const float4*>(col + 8 * q);
-          const float4 b1 = *reinterpret_cast<const float4*>(col + 8 * q + 4);
-          av[0] = a0.x; av[1] = a0.y; av[2] = a0.z; av[3] = a0.w;
-          av[4] = a1.x; av[5] = a1.y; av[6] = a1.z; av[7] = a1.w;
-          bv[0] = b0.x; bv[1] = b0.y; bv[2] = b0.z; bv[3] = b0.w;
-          bv[4] = b1.x; bv[5] = b1.y; bv[6] = b1.z; bv[7] = b1.w;
-        }
-        if (ACC64) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              accd[ACC64 ? i : 0][ACC64 ? j : 0] = fma((double)av[i], (double)bv[j], accd[ACC64 ? i : 0][ACC64 ? j : 0]);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-          if (++since == GV_VFLUSH) {
-            since = 0;
-            flush();
-          }
-        }
-      }
-    }
-  }
-  cp_async_wait<0>();
-  if (!ACC64) flush();
-  __syncthreads();  // stage buffers free (ACC64 writes its sums over them)
-  const double* red;  // [thread][GS_LD]
-  if (ACC64) {
-    double* r = reinterpret_cast<double*>(sm_gs);
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) r[tid * GS_LD + i * 8 + j] = accd[ACC64 ? i : 0][ACC64 ? j : 0];
-    red = r;
-  } else {
-    red = sacc - tid * GS_LD;
-  }
-  __syncthreads();
-  double* dst = part + (long long)blockIdx.x * 32 * 32;
-  for (int e = tid; e < 10 * 64; e += GS_NT) {
-    const int tt = e >> 6, ij = e & 63;
-    double sum = 0.0;
-    for (int w = 0; w < GS_NT / 32; ++w)
-      for (int uu = 0; uu < 3; ++uu) sum += red[(w * 32 + uu * 10 + tt) * GS_LD + ij];
-    const int pp = tt < 4 ? 0 : tt < 7 ? 1 : tt < 9 ? 2 : 3;
-    const int qq = tt < 4 ? tt : tt < 7 ? tt - 3 : tt < 9 ? tt - 5 : 3;
-    dst[(8 * pp + (ij >> 3)) * 32 + 8 * qq + (ij & 7)] = sum;
-  }
-}
-
-// Symmetric variant with FP64 products for 33 <= M <= 48 components (the Grams of B^T and of the
-// power basis Z at sketch widths 33..48), either layout: the upper triangle of TPM x TPM tiles
-// of 8 x 8 (15 tiles at TPM = 5, 21 at 6) times VPW = 32 / tiles vectors per warp, FP64 sums in
-// registers (a 40-wide vector costs 960 FMAs instead of the 3072 of three 32 x 32 warp blocks).
-template <int TPM, bool COL>
-__global__ void __launch_bounds__(GS_NT, 1) k_gram_symt(const float* __restrict__ x, long long nvec, int M,
-                                                       long long ld, long long vchunk, double* __restrict__ part) {
-  constexpr int MP = 8 * TPM;
-  constexpr int NTILE = TPM * (TPM + 1) / 2;
-  constexpr int VPW = 32 / NTILE;
-  extern __shared__ __align__(16) float sm_gt[];
-  const int stage_f = COL ? MP * GV_VC : GV_VC * M + MP;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int t = lane % NTILE, u = lane / NTILE;  // u >= VPW: idle lane
-  int p = 0, rem = t;
-  while (rem >= TPM - p) {
-    rem -= TPM - p;
-    ++p;
-  }
-  const int q = p + rem;
-  const long long vb = (long long)blockIdx.x * vchunk;
-  const long long ve = (vb + vchunk < nvec) ? vb + vchunk : nvec;
-  const long long nst = vb < ve ? (ve - vb + GV_VC - 1) / GV_VC : 0;
-  auto load = [&](long long st) {
-    const long long v0 = vb + st * GV_VC;
-    const int nv = (int)((ve - v0 < GV_VC) ? ve - v0 : GV_VC);
-    float* dst = sm_gt + (int)(st % GV_NS) * stage_f;
-    if (COL) {
-      gv_load_col<GS_NT>(dst, x, v0, nv, M, ld, tid);
-    } else {
-      const int n16 = nv * M / 4;
-      const float* src = x + v0 * M;
-      for (int f = tid; f < n16; f += GS_NT) cp_async16(dst + 4 * f, src + 4 * f);
-    }
-  };
-  double accd[8][8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) accd[i][j] = 0.0;
-#pragma unroll
-  for (int st = 0; st < GV_NS - 1; ++st) {
-    if (st < nst) load(st);
-    cp_async_commit();
-  }
-  for (long long it = 0; it < nst; ++it) {
-    cp_async_wait<GV_NS - 2>();
-    __syncthreads();
-    if (it + GV_NS - 1 < nst) load(it + GV_NS - 1);
-    cp_async_commit();
-    const float* buf = sm_gt + (int)(it % GV_NS) * stage_f;
-    const long long v0 = vb + it * GV_VC;
-    const int nv = (int)((ve - v0 < GV_VC) ? ve - v0 : GV_VC);
-    if (u < VPW) {
-      for (int v = VPW * warp + u; v < nv; v += VPW * (GS_NT / 32)) {
-        float av[8], bv[8];
-        if (COL) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            av[i] = buf[gv_col_at(8 * p + i, v)];
-            bv[i] = buf[gv_col_at(8 * q + i, v)];
-          }
-        } else {
-          const float* col = buf + v * M;
-          const float4 a0 = *reinterpret_cast<const float4*>(col + 8 * p);
-          const float4 a1 = *reinterpret_cast<const float4*>(col + 8 * p + 4);
-          const float4 b0 = *reinterpret_cast<const float4*>(col + 8 * q);
-          const float4 b1 = *reinterpret_cast<const float4*>(col + 8 * q + 4);
-          av[0] = a0.x; av[1] = a0.y; av[2] = a0.z; av[3] = a0.w;
-          av[4] = a1.x; av[5] = a1.y; av[6] = a1.z; av[7] = a1.w;
-          bv[0] = b0.x; bv[1] = b0.y; bv[2] = b0.z; bv[3] = b0.w;
-          bv[4] = b1.x; bv[5] = b1.y; bv[6] = b1.z; bv[7] = b1.w;
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j < 8; ++j) accd[i][j] = fma((double)av[i], (double)bv[j], accd[i][j]);
-      }
-    }
-  }
-  cp_async_wait<0>();
-  __syncthreads();  // stage buffers free: the per-lane sums go over them
-  double* red = reinterpret_cast<double*>(sm_gt);  // [thread][GS_LD]
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) red[tid * GS_LD + i * 8 + j] = accd[i][j];
-  __syncthreads();
-  double* dst = part + (long long)blockIdx.x * MP * MP;
-  for (int e = tid; e < NTILE * 64; e += GS_NT) {
-    const int tt = e >> 6, ij = e & 63;
-    double sum = 0.0;
-    for (int w = 0; w < GS_NT / 32; ++w)
-      for (int uu = 0; uu < VPW; ++uu) sum += red[(w * 32 + uu * NTILE + tt) * GS_LD + ij];
-    int pp = 0, rr = tt;
-    while (rr >= TPM - pp) {
-      rr -= TPM - pp;
-      ++pp;
-    }
-    const int qq = pp + rr;
-    dst[(8 * pp + (ij >> 3)) * MP + 8 * qq + (ij & 7)] = sum;
-  }
-}
-
-static size_t gram_symt_smem(int MP, int M, bool col) {
-  const size_t stages = (col ? (size_t)MP * GV_VC : (size_t)GV_VC * M + MP) * GV_NS * sizeof(float);
-  return std::max(stages, (size_t)GS_NT * GS_LD * sizeof(double));
-}
-
-// Vector Gram (k_gram_vec): taken for 17 <= M <= 64 and enough vectors to fill the GPU, with
-// x_j = x + j M (M % 4 == 0, 16-byte aligned base) or the column-major layout x[j + c es]
-// (vs = 1, es >= nvec).  Returns the block size MP (0: not taken), the grid and the vectors
-// per block.
-static int gram_vec_plan(const float* x, long long nvec, int M, long long vs, long long es, int* grid,
-                         long long* vchunk, bool* col) {
-  if (M < 17 || M > 64 || nvec < 8192) return 0;
-  *col = (vs == 1 && es >= nvec);
-  if (!*col) {
-    if (es != 1 || vs != M || (M & 3) != 0) return 0;
-    if (x && (reinterpret_cast<uintptr_t>(x) & 15) != 0) return 0;
-  }
-  const int MP = M <= 32 ? 32 : 64;
-  if (gram_vec_smem(MP, M, *col, true) > (size_t)max_optin_smem()) return 0;
-  const long long g = std::min<long long>((long long)num_sms(), ceil_div_ll(nvec, 4 * GV_VC));
-  long long vc = ceil_div_ll(nvec, g);
-  vc = ceil_div_ll(vc, GV_VC) * GV_VC;
-  *vchunk = vc;
-  *grid = (int)ceil_div_ll(nvec, vc);
-  return MP;
-}
-
-size_t gram_ws_bytes(long long nvec, int M) {
-  int nblk;
-  long long vc;
-  gram_plan(nvec, &nblk, &vc);
-  const int MP = gram_mp(M);
-  size_t b = (size_t)nblk * MP * MP * sizeof(double);
-  int g = 0;
-  bool col = false;
-  int MPv = gram_vec_plan(nullptr, nvec, M, M, 1, &g, &vc, &col);
-  if (MPv) b = std::max(b, (size_t)g * MPv * MPv * sizeof(double));
-  MPv = gram_vec_plan(nullptr, nvec, M, 1, nvec, &g, &vc, &col);
-  if (MPv) b = std::max(b, (size_t)g * MPv * MPv * sizeof(double));
-  return b + 4096;
-}
-
-int launch_gram(const float* x, long long nvec, int M, long long vs, long long es, double* w,
-                bool acc64, Arena& ws, cudaStream_t s) {
-  if (M <= 0) return TT_OK;
-  if (M > TT_MAX_SMALL) {
-    set_error(TT_ERR_UNSUPPORTED, "gram size %d > %d", M, TT_MAX_SMALL);
-    return TT_ERR_UNSUPPORTED;
-  }
-  int nblk;
-  long long vchunk;
-  {
-    bool col = false;
-    const int MPv = gram_vec_plan(x, nvec, M, vs, es, &nblk, &vchunk, &col);
-    if (MPv) {
-      const size_t mk = ws.mark();
-      double* part = ws.take<double>((size_t)nblk * MPv * MPv);
-      if (!part) {
-        set_error(TT_ERR_NOMEM, "gram workspace");
-        return TT_ERR_NOMEM;
-      }
-      const size_t shm = gram_vec_smem(MPv, M, col, acc64);
-      {
-        const int mx = max_optin_smem();
-#define GV_ATTR(MPV, A, C) smem_optin_k(k_gram_vec<MPV, A, C>, mx)
-        GV_ATTR(32, false, false); GV_ATTR(32, true, false); GV_ATTR(64, false, false); GV_ATTR(64, true, false);
-        GV_ATTR(32, false, true); GV_ATTR(32, true, true); GV_ATTR(64, false, true); GV_ATTR(64, true, true);
-#undef GV_ATTR
-      }
-      if (MPv == 32 && gram_sym_smem(M, acc64, col) <= (size_t)max_optin_smem()) {
-        {
-          const int mx = max_optin_smem();
-          smem_optin_k(k_gram_sym32<false, false>, mx);
-          smem_optin_k(k_gram_sym32<true, false>, mx);
-          smem_optin_k(k_gram_sym32<false, true>, mx);
-          smem_optin_k(k_gram_sym32<true, true>, mx);
-        }
-        const size_t sshm = gram_sym_smem(M, acc64, col);
-        const long long lds = col ? es : M;
-        if (col) {
-          if (acc64)
-            k_gram_sym32<true, true><<<nblk, GS_NT, sshm, s>>>(x, nvec, M, lds, vchunk, part);
-          else
-            k_gram_sym32<false, true><<<nblk, GS_NT, sshm, s>>>(x, nvec, M, lds, vchunk, part);
-        } else {
-          if (acc64)
-            k_gram_sym32<true, false><<<nblk, GS_NT, sshm, s>>>(x, nvec, M, lds, vchunk, part);
-          else
-            k_gram_sym32<false, false><<<nblk, GS_NT, sshm, s>>>(x, nvec, M, lds, vchunk, part);
-        }
-        count_launch();
-        TT_LAUNCH_CHECK();
-        launch_gram_reduce(part, nblk, 32, M, 8, w, s);
-        count_launch();
-        TT_LAUNCH_CHECK();
-        ws.reset(mk);
-        return TT_OK;
-      }
-      const long long ld = col ? es : M;
-      if (acc64 && M > 32 && M <= 48) {
-        const int MPs = M <= 40 ? 40 : 48;
-        const size_t tshm = gram_symt_smem(MPs, M, col);
-        if (tshm <= (size_t)max_optin_smem()) {
-          {
-            const int mx = max_optin_smem();
-            smem_optin_k(k_gram_symt<5, false>, mx);
-            smem_optin_k(k_gram_symt<5, true>, mx);
-            smem_optin_k(k_gram_symt<6, false>, mx);
-            smem_optin_k(k_gram_symt<6, true>, mx);
-          }
-          if (MPs == 40) {
-            if (col)
-              k_gram_symt<5, true><<<nblk, GS_NT, tshm, s>>>(x, nvec, M, ld, vchunk, part);
-            else
-              k_gram_symt<5, false><<<nblk, GS_NT, tshm, s>>>(x, nvec, M, ld, vchunk, part);
-          } else {
-            if (col)
-              k_gram_symt<6, true><<<nblk, GS_NT, tshm, s>>>(x, nvec, M, ld, vchunk, part);
-            else
-              k_gram_symt<6, false><<<nblk, GS_NT, tshm, s>>>(x, nvec, M, ld, vchunk, part);
-          }
-          count_launch();
-          TT_LAUNCH_CHECK();
-          launch_gram_reduce(part, nblk, MPs, M, 8, w, s);
-          count_launch();
-          TT_LAUNCH_CHECK();
-          ws.reset(mk);
-          return TT_OK;
-        }
-      }
-#define GV_LAUNCH(MPV, A, C) \
-  k_gram_vec<MPV, A, C><<<nblk, GramVecShape<MPV>::NT, shm, s>>>(x, nvec, M, ld, vchunk, part)
-      if (MPv == 32) {
-        if (col) {
-          if (acc64) GV_LAUNCH(32, true, true); else GV_LAUNCH(32, false, true);
-        } else {
-          if (acc64) GV_LAUNCH(32, true, false); else GV_LAUNCH(32, false, false);
-        }
-      } else {
-        if (col) {
-          if (acc64) GV_LAUNCH(64, true, true); else GV_LAUNCH(64, false, true);
-        } else {
-          if (acc64) GV_LAUNCH(64, true, false); else GV_LAUNCH(64, false, false);
-        }
-      }
-#undef GV_LAUNCH
-      count_launch();
-      TT_LAUNCH_CHECK();
-      launch_gram_reduce(part, nblk, MPv, M, 32, w, s);
-      count_launch();
-      TT_LAUNCH_CHECK();
-      ws.reset(mk);
-      return TT_OK;
-    }
-  }
-  gram_plan(std::max<long long>(nvec, 1), &nblk, &vchunk);
-  const int MP = gram_mp(M);
-  const size_t mk = ws.mark();
-  double* part = ws.take<double>((size_t)nblk * MP * MP);
-  if (!part) {
-    set_error(TT_ERR_NOMEM, "gram workspace");
-    return TT_ERR_NOMEM;
-  }
-#define GRAM_CASE(MPV)                                                                      \
-  case MPV:                                                                                 \
-    if (acc64)                                                                              \
-      k_gram<MPV, true><<<nblk, 256, 0, s>>>(x, nvec, M, vs, es, vchunk, part);             \
-    else                                                                                    \
-      k_gram<MPV, false><<<nblk, 256, 0, s>>>(x, nvec, M, vs, es, vchunk, part);            \
-    break;
-  switch (MP) {
-    GRAM_CASE(16)
-    GRAM_CASE(32)
-    GRAM_CASE(48)
-    GRAM_CASE(64)
-    GRAM_CASE(128)
-  }
-#undef GRAM_CASE
-  count_launch();
-  TT_LAUNCH_CHECK();
-  launch_gram_reduce(part, nblk, MP, M, 4, w, s);
-  count_launch();
-  TT_LAUNCH_CHECK();
-  ws.reset(mk);
-  return TT_OK;
-}
-
-static int max_optin_smem() { return dev_smem_max(); }
 
 // ---------------------------------------------------------------------------------------
 // Symmetric eigen-decomposition: parallel cyclic Jacobi (round-robin pairs), FP64

@@ -934,17 +934,6 @@ __global__ void __launch_bounds__(256, 1)
   }
 }
 
-// W (M x M, column-major) = sum over blocks of the upper-tile partials (fixed order).
-__global__ void k_gram32x_finish(const double* __restrict__ part, int nblk, int M, double* __restrict__ w) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < M * M; e += gridDim.x * blockDim.x) {
-    const int i = e % M, j = e / M;
-    const int r = i < j ? i : j, c = i < j ? j : i;
-    double sum = 0.0;
-    for (int b = 0; b < nblk; ++b) sum += part[(long long)b * 1024 + r * 32 + c];
-    w[e] = sum;
-  }
-}
-
 // Self-test of the bounded wait: one warp waits (with the pipeline limit and the abort-flag
 // path of the tensor-core kernels) on an mbarrier that nothing ever arrives at, and reports
 // TT_ERR_TIMEOUT through the status word when the limit runs out.  No copy or MMA is in flight,
@@ -1249,9 +1238,7 @@ int launch_gram32x(const float* x, long long nvec, int M, double* w, Arena& ws, 
   k_gram32x<<<grid, 256, G32_SMEM, s>>>(map, nvec, part, st);
   count_launch();
   TT_LAUNCH_CHECK();
-  k_gram32x_finish<<<ceil_div(M * M, 256), 256, 0, s>>>(part, grid, M, w);
-  count_launch();
-  TT_LAUNCH_CHECK();
+  TT_TRY(launch_gram32_reduce(part, grid, M, w, s));
   ws.reset(mk);
   return TT_OK;
 }

@@ -51,18 +51,18 @@ int launch_project(const float* a, long long m, long long n, const float* q, int
                    float* out, long long ldo, int mode, int r0, int r1, int engine, Arena& ws,
                    DevStatus* st, cudaStream_t s);
 
-// W (M x M, FP64, ld = M) = sum_j x_j x_j^T with x_j[c] = x[j*vs + c*es], M <= 128.
-// acc64: FP64 products and accumulation; else FP32 products with FP64 flush every 1024 vectors.
-int launch_gram(const float* x, long long nvec, int M, long long vs, long long es, double* w,
-                bool acc64, Arena& ws, cudaStream_t s);
+// W (M x M, FP64, ld = M) = sum_j x_j x_j^T with x_j[c] = x[j*vs + c*es], M <= 128; FP64 products.
+int launch_gram(const float* x, long long nvec, int M, long long vs, long long es, double* w, Arena& ws,
+                cudaStream_t s);
+// W (M x M, M <= 32) = sum of nblk partials of 32 x 32 (upper triangles) of the exact Grams below.
+int launch_gram32_reduce(const double* part, int nblk, int M, double* w, cudaStream_t s);
 
 // CholeskyQR2 on a tall FP32 matrix (n x N, column-major, ld), in place; y64 (or null): the matrix
 // in FP64 (ld = n), taken instead of y's contents.  Writes R (N x N, FP64, upper) when r != nullptr.
 int launch_cholqr2(const double* y64, float* y, long long n, int N, long long ld, double* r, Arena& ws,
                    cudaStream_t s);
-// One CholeskyQR pass (between power iterations): FP32-accumulated Gram, or FP64 products with
-// acc64 (graded spectra, whose small directions lie below the FP32 Gram's resolution).
-int launch_orth_power(float* y, long long n, int N, long long ld, Arena& ws, cudaStream_t s, bool acc64 = false);
+// One CholeskyQR pass (between power iterations).
+int launch_orth_power(float* y, long long n, int N, long long ld, Arena& ws, cudaStream_t s);
 
 // Arena bytes launch_syev takes for N > 64 (the rotation log); 0 for N <= 64.
 size_t syev_ws_bytes(int N, int max_sweeps);
@@ -153,6 +153,8 @@ int launch_expand_rows(const float* in, int Rin, float* out, int Rout, long long
 // TT_ERR_UNSUPPORTED (nothing launched) when the shape or device does not fit.
 size_t gram32x_ws_bytes();
 int launch_gram32x(const float* x, long long nvec, int M, double* w, Arena& ws, DevStatus* st, cudaStream_t s);
+// The same for any M <= 32 (16-byte aligned base), without the TMA; same scratch.
+int launch_gram32u(const float* x, long long nvec, int M, double* w, Arena& ws, cudaStream_t s);
 
 // Sketch variants that take their split-K scratch from the caller (no allocation).
 int launch_sketch_tc_static(const float* a, long long m, long long n, const float* w, int N,

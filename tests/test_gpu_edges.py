@@ -61,3 +61,49 @@ def test_cholqr2_edges(gpu, n, N):
     assert np.allclose(np.tril(rd, -1), 0.0) and np.all(np.diag(rd) > 0.0)
     q2, _ = _ttr().cholqr2(y, want_r=False)
     assert torch.equal(q, q2)  # R is a by-product: Q is the same with and without it
+
+
+@pytest.mark.parametrize("n,N", [(1, 1), (3, 7), (31, 8), (33, 9), (1000, 17), (128, 32), (129, 33), (20000, 31),
+                                 (65, 64), (40000, 65), (97, 128)])
+@pytest.mark.parametrize("layout", ["col", "row", "strided"])
+def test_gram_edges(gpu, n, N, layout):
+    """Chunk, tile and group remainders in either layout, and rows inside a wider matrix: FP64 products
+    of FP32 values are exact and the sums round at 2^-53 of the sum of magnitudes."""
+    import ctypes as C
+    import torch
+    ttr = _ttr()
+    rng = np.random.default_rng(n + N)
+    wide = rng.standard_normal((n, N + 3)).astype(np.float32)
+    z = torch.from_numpy(wide).to(gpu)
+    if layout == "col":
+        z = z[:, :N].t().contiguous()
+        rs, cs = 1, n
+    elif layout == "row":
+        z = z[:, :N].contiguous()
+        rs, cs = N, 1
+    else:
+        rs, cs = N + 3, 1
+    w = torch.empty((N, N), dtype=torch.float64, device=gpu)
+    ttr._lib.check(ttr.lib().tt_k_gram_tall(ttr._ctx_for(0), C.c_void_p(z.data_ptr()), n, N, rs, cs,
+                                            C.c_void_p(w.data_ptr())))
+    ref = wide[:, :N].astype(np.float64)
+    bound = n * 2.0 ** -53 * (np.abs(ref).T @ np.abs(ref)) + 1e-300
+    assert np.all(np.abs(w.cpu().numpy() - ref.T @ ref) <= 2 * bound)
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 5, 6, 17, 30, 31])
+@pytest.mark.parametrize("n", [1, 47, 48, 49, 100003])
+def test_gram_rows_unaligned(gpu, m, n):
+    """Unfoldings of up to 32 rows whose columns the TMA cannot address (through the decomposition's own
+    rule: an exact step of tt_svd): sigma against NumPy."""
+    import torch
+    ttr = _ttr()
+    rng = np.random.default_rng(m * n)
+    a = rng.standard_normal((m, n)).astype(np.float32)
+    r = min(m, n)
+    res = ttr.tt_svd(_dev(a, gpu), [1, r, 1])
+    ref = np.linalg.svd(a.astype(np.float64), compute_uv=False)
+    # FP32 products and 64-term sums: the Gram is within 64 u of its entries' magnitudes
+    tol = 64 * U32 * m * ref[0] ** 2
+    assert np.all(np.abs(res.sigmas[0][:r].astype(np.float64) ** 2 - ref[:r] ** 2) <= tol)
+    del torch
