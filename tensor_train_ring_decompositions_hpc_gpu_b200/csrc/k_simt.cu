@@ -1,6 +1,5 @@
-// CUDA-core kernels: the plain-FP32 GEMM engine and every small linear-algebra kernel of the
-// TT/TR-SVD chain (Gaussian test matrix, Jacobi eigen-solver,
-// bond permute, core folding, reconstruction error).
+// CUDA-core kernels of the TT/TR-SVD chain: Gaussian test matrix, Jacobi eigen-solvers, bond permute,
+// core folding, reconstruction error and the small helpers between them.
 #include <float.h>
 #include <stdlib.h>
 #include <math.h>
@@ -96,650 +95,6 @@ int launch_gaussian(float* out, long long rows, int cols, long long ld, unsigned
   k_gaussian<<<grid, 256, 0, s>>>(out, rows, total, ld, seed, stream_id);
   count_launch();
   TT_LAUNCH_CHECK();
-  return TT_OK;
-}
-
-// ---------------------------------------------------------------------------------------
-// Plain-FP32 sketch  Y = A * W  (split over the long dimension n, FP64 reduction of splits)
-// ---------------------------------------------------------------------------------------
-// 32 x RI rows of A per block (RI per thread) x NT sketch columns (NT / 8 per thread); narrow
-// sketches (NT <= 24) take RI = 16 rows per thread, so that each shared-memory load feeds more
-// FMAs.  The long dimension runs in chunks of JC columns of A (32 KB of A per chunk) streamed
-// through a 3-stage shared-memory ring by cp.async (two chunks in flight while the third is
-// multiplied: the loads need no registers), one barrier per chunk.  Products by paired FP32 FMAs
-// (fma.rn.f32x2, each lane rounded like fmaf), the row pairs straight from 16-byte shared loads;
-// W's rows are padded to NT + 1 words so its copies (JC consecutive rows per warp) hit distinct
-// banks.  Split partials are written in FP64.
-constexpr int kSkStages = 3;
-template <int NT>
-struct SkTile {
-  static constexpr int RI = NT <= 24 ? 16 : 8;  // rows per thread
-  static constexpr int TI = 32 * RI;             // rows per block
-  static constexpr int JC = 8192 / TI;           // columns of A per chunk (TI x JC = 8192 floats)
-  static constexpr int NTP = NT + 1;             // padded row of W in shared memory
-  static constexpr size_t smem = (size_t)kSkStages * (TI * JC + JC * NTP) * sizeof(float);
-};
-template <int NT>
-constexpr size_t sk_smem() { return SkTile<NT>::smem; }
-
-template <int NT>
-__global__ void __launch_bounds__(256, NT >= 40 ? 1 : 2) k_sketch_simt(const float* __restrict__ a, long long m,
-                                                                       long long n, const float* __restrict__ w,
-                                                                       int N, long long wj, long long wc,
-                                                                       long long jchunk, int cblk,
-                                                                       double* __restrict__ part) {
-  using T = SkTile<NT>;
-  constexpr int RI = T::RI, TI = T::TI, JC = T::JC, NTP = T::NTP, RC = NT / 8;
-  constexpr int AV = (TI * JC / 4) / 256;     // 16-byte copies of A per thread per chunk
-  constexpr int WV = (JC * NT + 255) / 256;   // W values per thread per chunk
-  extern __shared__ __align__(16) float sm_sk[];
-  float* as_base = sm_sk;                            // [ST][JC][TI]
-  float* ws_base = sm_sk + kSkStages * JC * TI;      // [ST][JC][NTP]
-  const int tid = threadIdx.x;
-  const long long i0 = (long long)blockIdx.x * TI;
-  const int split = blockIdx.y;
-  const int c0 = blockIdx.z * NT;
-  const long long jb = (long long)split * jchunk;
-  const long long je = (jb + jchunk < n) ? jb + jchunk : n;
-  const int ti = tid >> 3, tc = tid & 7;
-  // accumulators paired over rows: acc2[p][c] = (acc[2p][c], acc[2p + 1][c])
-  uint64_t acc2[RI / 2][RC];
-#pragma unroll
-  for (int e = 0; e < RI / 2; ++e)
-#pragma unroll
-    for (int c = 0; c < RC; ++c) acc2[e][c] = 0ull;
-  const bool vec = ((m & 3) == 0) && ((((uintptr_t)a) & 15) == 0);
-  const int nchunks = je > jb ? (int)((je - jb + JC - 1) / JC) : 0;
-  // Copies of chunk t into ring slot t % ST (one commit group per chunk, empty past the end).
-  auto fill = [&](int t) {
-    if (t < nchunks) {
-      const long long j0 = jb + (long long)t * JC;
-      float* as = as_base + (t % kSkStages) * JC * TI;
-      float* wsm = ws_base + (t % kSkStages) * JC * NTP;
-#pragma unroll
-      for (int q = 0; q < AV; ++q) {
-        const int f = tid + 256 * q;
-        const int jj = f / (TI / 4), i4 = f % (TI / 4);
-        const long long j = j0 + jj, i = i0 + 4 * i4;
-        float* dst = &as[jj * TI + 4 * i4];
-        const float* src = a + j * m + i;
-        if (j < je && vec && i + 3 < m) {
-          cp_async16(dst, src);
-        } else {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const bool ok = j < je && i + e < m;
-            cp_async4(dst + e, ok ? src + e : a, ok);
-          }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < WV; ++u) {
-        const int f = tid + 256 * u;
-        if (f < JC * NT) {
-          int jj, c;
-          if (wc == 1) {
-            c = f % NT;
-            jj = f / NT;
-          } else {
-            jj = f % JC;
-            c = f / JC;
-          }
-          const long long j = j0 + jj;
-          const bool ok = j < je && c0 + c < N;
-          cp_async4(&wsm[jj * NTP + c], ok ? w + j * wj + (long long)(c0 + c) * wc : w, ok);
-        }
-      }
-    }
-    cp_async_commit();
-  };
-  fill(0);
-  fill(1);
-  for (int t = 0; t < nchunks; ++t) {
-    cp_async_wait<kSkStages - 2>();  // this thread's copies of chunk t have landed
-    __syncthreads();                 // everyone's have; slot (t + 2) % ST was last read at t - 1
-    fill(t + 2);
-    const float* as = as_base + (t % kSkStages) * JC * TI;
-    const float* wsm = ws_base + (t % kSkStages) * JC * NTP;
-#pragma unroll
-    for (int jj = 0; jj < JC; ++jj) {
-      uint64_t xp[RI / 2];
-#pragma unroll
-      for (int q = 0; q < RI / 4; ++q) {
-        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(&as[jj * TI + ti * RI + 4 * q]);
-        xp[2 * q] = x.x;
-        xp[2 * q + 1] = x.y;
-      }
-#pragma unroll
-      for (int c = 0; c < RC; ++c) {
-        const uint64_t wd = f2_dup(wsm[jj * NTP + tc * RC + c]);
-#pragma unroll
-        for (int e = 0; e < RI / 2; ++e) ffma2(acc2[e][c], xp[e], wd);
-      }
-    }
-  }
-  cp_async_wait<0>();
-#pragma unroll
-  for (int e = 0; e < RI; ++e) {
-    const long long i = i0 + ti * RI + e;
-#pragma unroll
-    for (int c = 0; c < RC; ++c) {
-      const int col = c0 + tc * RC + c;
-      float lo, hi;
-      f2_unpack(acc2[e >> 1][c], lo, hi);
-      if (i < m && col < N) part[((long long)split * N + col) * m + i] = (double)((e & 1) ? hi : lo);
-    }
-  }
-  (void)cblk;
-}
-
-// Launch of k_sketch_simt with the tile width covering N (multiples of 8 up to 64; wider N
-// takes several column blocks of 64).
-static void launch_sketch_simt_kernel(const float* a, long long m, long long n, const float* w, int N, long long wj,
-                                      long long wc, long long jchunk, int nsplit, double* part, cudaStream_t s) {
-  const int NT = N <= 16 ? 16 : N <= 24 ? 24 : N <= 32 ? 32 : N <= 40 ? 40 : N <= 48 ? 48 : 64;
-  const int cblk = ceil_div(N, NT);
-  const int TI = NT <= 24 ? SkTile<16>::TI : SkTile<64>::TI;
-  dim3 grid(ceil_div(m, TI), nsplit, cblk);
-  const size_t shm = NT == 16 ? sk_smem<16>() : NT == 24 ? sk_smem<24>() : NT == 32 ? sk_smem<32>()
-                   : NT == 40 ? sk_smem<40>() : NT == 48 ? sk_smem<48>() : sk_smem<64>();
-#define SK_ATTR(V) smem_optin_k(k_sketch_simt<V>, sk_smem<V>())
-  SK_ATTR(16); SK_ATTR(24); SK_ATTR(32); SK_ATTR(40); SK_ATTR(48); SK_ATTR(64);
-#undef SK_ATTR
-#define SK_CASE(V) \
-  case V: k_sketch_simt<V><<<grid, 256, shm, s>>>(a, m, n, w, N, wj, wc, jchunk, cblk, part); break;
-  switch (NT) {
-    SK_CASE(16)
-    SK_CASE(24)
-    SK_CASE(32)
-    SK_CASE(40)
-    SK_CASE(48)
-    default: k_sketch_simt<64><<<grid, 256, shm, s>>>(a, m, n, w, N, wj, wc, jchunk, cblk, part); break;
-  }
-#undef SK_CASE
-}
-
-// Sum of nsplit partial blocks: each 256-thread block owns 32 consecutive outputs, its 8 warps
-// read interleaved splits (coalesced 256-byte rows, several loads in flight per lane) and the
-// 8 warp sums are added in a fixed order, so the result does not depend on scheduling.
-__global__ void __launch_bounds__(256) k_reduce_splits(const double* __restrict__ part, long long count,
-                                                       int nsplit, double* __restrict__ y) {
-  __shared__ double red[8][33];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (long long base = (long long)blockIdx.x * 32; base < count; base += (long long)gridDim.x * 32) {
-    const long long idx = base + lane;
-    double s0 = 0.0, s1 = 0.0;
-    if (idx < count) {
-      int k = warp;
-      for (; k + 8 < nsplit; k += 16) {
-        s0 += part[(long long)k * count + idx];
-        s1 += part[(long long)(k + 8) * count + idx];
-      }
-      if (k < nsplit) s0 += part[(long long)k * count + idx];
-    }
-    red[warp][lane] = s0 + s1;
-    __syncthreads();
-    if (warp == 0 && idx < count) {
-      double t = 0.0;
-#pragma unroll
-      for (int w = 0; w < 8; ++w) t += red[w][lane];
-      y[idx] = t;
-    }
-    __syncthreads();
-  }
-}
-
-static void sketch_split_plan(long long m, long long n, long long* jchunk, int* nsplit) {
-  const int mtiles = ceil_div(m, 256);
-  const int target = 4 * num_sms();
-  long long splits = std::max<long long>(1, target / std::max(1, mtiles));
-  long long jc = ceil_div_ll(n, splits);
-  if (jc < 256) jc = 256;
-  jc = ceil_div_ll(jc, 32) * 32;
-  *jchunk = jc;
-  *nsplit = (int)ceil_div_ll(n, jc);
-}
-
-size_t sketch_ws_bytes(long long m, long long n, int N) {
-  long long jchunk;
-  int nsplit;
-  sketch_split_plan(m, n, &jchunk, &nsplit);
-  const size_t simt = (size_t)nsplit * (size_t)N * (size_t)m * sizeof(double) + 4096;
-  return std::max(simt, sketch_tc_ws_bytes(m, n, N));
-}
-
-int launch_reduce_splits(const double* part, long long count, int nsplit, double* y, cudaStream_t s) {
-  if (count <= 0) return TT_OK;
-  k_reduce_splits<<<(int)std::min<long long>(ceil_div_ll(count, 32), 16LL * num_sms()), 256, 0, s>>>(
-      part, count, nsplit, y);
-  count_launch();
-  TT_LAUNCH_CHECK();
-  return TT_OK;
-}
-
-int launch_sketch(const float* a, long long m, long long n, const float* w, int N, long long wj,
-                  long long wc, double* y, int engine, Arena& ws, DevStatus* st, cudaStream_t s) {
-  if (m <= 0 || n <= 0 || N <= 0) return TT_OK;
-  if (engine == TT_GEMM_TC) {
-    int rc = launch_sketch_tc(a, m, n, w, N, wj, wc, y, ws, st, s);
-    if (rc != TT_ERR_UNSUPPORTED) return rc;
-  }
-  long long jchunk;
-  int nsplit;
-  sketch_split_plan(m, n, &jchunk, &nsplit);
-  const size_t mk = ws.mark();
-  double* part = ws.take<double>((size_t)nsplit * N * m);
-  if (!part) {
-    set_error(TT_ERR_NOMEM, "sketch workspace");
-    return TT_ERR_NOMEM;
-  }
-  launch_sketch_simt_kernel(a, m, n, w, N, wj, wc, jchunk, nsplit, part, s);
-  count_launch();
-  TT_LAUNCH_CHECK();
-  TT_TRY(launch_reduce_splits(part, (long long)N * m, nsplit, y, s));
-  ws.reset(mk);
-  return TT_OK;
-}
-
-// FP32 sketch with the split partials in caller-provided scratch (`part`, `part_cap` doubles);
-// the split count is lowered until the partials fit.  Allocates nothing.
-int launch_sketch_simt_static(const float* a, long long m, long long n, const float* w, int N,
-                              long long wj, long long wc, double* y, double* part, size_t part_cap,
-                              cudaStream_t s) {
-  if (m <= 0 || n <= 0 || N <= 0) return TT_OK;
-  long long jchunk;
-  int nsplit;
-  sketch_split_plan(m, n, &jchunk, &nsplit);
-  const long long max_ns = (long long)(part_cap / ((size_t)N * (size_t)m));
-  if (max_ns < 1) {
-    set_error(TT_ERR_SHAPE, "sketch partials of %lld x %d doubles exceed the scratch of %zu doubles", m, N,
-              part_cap);
-    return TT_ERR_SHAPE;
-  }
-  if (nsplit > max_ns) {
-    jchunk = (n + max_ns - 1) / max_ns;
-    jchunk = (jchunk + 31) / 32 * 32;
-    nsplit = (int)((n + jchunk - 1) / jchunk);
-  }
-  launch_sketch_simt_kernel(a, m, n, w, N, wj, wc, jchunk, nsplit, part, s);
-  count_launch();
-  TT_LAUNCH_CHECK();
-  return launch_reduce_splits(part, (long long)N * m, nsplit, y, s);
-}
-
-// ---------------------------------------------------------------------------------------
-// Plain-FP32 projection  out = A^T Q  (A column-major m x n, contraction over m)
-// ---------------------------------------------------------------------------------------
-__device__ __forceinline__ int swz(int row, int col) { return col ^ (((row >> 2) & 7) << 2); }
-
-// 256 columns of A per block (8 per thread) x NT outputs (NT / 8 per thread), K in chunks of
-// 32: the next chunk is loaded into registers while the current one is multiplied out of
-// shared memory (two buffers, one barrier per chunk).
-template <int NT>
-__global__ void __launch_bounds__(256, NT >= 64 ? 1 : 2) k_project_simt(const float* __restrict__ a, long long m,
-                                                                        long long n, const float* __restrict__ q,
-                                                                        int N, long long ldq, float* __restrict__ out,
-                                                                        long long ldo, int mode, int r0, int r1,
-                                                                        long long kchunk) {
-  constexpr int TJ = 256, KC = 32, RJ = 8, RC = NT / 8;
-  constexpr int AV = (TJ * KC / 4) / 256;    // float4 loads of A per thread per chunk
-  constexpr int QV = (KC * NT + 255) / 256;  // Q values per thread per chunk
-  extern __shared__ __align__(16) float sm_ps[];
-  float* as_base = sm_ps;                // [2][KC][TJ]
-  float* qs_base = sm_ps + 2 * KC * TJ;  // [2][KC][NT]
-  const int tid = threadIdx.x;
-  const long long j0 = (long long)blockIdx.x * TJ;
-  const int c0 = blockIdx.y * NT;
-  const int tj = tid >> 3, tc = tid & 7;
-  // accumulators paired over output rows (fma.rn.f32x2), as in k_sketch_simt
-  uint64_t acc2[RJ / 2][RC];
-#pragma unroll
-  for (int e = 0; e < RJ / 2; ++e)
-#pragma unroll
-    for (int c = 0; c < RC; ++c) acc2[e][c] = 0ull;
-  const bool vec = ((m & 3) == 0) && ((((uintptr_t)a) & 15) == 0);
-  // K range of this split (blockIdx.z); the split's output block is out + z * n * ldo.
-  const long long kb = (long long)blockIdx.z * kchunk;
-  const long long ke = (kb + kchunk < m) ? kb + kchunk : m;
-  out += (long long)blockIdx.z * n * ldo;
-  float4 ra[AV];
-  float rq[QV];
-  auto fetch = [&](long long k0) {
-#pragma unroll
-    for (int qq = 0; qq < AV; ++qq) {
-      const int f = tid + 256 * qq;
-      const int jj = f >> 3, k4 = f & 7;
-      const long long j = j0 + jj, k = k0 + 4 * k4;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (j < n) {
-        const float* p = a + j * m + k;
-        if (vec && k + 3 < ke) {
-          v = __ldg(reinterpret_cast<const float4*>(p));
-        } else {
-          if (k < ke) v.x = p[0];
-          if (k + 1 < ke) v.y = p[1];
-          if (k + 2 < ke) v.z = p[2];
-          if (k + 3 < ke) v.w = p[3];
-        }
-      }
-      ra[qq] = v;
-    }
-#pragma unroll
-    for (int u = 0; u < QV; ++u) {
-      const int f = tid + 256 * u;
-      const int kk = f % KC, c = f / KC;
-      const long long k = k0 + kk;
-      rq[u] = (f < KC * NT && k < ke && c0 + c < N) ? q[k + ldq * (long long)(c0 + c)] : 0.f;
-    }
-  };
-  auto stash = [&](int b) {
-    float* as = as_base + b * KC * TJ;
-    float* qs = qs_base + b * KC * NT;
-#pragma unroll
-    for (int qq = 0; qq < AV; ++qq) {
-      const int f = tid + 256 * qq;
-      const int jj = f >> 3, kk = 4 * (f & 7);
-      as[(kk + 0) * TJ + swz(kk + 0, jj)] = ra[qq].x;
-      as[(kk + 1) * TJ + swz(kk + 1, jj)] = ra[qq].y;
-      as[(kk + 2) * TJ + swz(kk + 2, jj)] = ra[qq].z;
-      as[(kk + 3) * TJ + swz(kk + 3, jj)] = ra[qq].w;
-    }
-#pragma unroll
-    for (int u = 0; u < QV; ++u) {
-      const int f = tid + 256 * u;
-      if (f < KC * NT) qs[(f % KC) * NT + f / KC] = rq[u];
-    }
-  };
-  if (kb < ke) {
-    fetch(kb);
-    stash(0);
-  }
-  __syncthreads();
-  int b = 0;
-  for (long long k0 = kb; k0 < ke; k0 += KC) {
-    const bool more = k0 + KC < ke;
-    if (more) fetch(k0 + KC);
-    const float* as = as_base + b * KC * TJ;
-    const float* qs = qs_base + b * KC * NT;
-#pragma unroll
-    for (int kk = 0; kk < KC; ++kk) {
-      const ulonglong2 x0 = *reinterpret_cast<const ulonglong2*>(&as[kk * TJ + swz(kk, tj * RJ)]);
-      const ulonglong2 x1 = *reinterpret_cast<const ulonglong2*>(&as[kk * TJ + swz(kk, tj * RJ + 4)]);
-      const uint64_t xp[4] = {x0.x, x0.y, x1.x, x1.y};
-#pragma unroll
-      for (int c = 0; c < RC; ++c) {
-        const uint64_t qd = f2_dup(qs[kk * NT + tc * RC + c]);
-#pragma unroll
-        for (int e = 0; e < RJ / 2; ++e) ffma2(acc2[e][c], xp[e], qd);
-      }
-    }
-    if (more) stash(b ^ 1);
-    __syncthreads();
-    b ^= 1;
-  }
-#pragma unroll
-  for (int e = 0; e < RJ; ++e) {
-    const long long j = j0 + tj * RJ + e;
-    if (j >= n) continue;
-#pragma unroll
-    for (int c = 0; c < RC; ++c) {
-      const int col = c0 + tc * RC + c;
-      if (col >= N) continue;
-      float lo, hi;
-      f2_unpack(acc2[e >> 1][c], lo, hi);
-      const float v = (e & 1) ? hi : lo;
-      if (mode == OUT_ROWMAJOR) {
-        out[j * ldo + col] = v;
-      } else if (mode == OUT_COLMAJOR) {
-        out[j + ldo * col] = v;
-      } else {
-        const int ai = col % r0, bi = col / r0;
-        out[(long long)bi + (long long)r1 * (j + n * (long long)ai)] = v;
-      }
-    }
-  }
-}
-
-// Small-K projection out = Q^T A for K = m <= 64 (the rotation E_r^T B of a small factor, or
-// an m <= 64 unfolding).  A's columns are contiguous, so a tile of TJ columns is one contiguous
-// block: it is staged through shared memory with coalesced float4 loads (odd row stride,
-// conflict-free), Q sits in shared memory as float4 rows, and each column's NP outputs are
-// computed by SPLIT threads (NP / SPLIT each, which keeps registers low enough for several
-// blocks per SM).  Row-major outputs and the TR bond permute leave through shared memory as
-// contiguous runs.
-template <int NP, int SPLIT>
-__global__ void __launch_bounds__(256) k_proj_smallk(const float* __restrict__ a, int m, long long n,
-                                                     const float* __restrict__ q, int N, long long ldq,
-                                                     float* __restrict__ out, long long ldo, int mode,
-                                                     int r0, int r1) {
-  constexpr int TJ = 256 / SPLIT;   // columns per tile
-  constexpr int NPT = NP / SPLIT;   // outputs per thread
-  static_assert(NPT % 4 == 0, "outputs per thread");
-  extern __shared__ __align__(16) float sm_pk[];
-  float* Es = sm_pk;            // m x NP: Es[k * NP + c] = Q[k + ldq c]
-  float* Xs = Es + 64 * NP;     // TJ x S input tile, then TJ x (NP + 1) output tile
-  const int S = (m & 1) ? m : m + 1;
-  constexpr int OS = NP + 1;
-  const int tid = threadIdx.x;
-  const int col_t = tid % TJ, grp = tid / TJ;
-  for (int idx = tid; idx < m * NP; idx += 256) {
-    const int k = idx / NP, c = idx - (idx / NP) * NP;
-    Es[idx] = (c < N) ? q[k + ldq * (long long)c] : 0.f;
-  }
-  const bool vec = (m & 3) == 0 && ((reinterpret_cast<uintptr_t>(a) & 15) == 0);
-  // Row-major outputs with ldo == N form one contiguous block per tile; bond-permuted outputs
-  // (r0, r1, n) -> (r1, n, r0) form r0 contiguous runs of r1 * nj values per tile.
-  const bool staged_out = (mode == OUT_ROWMAJOR && ldo == N) || (mode == OUT_PERM231 && r0 * r1 == N);
-  // Quotients of tile-local indices (< 2^15) by m, N or r1 (<= 128) through a float reciprocal:
-  // the rounding error is far below the 0.5 / divisor margin, so the floor is exact.
-  const float inv_m = 1.0f / (float)m, inv_n = 1.0f / (float)N, inv_r1 = 1.0f / (float)(r1 > 0 ? r1 : 1);
-  auto qdiv = [](int e, float inv) { return (int)(((float)e + 0.5f) * inv); };
-  for (long long tile = blockIdx.x; tile * TJ < n; tile += gridDim.x) {
-    const long long j0 = tile * TJ;
-    const int nj = (int)((n - j0 < TJ) ? n - j0 : TJ);
-    const float* src = a + j0 * m;
-    const int cnt = nj * m;
-    __syncthreads();
-    if (vec) {
-      for (int f4 = tid; f4 < (cnt >> 2); f4 += 256) {
-        const float4 v = __ldg(reinterpret_cast<const float4*>(src) + f4);
-        const int e = 4 * f4, col = qdiv(e, inv_m), k = e - col * m;
-        float* d = Xs + col * S + k;
-        d[0] = v.x;
-        d[1] = v.y;
-        d[2] = v.z;
-        d[3] = v.w;
-      }
-    } else {
-      for (int f = tid; f < cnt; f += 256) {
-        const int col = qdiv(f, inv_m), k = f - col * m;
-        Xs[col * S + k] = __ldg(src + f);
-      }
-    }
-    __syncthreads();
-    float acc[NPT];
-#pragma unroll
-    for (int c = 0; c < NPT; ++c) acc[c] = 0.f;
-    if (col_t < nj) {
-      const float* xr = Xs + col_t * S;
-      for (int k = 0; k < m; ++k) {
-        const float x = xr[k];
-        const float4* er = reinterpret_cast<const float4*>(Es + k * NP + grp * NPT);
-#pragma unroll
-        for (int c4 = 0; c4 < NPT / 4; ++c4) {
-          const float4 e = er[c4];
-          acc[4 * c4] = fmaf(x, e.x, acc[4 * c4]);
-          acc[4 * c4 + 1] = fmaf(x, e.y, acc[4 * c4 + 1]);
-          acc[4 * c4 + 2] = fmaf(x, e.z, acc[4 * c4 + 2]);
-          acc[4 * c4 + 3] = fmaf(x, e.w, acc[4 * c4 + 3]);
-        }
-      }
-    }
-    if (staged_out) {
-      __syncthreads();
-      if (col_t < nj) {
-#pragma unroll
-        for (int c = 0; c < NPT; ++c)
-          if (grp * NPT + c < N) Xs[col_t * OS + grp * NPT + c] = acc[c];
-      }
-      __syncthreads();
-      if (mode == OUT_ROWMAJOR) {
-        float* dst = out + j0 * N;
-        for (int f = tid; f < nj * N; f += 256) {
-          const int col = qdiv(f, inv_n), c = f - col * N;
-          dst[f] = Xs[col * OS + c];
-        }
-      } else {
-        const int run = r1 * nj;
-        for (int ai = 0; ai < r0; ++ai) {
-          float* dst = out + (long long)r1 * (j0 + n * (long long)ai);
-          for (int f = tid; f < run; f += 256) {
-            const int col = qdiv(f, inv_r1), bi = f - col * r1;
-            dst[f] = Xs[col * OS + ai + r0 * bi];
-          }
-        }
-      }
-    } else if (col_t < nj) {
-      const long long j = j0 + col_t;
-#pragma unroll
-      for (int cc = 0; cc < NPT; ++cc) {
-        const int c = grp * NPT + cc;
-        if (c >= N) continue;
-        if (mode == OUT_ROWMAJOR) {
-          out[j * ldo + c] = acc[cc];
-        } else if (mode == OUT_COLMAJOR) {
-          out[j + ldo * c] = acc[cc];
-        } else {
-          const int ai = c % r0, bi = c / r0;
-          out[(long long)bi + (long long)r1 * (j + n * (long long)ai)] = acc[cc];
-        }
-      }
-    }
-  }
-}
-
-// Sum of the K-split partial projections (row-major n x N blocks) into the requested layout.
-__global__ void k_project_reduce(const float* __restrict__ part, long long n, int N, int nsplit,
-                                 float* __restrict__ out, long long ldo, int mode, int r0, int r1) {
-  const long long total = n * N;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    float v = 0.f;
-    for (int z = 0; z < nsplit; ++z) v += part[(long long)z * total + idx];
-    const long long j = idx / N;
-    const int c = (int)(idx - j * N);
-    if (mode == OUT_ROWMAJOR) {
-      out[j * ldo + c] = v;
-    } else if (mode == OUT_COLMAJOR) {
-      out[j + ldo * c] = v;
-    } else {
-      const int ai = c % r0, bi = c / r0;
-      out[(long long)bi + (long long)r1 * (j + n * (long long)ai)] = v;
-    }
-  }
-}
-
-namespace {
-constexpr size_t kProjectSplitCap = 16u << 20;  // bytes of K-split partials
-
-// K splits for projections whose column tiles alone cannot fill the GPU.
-int project_ksplit(long long m, long long n, int N, long long* kchunk) {
-  const int NT = N <= 16 ? 16 : N <= 32 ? 32 : N <= 48 ? 48 : 64;
-  const long long blocks = ceil_div_ll(n, 256) * ceil_div_ll(N, NT);
-  int ks = 1;
-  if (m >= 256 && blocks < 2LL * num_sms()) {
-    ks = (int)std::min<long long>(ceil_div_ll(2LL * num_sms(), blocks), m / 64);
-    const long long cap = (long long)(kProjectSplitCap / (sizeof(float) * (size_t)n * N));
-    ks = (int)std::max<long long>(1, std::min<long long>(ks, cap));
-  }
-  long long kc = ceil_div_ll(m, ks);
-  kc = ceil_div_ll(kc, 32) * 32;
-  *kchunk = kc;
-  return (int)ceil_div_ll(m, kc);
-}
-}  // namespace
-
-size_t project_ws_bytes(long long m, long long n, int N) {
-  long long kc;
-  const int ks = project_ksplit(m, n, N, &kc);
-  const size_t split = ks > 1 ? (size_t)ks * n * N * sizeof(float) : 0;
-  return split + 2 * (size_t)m * N * sizeof(float) + 4096;
-}
-
-int launch_project(const float* a, long long m, long long n, const float* q, int N, long long ldq,
-                   float* out, long long ldo, int mode, int r0, int r1, int engine, Arena& ws,
-                   DevStatus* st, cudaStream_t s) {
-  if (n <= 0 || N <= 0) return TT_OK;
-  if (engine == TT_GEMM_TC) {
-    int rc = launch_project_tc(a, m, n, q, N, ldq, out, ldo, mode, r0, r1, ws, st, s);
-    if (rc != TT_ERR_UNSUPPORTED) return rc;
-  }
-  const int NT = N <= 16 ? 16 : N <= 32 ? 32 : N <= 48 ? 48 : 64;
-  if (m <= 64 && N <= 64) {
-    // SPLIT threads per column: 1 for NP = 16, 2 for 32 and 48, 4 for 64.
-    const int split = NT <= 16 ? 1 : NT <= 48 ? 2 : 4;
-    const int tj = 256 / split;
-    const size_t shm = (64 * (size_t)NT + (size_t)tj * std::max<long long>(m + 1, NT + 1)) * sizeof(float);
-    smem_optin_k(k_proj_smallk<16, 1>, 100 * 1024);
-    smem_optin_k(k_proj_smallk<32, 2>, 100 * 1024);
-    smem_optin_k(k_proj_smallk<48, 2>, 100 * 1024);
-    smem_optin_k(k_proj_smallk<64, 4>, 100 * 1024);
-    const int grid = (int)std::min<long long>(ceil_div_ll(n, tj), 64LL * num_sms());
-    const int mi = (int)m;
-    switch (NT) {
-      case 16: k_proj_smallk<16, 1><<<grid, 256, shm, s>>>(a, mi, n, q, N, ldq, out, ldo, mode, r0, r1); break;
-      case 32: k_proj_smallk<32, 2><<<grid, 256, shm, s>>>(a, mi, n, q, N, ldq, out, ldo, mode, r0, r1); break;
-      case 48: k_proj_smallk<48, 2><<<grid, 256, shm, s>>>(a, mi, n, q, N, ldq, out, ldo, mode, r0, r1); break;
-      default: k_proj_smallk<64, 4><<<grid, 256, shm, s>>>(a, mi, n, q, N, ldq, out, ldo, mode, r0, r1); break;
-    }
-    count_launch();
-    TT_LAUNCH_CHECK();
-    return TT_OK;
-  }
-  long long kc;
-  int ks = project_ksplit(m, n, N, &kc);
-  float* part = nullptr;
-  const size_t mk = ws.mark();
-  if (ks > 1) {
-    part = ws.take<float>((size_t)ks * n * N);
-    if (!part) {
-      ks = 1;
-      kc = m;
-    }
-  } else {
-    kc = m;
-  }
-  // output tile width: the smallest multiple of 8 in {16, 24, 32, 40, 48, 64} covering N
-  const int NTs = N <= 16 ? 16 : N <= 24 ? 24 : N <= 32 ? 32 : N <= 40 ? 40 : N <= 48 ? 48 : 64;
-  dim3 grid(ceil_div(n, 256), ceil_div(N, NTs), ks);
-  float* dst = ks > 1 ? part : out;
-  const long long ldd = ks > 1 ? N : ldo;
-  const int md = ks > 1 ? OUT_ROWMAJOR : mode;
-#define PS_ATTR(V) smem_optin_k(k_project_simt<V>, (size_t)2 * 32 * (256 + V) * 4)
-  PS_ATTR(16); PS_ATTR(24); PS_ATTR(32); PS_ATTR(40); PS_ATTR(48); PS_ATTR(64);
-#undef PS_ATTR
-  const size_t pshm = (size_t)2 * 32 * (256 + NTs) * sizeof(float);
-#define PS_CASE(V) \
-  case V: k_project_simt<V><<<grid, 256, pshm, s>>>(a, m, n, q, N, ldq, dst, ldd, md, r0, r1, kc); break;
-  switch (NTs) {
-    PS_CASE(16)
-    PS_CASE(24)
-    PS_CASE(32)
-    PS_CASE(40)
-    PS_CASE(48)
-    default: k_project_simt<64><<<grid, 256, pshm, s>>>(a, m, n, q, N, ldq, dst, ldd, md, r0, r1, kc); break;
-  }
-#undef PS_CASE
-  count_launch();
-  TT_LAUNCH_CHECK();
-  if (ks > 1) {
-    const long long total = n * N;
-    k_project_reduce<<<(int)std::min<long long>(ceil_div_ll(total, 256), 8LL * num_sms()), 256, 0, s>>>(
-        part, n, N, ks, out, ldo, mode, r0, r1);
-    count_launch();
-    TT_LAUNCH_CHECK();
-  }
-  ws.reset(mk);
   return TT_OK;
 }
 

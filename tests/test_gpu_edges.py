@@ -107,3 +107,31 @@ def test_gram_rows_unaligned(gpu, m, n):
     tol = 64 * U32 * m * ref[0] ** 2
     assert np.all(np.abs(res.sigmas[0][:r].astype(np.float64) ** 2 - ref[:r] ** 2) <= tol)
     del torch
+
+
+@pytest.mark.parametrize("m,n,N", [(1, 1, 1), (63, 9, 7), (64, 64, 16), (65, 63, 17), (100, 1000, 24), (129, 8, 40),
+                                   (192, 100000, 33), (577, 4097, 41), (64, 513, 64), (66, 777, 65), (320, 640, 128)])
+def test_sketch_fp32_edges(gpu, m, n, N):
+    """Row tiles of 64, chunks of 8 columns dealt to 8 warps, column blocks above 64; rows that are not a
+    multiple of 4.  A product-sum of n FP32 terms is off by at most n u of the sum of magnitudes; random
+    signs leave about sqrt(n) of it, 8x that is allowed."""
+    rng = np.random.default_rng(m + n + N)
+    a, w = rng.standard_normal((m, n)).astype(np.float32), rng.standard_normal((n, N)).astype(np.float32)
+    y = _ttr().sketch(_dev(a, gpu), _dev(w, gpu), "fp32").cpu().numpy()
+    ref = a.astype(np.float64) @ w.astype(np.float64)
+    bound = 8 * np.sqrt(n) * U32 * (np.linalg.norm(a, axis=1)[:, None] * np.linalg.norm(w, axis=0)[None, :])
+    assert np.all(np.abs(y - ref) <= bound)
+
+
+@pytest.mark.parametrize("m,n,N", [(65, 127, 5), (66, 128, 16), (67, 129, 17), (128, 1000, 24), (131, 400, 40),
+                                   (600, 70, 57), (96, 300, 65), (1300, 20, 128), (68, 60000, 33),
+                                   # up to 64 rows: the small-K kernel, one and several columns per thread
+                                   (1, 5, 1), (30, 200000, 20), (33, 80000, 9), (64, 100000, 64), (48, 90000, 48),
+                                   (24, 100001, 8), (63, 300, 32), (2, 77777, 3)])
+def test_project_fp32_edges(gpu, m, n, N):
+    rng = np.random.default_rng(m + n + N)
+    a, q = rng.standard_normal((m, n)).astype(np.float32), rng.standard_normal((m, N)).astype(np.float32)
+    y = _ttr().project(_dev(a, gpu), _dev(q, gpu), "fp32").cpu().numpy()
+    ref = q.astype(np.float64).T @ a.astype(np.float64)
+    bound = 8 * np.sqrt(m) * U32 * (np.linalg.norm(q, axis=0)[:, None] * np.linalg.norm(a, axis=0)[None, :])
+    assert np.all(np.abs(y - ref) <= bound)
