@@ -11,7 +11,6 @@
 #include <string.h>
 
 #include <algorithm>
-#include <cmath>
 #include <string>
 #include <vector>
 
@@ -1343,69 +1342,69 @@ extern "C" int tt_rel_error(tt_ctx* c, const float* x, int d, const int* n, cons
     return TT_ERR_UNSUPPORTED;
   }
   // Left part of a split after core k (k cores): (r0, P_k, r_k); right part: (r_k, N_k, r_d).  Any
-  // split gives the same product; its cost is the final contraction (2 |X| r0 r_k, in tiles of 128
-  // x 128) plus the merges of both sides, least where both sides are small.  Scratch: two buffers
-  // a side, at most what merging everything right of core 1 takes.
-  std::vector<double> P((size_t)d + 1, 1.0);
+  // split gives the same product; its cost is the final contraction (r0 r_k FMAs per element, in whole
+  // tiles) plus the merges of both sides, least where both sides are small.  Scratch (FP64): the
+  // last two merges of a side, at most what merging everything right of core 1 takes.
+  std::vector<long long> P((size_t)d + 1, 1);
   for (int k = 0; k < d; ++k) P[(size_t)k + 1] = P[(size_t)k] * n[k];
-  const double most = [&] {
-    double m = 0.0;
-    for (int k = d - 1; k >= 1; --k) m = std::max(m, (double)r[k] * (P[(size_t)d] / P[(size_t)k]) * r[d]);
-    return m;
-  }();
+  auto right_of = [&](int k) { return P[(size_t)d] / P[(size_t)k]; };  // n_k ... n_{d-1}
+  auto left_elems = [&](int k) { return (size_t)(rr0 * P[(size_t)k] * r[k]); };
+  auto right_elems = [&](int k) { return (size_t)r[k] * (size_t)right_of(k) * (size_t)r[d]; };
+  // ping-pong buffers of the merges up to a split: [0] the even merges, [1] the odd ones
+  struct Bufs2 {
+    size_t b[2] = {0, 0};
+  };
+  auto left_bufs = [&](int cut) {
+    Bufs2 q;
+    for (int k = 2; k <= cut; ++k) q.b[k & 1] = std::max(q.b[k & 1], left_elems(k));
+    return q;
+  };
+  auto right_bufs = [&](int cut) {
+    Bufs2 q;
+    for (int k = d - 2; k >= cut; --k) q.b[k & 1] = std::max(q.b[k & 1], right_elems(k));
+    return q;
+  };
+  const Bufs2 all = right_bufs(1);
   int cut = 1;
   double best = -1.0;
   for (int k = 1; k < d; ++k) {
-    const double Nk = P[(size_t)d] / P[(size_t)k];
-    const double tiles = std::ceil(P[(size_t)k] / 128.0) * std::ceil(Nk / 128.0);
-    double cost = tiles * 16384.0 * rr0 * r[k], lmax = 0.0, rmax = 0.0;
-    for (int j = 2; j <= k; ++j) {
-      cost += (double)rr0 * P[(size_t)j] * r[j - 1] * r[j];
-      lmax = std::max(lmax, (double)rr0 * P[(size_t)j] * r[j]);
-    }
-    for (int j = d - 2; j >= k; --j) {
-      const double out = (double)r[j] * (P[(size_t)d] / P[(size_t)j]) * r[d];
-      cost += out * r[j + 1];
-      rmax = std::max(rmax, out);
-    }
-    if (k > 1 && lmax + rmax > most) continue;
+    double cost = (double)recon_tiles(P[(size_t)k], right_of(k)) * 8192.0 * rr0 * r[k];
+    for (int j = 2; j <= k; ++j) cost += (double)left_elems(j) * r[j - 1];
+    for (int j = d - 2; j >= k; --j) cost += (double)right_elems(j) * r[j + 1];
+    const Bufs2 lb = left_bufs(k), rb = right_bufs(k);
+    if (k > 1 && lb.b[0] + lb.b[1] + rb.b[0] + rb.b[1] > all.b[0] + all.b[1]) continue;
     if (best < 0.0 || cost < best) {
       best = cost;
       cut = k;
     }
   }
-  auto left_elems = [&](int k) { return (size_t)rr0 * (size_t)P[(size_t)k] * (size_t)r[k]; };
-  auto right_elems = [&](int k) { return (size_t)r[k] * (size_t)(P[(size_t)d] / P[(size_t)k]) * (size_t)r[d]; };
-  size_t lmax = 1, rmax = 1;
-  for (int k = 2; k <= cut; ++k) lmax = std::max(lmax, left_elems(k));
-  for (int k = d - 2; k >= cut; --k) rmax = std::max(rmax, right_elems(k));
-  TT_TRY(tt_ctx_reserve(c, sizeof(float) * 2 * (lmax + rmax) + 4096 + (1 << 20)));
+  const Bufs2 lb = left_bufs(cut), rb = right_bufs(cut);
+  TT_TRY(tt_ctx_reserve(c, sizeof(double) * (lb.b[0] + lb.b[1] + rb.b[0] + rb.b[1]) + 8192 + (1 << 20)));
   Arena a{c->arena, c->cap, 0};
-  float* lbuf[2] = {a.take<float>(lmax), a.take<float>(lmax)};
-  float* rbuf[2] = {a.take<float>(rmax), a.take<float>(rmax)};
+  double* lbuf[2] = {a.take<double>(lb.b[0]), a.take<double>(lb.b[1])};
+  double* rbuf[2] = {a.take<double>(rb.b[0]), a.take<double>(rb.b[1])};
   double* acc = a.take<double>(2);
-  if (!lbuf[1] || !rbuf[1] || !acc) {
+  if (!lbuf[0] || !lbuf[1] || !rbuf[0] || !rbuf[1] || !acc) {
     set_error(TT_ERR_NOMEM, "error workspace");
     return TT_ERR_NOMEM;
   }
   cudaStream_t s = c->stream;
-  const float* lf = cores[0];
+  const void* lf = cores[0];
   for (int k = 2; k <= cut; ++k) {
     // (r0, P_k, r_k) = (r0 P_{k-1} x r_{k-1}) * (r_{k-1} x n_{k-1} r_k)
-    TT_TRY(launch_gemm_nn(lf, rr0 * (long long)P[(size_t)k - 1], r[k - 1], cores[k - 1], (long long)n[k - 1] * r[k],
-                          lbuf[k & 1], s));
+    TT_TRY(launch_merge(lf, k > 2, rr0 * P[(size_t)k - 1], r[k - 1], cores[k - 1], false, (long long)n[k - 1] * r[k],
+                        lbuf[k & 1], s));
     lf = lbuf[k & 1];
   }
-  const float* rf = cores[d - 1];
+  const void* rf = cores[d - 1];
   for (int k = d - 2; k >= cut; --k) {
     // (r_k, N_k, r_d) = (r_k n_k x r_{k+1}) * (r_{k+1} x N_{k+1} r_d)
-    TT_TRY(launch_gemm_nn(cores[k], (long long)r[k] * n[k], r[k + 1], rf,
-                          (long long)(P[(size_t)d] / P[(size_t)k + 1]) * r[d], rbuf[k & 1], s));
+    TT_TRY(launch_merge(cores[k], false, (long long)r[k] * n[k], r[k + 1], rf, k < d - 2, right_of(k + 1) * r[d],
+                        rbuf[k & 1], s));
     rf = rbuf[k & 1];
   }
   TT_CUDA(cudaMemsetAsync(acc, 0, 2 * sizeof(double), s));
-  TT_TRY(launch_recon_err(x, (long long)P[(size_t)cut], (long long)(P[(size_t)d] / P[(size_t)cut]), lf, rf, (int)rr0,
-                          r[cut], acc, s));
+  TT_TRY(launch_recon_err(x, P[(size_t)cut], right_of(cut), lf, cut > 1, rf, cut < d - 1, (int)rr0, r[cut], acc, s));
   double h[2] = {0, 0};
   TT_CUDA(cudaMemcpyAsync(h, acc, sizeof(h), cudaMemcpyDeviceToHost, s));
   TT_CUDA(cudaStreamSynchronize(s));

@@ -1,5 +1,5 @@
 // CUDA-core kernels of the TT/TR-SVD chain: Gaussian test matrix, Jacobi eigen-solvers, bond permute,
-// core folding, reconstruction error and the small helpers between them.
+// core folding and the small helpers between them.
 #include <float.h>
 #include <stdlib.h>
 #include <math.h>
@@ -993,227 +993,6 @@ int launch_diff_norm(const float* x, const float* y, long long count, double* ac
   if (count <= 0) return TT_OK;
   k_diff_norm<<<(int)std::min<long long>(ceil_div_ll(count, 256), 4LL * num_sms()), 256, 0, s>>>(
       x, y, count, acc);
-  count_launch();
-  TT_LAUNCH_CHECK();
-  return TT_OK;
-}
-
-// C (M x N) = A (M x K) * B (K x N), column-major, K small.
-__global__ void __launch_bounds__(256) k_gemm_nn(const float* __restrict__ a, long long M, int K,
-                                                 const float* __restrict__ b, long long N,
-                                                 float* __restrict__ c) {
-  __shared__ float bs[32][65];
-  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
-  const long long n0 = (long long)blockIdx.y * 32;
-  float acc[32];
-#pragma unroll
-  for (int u = 0; u < 32; ++u) acc[u] = 0.f;
-  for (int k0 = 0; k0 < K; k0 += 64) {
-    for (int f = threadIdx.x; f < 32 * 64; f += 256) {
-      const int kk = f % 64, u = f / 64;
-      const long long col = n0 + u;
-      bs[u][kk] = (col < N && k0 + kk < K) ? b[(k0 + kk) + (long long)K * col] : 0.f;
-    }
-    __syncthreads();
-    if (i < M) {
-      const int kmax = (K - k0 < 64) ? K - k0 : 64;
-#pragma unroll 8  // loads of A in flight: a merge of small cores is all latency
-      for (int kk = 0; kk < kmax; ++kk) {
-        const float av = a[i + M * (long long)(k0 + kk)];
-#pragma unroll
-        for (int u = 0; u < 32; ++u) acc[u] = fmaf(av, bs[u][kk], acc[u]);
-      }
-    }
-    __syncthreads();
-  }
-  if (i < M) {
-#pragma unroll
-    for (int u = 0; u < 32; ++u) {
-      const long long col = n0 + u;
-      if (col < N) c[i + M * col] = acc[u];
-    }
-  }
-}
-
-int launch_gemm_nn(const float* a, long long M, int K, const float* b, long long N, float* c,
-                   cudaStream_t s) {
-  if (M <= 0 || N <= 0) return TT_OK;
-  const long long gy = ceil_div_ll(N, 32);
-  // grid.y is limited to 65535: chunk the column range.
-  for (long long y0 = 0; y0 < gy; y0 += 65535) {
-    const long long ny = std::min<long long>(65535, gy - y0);
-    dim3 grid(ceil_div(M, 256), (unsigned)ny);
-    k_gemm_nn<<<grid, 256, 0, s>>>(a, M, K, b + (long long)K * 32 * y0, N - 32 * y0,
-                                   c + M * 32 * y0);
-    count_launch();
-    TT_LAUNCH_CHECK();
-  }
-  return TT_OK;
-}
-
-// err^2 += sum_{i,J} (X[i + P J] - sum_{a,b} L[a + r0 (i + P b)] R[b + rk (J + N a)])^2, and ||X||^2.
-//
-// A GEMM over q = r0 rk whose 128 x 128 result tile is compared with X in registers and never
-// written.  Bound by the FP32 FMAs (2 q per element of X; 0.93 ms for a 32^6 tensor at q = 32) next
-// to one read of X (0.66 ms).  256 threads of 8 x 8 entries: 4 shared-memory loads of 16 bytes feed
-// 32 paired FMAs, the 32-deep K chunks of both factors double-buffered by cp.async.  Difference and
-// sums are FP64; two blocks per SM, so one block's X loads and conversions run beside the other's
-// FMAs.  (The kernel this one replaces took two shared-memory loads per FMA, and a merged factor as
-// large as X besides: 18.0 ms for the 32^6 check at ranks 32, 2.4 ms now.)
-constexpr int RE_T = 128, RE_KC = 32, RE_LD = RE_T + 4;
-constexpr size_t RE_SMEM = (size_t)2 * 2 * RE_KC * RE_LD * sizeof(float);
-
-template <bool RING>
-__global__ void __launch_bounds__(256, 2) k_recon_err(const float* __restrict__ x, long long P, long long N,
-                                                      const float* __restrict__ lf, const float* __restrict__ rf,
-                                                      int r0, int rk, double* acc) {
-  extern __shared__ __align__(16) float sm_re[];
-  float* const ls = sm_re;                       // [2][KC][LD] rows i
-  float* const rs = sm_re + 2 * RE_KC * RE_LD;   // [2][KC][LD] columns J
-  __shared__ double sh[32];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int q = r0 * rk, nk = (q + RE_KC - 1) / RE_KC;
-  const long long pt = (P + RE_T - 1) / RE_T, nt = (N + RE_T - 1) / RE_T, ntiles = pt * nt;
-  const long long my = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;  // tiles of this block
-  const long long stages = my * nk;
-  const bool lv = r0 == 1 && (P & 3) == 0 && (reinterpret_cast<uintptr_t>(lf) & 15) == 0;
-  const bool xv = (P & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-  // stage st: K chunk st % nk of this block's tile st / nk, into buffer st & 1
-  auto load = [&](long long st) {
-    const long long t = blockIdx.x + (st / nk) * gridDim.x;
-    const int k0 = (int)(st % nk) * RE_KC;
-    const long long i0 = (t % pt) * RE_T, j0 = (t / pt) * RE_T;
-    float* const l = ls + (st & 1) * RE_KC * RE_LD;
-    float* const r = rs + (st & 1) * RE_KC * RE_LD;
-    if (lv) {
-      const int kk = tid >> 5, i4 = 4 * (tid & 31);
-      const float* src = lf + (i0 + i4) + P * (k0 + kk);
-      const bool in = i0 + i4 < P;  // P % 4 == 0: four rows or none
-#pragma unroll
-      for (int u = 0; u < RE_KC / 8; ++u) {
-        const bool ok = in && k0 + kk + 8 * u < q;
-        cp_async16z(l + (kk + 8 * u) * RE_LD + i4, ok ? src + 8 * u * P : lf, ok);
-      }
-    } else {
-#pragma unroll 4
-      for (int u = 0; u < RE_KC * RE_T / 256; ++u) {
-        const int f = tid + 256 * u, kk = f >> 7, i = f & 127;
-        const int c = k0 + kk, b = RING ? c / r0 : c, a = RING ? c - b * r0 : 0;
-        const bool ok = c < q && i0 + i < P;
-        cp_async4(l + kk * RE_LD + i, ok ? lf + a + r0 * ((i0 + i) + P * b) : lf, ok);
-      }
-    }
-    // consecutive lanes take consecutive contraction indices: for a train R's columns are contiguous
-    const int kk = tid & 31, c = k0 + kk, b = RING ? c / r0 : c, a = RING ? c - b * r0 : 0;
-    const float* src = rf + b + rk * ((j0 + (tid >> 5)) + N * a);
-    const int nj = c < q ? (int)min((long long)RE_T, N - j0) : 0;
-#pragma unroll
-    for (int u = 0; u < RE_T / 8; ++u) {
-      const int j = (tid >> 5) + 8 * u;
-      cp_async4(r + kk * RE_LD + j, j < nj ? src + (long long)(8 * rk) * u : rf, j < nj);
-    }
-  };
-  uint64_t s2[4][8];  // rows (i, i + 1) of four row pairs x 8 columns
-  double d2 = 0.0, x2 = 0.0;
-  if (stages > 0) load(0);
-  cp_async_commit();
-  for (long long st = 0; st < stages; ++st) {
-    cp_async_wait<0>();
-    __syncthreads();  // stage st landed for every thread; buffer (st + 1) & 1 is no longer read
-    if (st + 1 < stages) load(st + 1);
-    cp_async_commit();
-    const int kc = (int)(st % nk);
-    const long long t = blockIdx.x + (st / nk) * gridDim.x;
-    const long long ib = (t % pt) * RE_T, jb = (t / pt) * RE_T;
-    const bool whole = xv && ib + RE_T <= P && jb + RE_T <= N;
-    if (kc == 0) {
-      if (whole) {  // the tile of X into L2 while its products are formed: 512 lines, 2 per thread
-#pragma unroll
-        for (int u = 0; u < 2; ++u)
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(x + ib + 32 * (tid & 3) + P * (jb + (tid >> 2) + 64 * u)));
-      }
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-#pragma unroll
-        for (int c = 0; c < 8; ++c) s2[e][c] = 0ull;
-    }
-    const float* l = ls + (st & 1) * RE_KC * RE_LD + 4 * tx;
-    const float* r = rs + (st & 1) * RE_KC * RE_LD + 4 * ty;
-    const int kmax = min(RE_KC, q - kc * RE_KC);
-#pragma unroll 4
-    for (int kk = 0; kk < kmax; ++kk) {
-      const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(l + kk * RE_LD);
-      const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(l + kk * RE_LD + 64);
-      const float4 b0 = *reinterpret_cast<const float4*>(r + kk * RE_LD);
-      const float4 b1 = *reinterpret_cast<const float4*>(r + kk * RE_LD + 64);
-      const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const uint64_t bd = f2_dup(b[c]);
-        ffma2(s2[0][c], a0.x, bd);
-        ffma2(s2[1][c], a0.y, bd);
-        ffma2(s2[2][c], a1.x, bd);
-        ffma2(s2[3][c], a1.y, bd);
-      }
-    }
-    if (kc + 1 < nk) continue;
-    const long long i0 = ib + 4 * tx, j0 = jb + 4 * ty;
-    auto add = [&](float xe, float se) {
-      const double xd = xe, dv = xd - (double)se;
-      d2 = fma(dv, dv, d2);
-      x2 = fma(xd, xd, x2);
-    };
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const long long i = i0 + 64 * h;
-      if (whole) {
-        // 8 loads in flight (a load at a time, each waited for, took 4.1 ms instead of 2.4)
-        float4 v[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-          v[c] = __ldcs(reinterpret_cast<const float4*>(x + i + P * (j0 + (c & 3) + (c & 4) * 16)));
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          float s0, s1, s3, s4;
-          f2_unpack(s2[2 * h][c], s0, s1);
-          f2_unpack(s2[2 * h + 1][c], s3, s4);
-          add(v[c].x, s0);
-          add(v[c].y, s1);
-          add(v[c].z, s3);
-          add(v[c].w, s4);
-        }
-      } else {
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          const long long j = j0 + (c & 3) + (c & 4) * 16;
-          float sr[4];
-          f2_unpack(s2[2 * h][c], sr[0], sr[1]);
-          f2_unpack(s2[2 * h + 1][c], sr[2], sr[3]);
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            if (j < N && i + e < P) add(x[i + e + P * j], sr[e]);
-        }
-      }
-    }
-  }
-  d2 = block_sum(d2, sh);
-  x2 = block_sum(x2, sh);
-  if (threadIdx.x == 0) {
-    atomicAdd(&acc[0], d2);
-    atomicAdd(&acc[1], x2);
-  }
-}
-
-int launch_recon_err(const float* x, long long P, long long N, const float* lf, const float* rf, int r0, int rk,
-                     double* acc, cudaStream_t s) {
-  TT_TRY(smem_optin_k(k_recon_err<false>, RE_SMEM));
-  TT_TRY(smem_optin_k(k_recon_err<true>, RE_SMEM));
-  const long long tiles = ceil_div_ll(P, RE_T) * ceil_div_ll(N, RE_T);
-  const int grid = (int)std::min<long long>(tiles, 2LL * num_sms());
-  if (r0 == 1)
-    k_recon_err<false><<<grid, 256, RE_SMEM, s>>>(x, P, N, lf, rf, r0, rk, acc);
-  else
-    k_recon_err<true><<<grid, 256, RE_SMEM, s>>>(x, P, N, lf, rf, r0, rk, acc);
   count_launch();
   TT_LAUNCH_CHECK();
   return TT_OK;

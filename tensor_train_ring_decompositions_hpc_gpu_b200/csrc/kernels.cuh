@@ -119,15 +119,16 @@ int launch_check_finite(const float* x, long long count, int* flag, cudaStream_t
 // Sum of squares (FP64) of (x - y) and of x, accumulated into acc[0], acc[1].
 int launch_diff_norm(const float* x, const float* y, long long count, double* acc, cudaStream_t s);
 
-// Dense C (M x N) = A (M x K) * B (K x N), all FP32 column-major, small K (core merging).
-int launch_gemm_nn(const float* a, long long M, int K, const float* b, long long N, float* c,
-                   cudaStream_t s);
+// C (M x N, FP64) = A (M x K) * B (K x N), column-major, each FP32 or FP64 (a64, b64): core merging.
+int launch_merge(const void* a, bool a64, long long M, int K, const void* b, bool b64, long long N, double* c,
+                 cudaStream_t s);
 
 // Fused reconstruction check of a ring/train: acc += ||X - X^||^2 and ||X||^2, X (P x N) and
 // X^[i, J] = sum_{a,b} L[a, i, b] R[b, J, a] with the merged left cores L (r0, P, rk) and the merged
-// right cores R (rk, N, r0).
-int launch_recon_err(const float* x, long long P, long long N, const float* lf, const float* rf, int r0, int rk,
-                     double* acc, cudaStream_t s);
+// right cores R (rk, N, r0), each FP64 (merged) or FP32 (a core as it is); recon_tiles: its tile count.
+long long recon_tiles(long long P, long long N);
+int launch_recon_err(const float* x, long long P, long long N, const void* lf, bool l64, const void* rf, bool r64,
+                     int r0, int rk, double* acc, cudaStream_t s);
 
 // Learned predictor (mlp.cu).  Features from the descending probe eigenvalues mu
 // (TT_PROBE_COLS of them); network inference; training (mode 0: Adam steps on Philox-drawn

@@ -32,8 +32,8 @@ def _dev(x, dev, dtype=np.float32):
     (True, (130, 3, 131), (2, 5, 6, 2)),
 ])
 def test_rel_error_edges(gpu, ring, n, ranks):
-    """Every merged entry is a chain of FP32 FMAs (one contraction per bond): relative errors of
-    (sum of the bond sizes + order) u of the absolute sums, taken as 4x the sums themselves."""
+    """FP32 products would be off by (sum of the bond sizes + order) u of the absolute sums, taken as 4x
+    the sums themselves; FP64 ones are far inside."""
     rng = np.random.default_rng(sum(n))
     d = len(n)
     cores = [rng.standard_normal((ranks[k], n[k], ranks[k + 1])).astype(np.float32) for k in range(d)]
