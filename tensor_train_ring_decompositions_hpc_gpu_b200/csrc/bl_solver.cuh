@@ -18,27 +18,24 @@ namespace ttr {
 // read as one 16-byte load; W is symmetrised on input ((W + W^T) / 2).
 // The warps split three ways each round, with one barrier per round:
 //   - the W warps update the upper 2 x 2 blocks, one per thread;
-//   - the V warps hold the eigenvectors in registers.  For N <= 32 one warp does it all: lane i
-//     keeps row i of V by position (Np registers), applies the round's Np / 2 rotations and the
-//     shear as a fixed register permutation (compiled per Np), so no eigenvector entry leaves its
-//     thread.  It runs one round behind, with the FP64 rotations that the W threads of the
-//     diagonal blocks publish (they renormalise them anyway), and applies the last round after
-//     the loop.  Moving V by shuffles or through shared memory every round costs more than the
-//     rotation itself (the shuffle / shared-memory path is the round's bottleneck once all of V
-//     crosses it).  For 32 < N <= 64 V is split by components: lane k of a V warp keeps positions
-//     2k and 2k+1 of up to kBlVRows components and passes results on with two shuffles (lane k's
-//     new even entry comes from lane k+1, its odd entry from lane k-1);
+//   - the V warps hold the eigenvectors in registers, a row per lane, the positions of a row split over
+//     four warps (contiguous pairs each).  A warp applies the round's rotations of its pairs and the
+//     shear as a fixed register permutation (compiled per Np and part); the two entries per row that the
+//     shear carries over a boundary go through shared memory and are picked up after the round's barrier.
+//     V runs one round behind, with the FP64 rotations that the W threads of the diagonal blocks publish
+//     (they renormalise them anyway), and applies the last round after the loop.  (A whole row per lane
+//     took a warp 500 cycles a round, longer than the rotation chain; moving all of V by shuffles or
+//     through shared memory costs more than the rotations themselves.);
 //   - the last warp computes the next round's rotations meanwhile, from the current blocks and
-//     rotations (jacobi_cs32: two reciprocal square roots, no division).  The rotations are
-//     published as FP32 pairs; the W and V warps renormalise them to FP64 (rot_from_cs32), while
+//     rotations (jacobi_cs32: two approximate reciprocal square roots, no division).  The rotations are
+//     published as FP32 pairs; the W threads renormalise them to FP64 (rot_from_cs32), while
 //     the rotation warp forms the next round's 2 x 2 blocks from the FP32 pairs as they are: the
 //     renormalisation scales both entries of a pair by the same factor 1 + O(1e-7), so those
 //     blocks come out with relative errors of that size only (the off-diagonal entry included),
 //     which moves the next rotation's angle by as much as FP32 (c, s) rounding does, and keeps
-//     the renormalisation off the chain.  That chain bounds the round, so for N <= 48 it gets a
+//     the renormalisation off the chain.  That chain bounds the round, so up to N = 46 it gets a
 //     scheduler of its own: warps w with w % 4 == 3 (one scheduler's share, as warps are spread over the
-//     four schedulers by w % 4) do no work but the barrier, and the W and V warps use the others
-//     (measured 126 vs 178 us for N = 32; at N = 64 the W and V warps need all four).
+//     four schedulers by w % 4) do no work but the barrier, and the W and V warps use the others.
 // Pairs with a_pq^2 <= 1e-24 |a_pp a_qq| or |a_pq| <= 1e-14 max|diag| are not rotated
 // (jacobi_needed); the solve ends after the first sweep that leaves no pair to rotate.
 // Eigenvalues are ordered by a parallel rank count.
@@ -56,61 +53,97 @@ __host__ __device__ constexpr int bl_move(int P, int Np) {
   return P >= 4 ? P - 2 : (P == 2 ? 1 : 0);       // even positions down one pair; 2 turns up, 0 stays
 }
 
-constexpr int kBlVRows = 5;  // eigenvector components per V warp (32 < N <= 64)
+// VN: the largest N (rounded up) a solver instance serves: 32, 48 (N <= 46) or 64.
+constexpr int kBlParts = 4;  // warps sharing a row of V, VN / 4 positions per lane
+__host__ __device__ constexpr int bl_vn(int N) { return N <= 32 ? 32 : N <= 46 ? 48 : 64; }
 
-// One round of the row-resident V (N <= 32): v holds row i of V by position; rotate the NP / 2
-// pairs with the FP64 rotations cs and move every result to its next-round position, in place.
-// Pair k's results go to positions 2k - 2 (pair k - 1's even slot, or 0 / 1 for k = 0 / 1) and
-// 2k + 3 (pair k + 1's odd slot, or NP - 2 for the last pair), so in increasing k every
-// destination but the next pair's odd slot has been read already; that one old value is carried.
-// The rotations are read 8 pairs at a time (a warp barrier between the groups keeps the compiler
-// from loading all of them ahead, which would hold 4 NP more registers).
-template <int NP, int VN>
-__device__ __forceinline__ void bl_vrow_round(double (&v)[VN], const double2* __restrict__ cs) {
-  if (NP == 2) {
-    const double2 r = cs[0];
-    const double a = v[0], b = v[1];
-    v[0] = a * r.x - b * r.y;
-    v[1] = a * r.y + b * r.x;
-    return;
-  }
-  double ob = v[1];  // the old odd entry of the pair being rotated
+// Pairs of part p of a row of NP positions: [bl_first(NP, parts, p), bl_first(NP, parts, p + 1)).  Rows of
+// fewer pairs than parts stay whole in part 0.
+constexpr int bl_first(int NP, int p) {
+  const int H = NP / 2;
+  return H < kBlParts ? (p == 0 ? 0 : H) : H * p / kBlParts;
+}
+
+// One round of part PART of a row of V: rotate its pairs with the FP64 rotations cs and move every result
+// to its next-round position.  Pair k's results go to pair k - 1's even slot (pair 1's to pair 0's odd one,
+// pair 0's stays) and to pair k + 1's odd slot (the last pair's to its own even one), so in increasing k
+// every destination but the next pair's odd slot has been read already; that one old value is carried.
+// Results that leave the part go to dn (its first pair's even one) and up (its last pair's odd one).
+template <int NP, int PART, int VL>
+__device__ __forceinline__ void bl_vpart_round(double (&v)[VL], const double2* __restrict__ cs, double* dn,
+                                               double* up) {
+  constexpr int H = NP / 2, K0 = bl_first(NP, PART), K1 = bl_first(NP, PART + 1);
+  if constexpr (K0 < K1) {
+    if constexpr (NP == 2) {
+      const double2 r = cs[0];
+      const double a = v[0], b = v[1];
+      v[0] = a * r.x - b * r.y;
+      v[1] = a * r.y + b * r.x;
+    } else {
+      double ob = v[1];  // the old odd entry of the pair being rotated
 #pragma unroll
-  for (int k = 0; k < NP / 2; ++k) {
-    if (k > 0 && k % 8 == 0) __syncwarp();
-    const double2 r = cs[k];
-    const double a = v[2 * k], b = ob;
-    if (k + 1 < NP / 2) ob = v[2 * k + 3];
-    v[bl_move(2 * k, NP)] = a * r.x - b * r.y;
-    v[bl_move(2 * k + 1, NP)] = a * r.y + b * r.x;
+      for (int k = K0; k < K1; ++k) {
+        const double2 r = cs[k];
+        const double a = v[2 * (k - K0)], b = ob;
+        if (k + 1 < K1) ob = v[2 * (k - K0) + 3];
+        const double even = a * r.x - b * r.y, odd = a * r.y + b * r.x;
+        if (k == K0 && K0 > 0) *dn = even;
+        else v[bl_move(2 * k, NP) - 2 * K0] = even;
+        if (k + 1 == K1 && K1 < H) *up = odd;
+        else v[bl_move(2 * k + 1, NP) - 2 * K0] = odd;
+      }
+    }
   }
 }
-template <int VN>
-__device__ __forceinline__ void bl_vrow_apply(int Np, double (&v)[VN], const double2* __restrict__ cs) {
-  switch (Np) {
-#define BL_VR(NP)                                  \
-  case NP:                                         \
-    if constexpr (NP <= VN) bl_vrow_round<NP, VN>(v, cs); \
-    break;
-    BL_VR(2) BL_VR(4) BL_VR(6) BL_VR(8) BL_VR(10) BL_VR(12) BL_VR(14) BL_VR(16)
-    BL_VR(18) BL_VR(20) BL_VR(22) BL_VR(24) BL_VR(26) BL_VR(28) BL_VR(30) BL_VR(32)
-    BL_VR(34) BL_VR(36) BL_VR(38) BL_VR(40) BL_VR(42) BL_VR(44) BL_VR(46) BL_VR(48)
-#undef BL_VR
-    default:
-      break;
+// The entries that the previous round carried into part PART: from below (the part before, through its
+// up) and from above.
+template <int NP, int PART, int VL>
+__device__ __forceinline__ void bl_vpart_take(double (&v)[VL], const double* below, const double* above) {
+  constexpr int H = NP / 2, K0 = bl_first(NP, PART), K1 = bl_first(NP, PART + 1);
+  if constexpr (K0 < K1) {
+    if constexpr (K0 > 0) v[bl_move(2 * K0 - 1, NP) - 2 * K0] = *below;
+    if constexpr (K1 < H) v[bl_move(2 * K1, NP) - 2 * K0] = *above;
   }
 }
 
-// Launch shape of the solver: the block's warp count (the last one the rotation warp) and whether
-// the rotation warp has a scheduler of its own (warps w % 4 == 3 idle), which needs the W warps
-// (one block per thread) and the V warps to fit on three schedulers' 24 warp slots (N <= 48);
-// larger N use every warp.  rowv: V row-resident (a row of V per lane, N <= 46), in at most 12
-// warps (the registers of a row of V), so N = 45, 46 give up the rotation warp's scheduler.
-__host__ __device__ inline void bl_shape(int N, bool rowv, int* iso, int* warps) {
+template <int V>
+struct BlInt {
+  static constexpr int value = V;
+};
+// f(BlInt<Np>, BlInt<part>) for the sizes an instance serves.
+template <int VN, class F>
+__device__ __forceinline__ void bl_dispatch(int Np, int part, F&& f) {
+#define BL_NP(NP)                                                     \
+  case NP:                                                            \
+    if constexpr (NP <= VN) {                                         \
+      if (part == 0) f(BlInt<NP>{}, BlInt<0>{});                      \
+      if (part == 1) f(BlInt<NP>{}, BlInt<1>{});                      \
+      if (part == 2) f(BlInt<NP>{}, BlInt<2>{});                      \
+      if (part == 3) f(BlInt<NP>{}, BlInt<3>{});                      \
+    }                                                                 \
+    break;
+  if constexpr (VN == 32) {
+    switch (Np) {
+      BL_NP(2) BL_NP(4) BL_NP(6) BL_NP(8) BL_NP(10) BL_NP(12) BL_NP(14) BL_NP(16)
+      BL_NP(18) BL_NP(20) BL_NP(22) BL_NP(24) BL_NP(26) BL_NP(28) BL_NP(30) BL_NP(32)
+    }
+  } else if constexpr (VN == 48) {
+    switch (Np) { BL_NP(34) BL_NP(36) BL_NP(38) BL_NP(40) BL_NP(42) BL_NP(44) BL_NP(46) }
+  } else {
+    switch (Np) {
+      BL_NP(48) BL_NP(50) BL_NP(52) BL_NP(54) BL_NP(56) BL_NP(58) BL_NP(60) BL_NP(62) BL_NP(64)
+    }
+  }
+#undef BL_NP
+}
+
+// Launch shape of the solver: the block's warp count (the last one the rotation warp) and whether the
+// rotation warp has a scheduler of its own (warps w % 4 == 3 idle); N > 46 use every warp.
+__host__ __device__ inline void bl_shape(int N, int* iso, int* warps) {
   const int Np = N + (N & 1), H = Np / 2, NWB = H * (H + 1) / 2;
-  const int nv = rowv ? (N + 31) / 32 : (N + kBlVRows - 1) / kBlVRows;
+  const int nv = kBlParts * ((N + 31) / 32);
   const int wu = (NWB + 31) / 32;
-  *iso = (wu + nv <= 24 && !(rowv && 4 * ((wu + nv + 2) / 3) > 12)) ? 1 : 0;
+  *iso = N <= 46 ? 1 : 0;
   *warps = *iso ? 4 * ((wu + nv + 2) / 3) : wu + nv + 1;
 }
 
@@ -118,13 +151,12 @@ __host__ __device__ inline void bl_shape(int N, bool rowv, int* iso, int* warps)
 // count): W (N x N, symmetric, any layout) -> evals (descending), evecs (N x N column-major);
 // `wbuf` holds 2 (N + N % 2)^2 doubles of shared memory.  Returns the sweeps run, or
 // max_sweeps + 1 when the last sweep still rotated.  Ends with a block barrier.
-// VN: 32 or 48 keeps V row-resident and serves N <= min(VN, 46); 0 splits V by components
-// (N <= 64).
+// VN: bl_vn(N).
 template <int VN>
 __device__ __forceinline__ int bl_solve(const double* __restrict__ w_in, int N, double* __restrict__ evals,
                                         double* __restrict__ evecs, int max_sweeps, double* wbuf) {
-  static_assert(VN == 0 || VN == 32 || VN == 48, "bl_solve: VN is 0, 32 or 48");
-  constexpr bool vrow = VN > 0;                      // V rows resident, one per lane of one warp
+  static_assert(VN == 32 || VN == 48 || VN == 64, "bl_solve: VN is 32, 48 or 64");
+  constexpr int PARTS = kBlParts, VL = VN / kBlParts, VR = VN <= 32 ? 32 : 64;
   const int PW = (int)(blockDim.x >> 5) - 1;  // the last warp computes the next round's rotations
   const int Np = N + (N & 1);
   const int NR = Np - 1;
@@ -133,32 +165,34 @@ __device__ __forceinline__ int bl_solve(const double* __restrict__ w_in, int N, 
   double* Wb0 = wbuf;
   double* Wb1 = Wb0 + NN;
   __shared__ float2 pcs[2][32];   // FP32 (c, s) of each pair, current and next round
-  __shared__ double2 pcd[2][32];  // the same renormalised to FP64, for the row-resident V
+  __shared__ double2 pcd[2][32];  // the same renormalised to FP64, for V
+  __shared__ double xup[2][PARTS][VR], xdn[2][PARTS][VR];  // entries of V crossing the boundary above a part
   __shared__ int imv[64];
   __shared__ double dg[64];
   __shared__ int rk[64], pidx[64];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int iso, nwarps;
-  bl_shape(N, vrow, &iso, &nwarps);
+  bl_shape(N, &iso, &nwarps);
   const int NWB = H * (H + 1) / 2;                   // upper blocks (a <= b), one per W thread
   const int WU = (NWB + 31) / 32;                    // W warps
-  const int NVW = vrow ? (N + 31) / 32 : (N + kBlVRows - 1) / kBlVRows;  // V warps
-  const int vrows = (N + NVW - 1) / NVW;             // components per V warp (<= kBlVRows)
+  const int NVW = PARTS * ((N + 31) / 32);           // V warps: part of a row, then 32 rows
   // role index among the working warps (with iso, those with w % 4 != 3); -1 for the idle ones
   // and the rotation warp
   const int ai = (warp == PW || (iso && (warp & 3) == 3)) ? -1 : iso ? (warp >> 2) * 3 + (warp & 3) : warp;
   const bool ww = ai >= 0 && ai < WU;                // W warp
   const bool vw = ai >= WU && ai < WU + NVW;         // V warp
   for (int P = tid; P < Np; P += blockDim.x) imv[Np >= 4 ? bl_move(P, Np) : P] = P;
-  for (int idx = tid; idx < NN; idx += blockDim.x) {
-    const int i = idx / Np, j = idx - (idx / Np) * Np;
-    const int Pi = bl_pos(i, Np), Pj = bl_pos(j, Np);  // round 0: index i sits in slot i
-    double x = 0.0;
-    if (i < N && j < N) x = 0.5 * (w_in[i + (long long)N * j] + w_in[j + (long long)N * i]);
-    Wb0[Pi * Np + Pj] = x;
-  }
+  for (int i = warp; i < Np; i += (int)(blockDim.x >> 5))
+    for (int j = lane; j < Np; j += 32) {
+      const int Pi = bl_pos(i, Np), Pj = bl_pos(j, Np);  // round 0: index i sits in slot i
+      double x = 0.0;
+      if (i < N && j < N) x = 0.5 * (w_in[i + (long long)N * j] + w_in[j + (long long)N * i]);
+      Wb0[Pi * Np + Pj] = x;
+    }
   double dm = 0.0;
-  for (int i = 0; i < N; ++i) dm = fmax(dm, fabs(w_in[i + (long long)N * i]));
+  for (int i = lane; i < N; i += 32) dm = fmax(dm, fabs(w_in[i + (long long)N * i]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) dm = fmax(dm, __shfl_xor_sync(0xffffffffu, dm, o));
   const double inv_s = dm > 0.0 ? 1.0 / dm : 1.0;
   __syncthreads();
   // Rotations of round 0.
@@ -189,10 +223,9 @@ __device__ __forceinline__ int bl_solve(const double* __restrict__ w_in, int N, 
         if (rnd + 1 == NR) {
           const double* Wn = (R & 1) ? Wb0 : Wb1;  // written this round
           int need = 0;
-          for (int idx = tid; idx < NN; idx += blockDim.x) {
-            const int P = idx / Np, Q = idx - (idx / Np) * Np;
-            if (P < Q && jacobi_needed(Wn[P * Np + P], Wn[Q * Np + Q], Wn[P * Np + Q], inv_s)) need = 1;
-          }
+          for (int P = warp; P < Np; P += (int)(blockDim.x >> 5))
+            for (int Q = lane; Q < Np; Q += 32)
+              if (P < Q && jacobi_needed(Wn[P * Np + P], Wn[Q * Np + Q], Wn[P * Np + Q], inv_s)) need = 1;
           if (!__syncthreads_or(need)) stop = true;
         }
       }
@@ -203,8 +236,9 @@ __device__ __forceinline__ int bl_solve(const double* __restrict__ w_in, int N, 
       }
     }
   };
-  const int vi0 = vw ? (ai - WU) * (vrow ? 32 : vrows) : 0;
-  double v[vrow ? VN : 2 * kBlVRows];
+  // V warp: part vp of the rows vr0 + lane
+  const int vp = vw ? (ai - WU) % PARTS : 0, vr0 = vw ? (ai - WU) / PARTS * 32 : 0;
+  double v[VL];
   if (ww) {
     // W thread: upper block (a, b) of W, a <= b (a = -1 for none)
     int a = -1, b = 0;
@@ -229,7 +263,7 @@ __device__ __forceinline__ int bl_solve(const double* __restrict__ w_in, int N, 
       double ca, sa, cbv, sb;
       rot_from_cs32(cs_[a], ca, sa);
       rot_from_cs32(cs_[b], cbv, sb);
-      if (vrow && a == b) pcd[cb][a] = make_double2(ca, sa);  // for V, next round
+      if (a == b) pcd[cb][a] = make_double2(ca, sa);  // for V, next round
       // Only the upper triangle (row <= column) of W is kept.  Block (a, b), a < b, lies
       // wholly above the diagonal; a diagonal block's lower entry is its upper one.
       const double2 r0v = *reinterpret_cast<const double2*>(&W[(2 * a) * Np + 2 * b]);
@@ -250,41 +284,27 @@ __device__ __forceinline__ int bl_solve(const double* __restrict__ w_in, int N, 
       Wn[min(r1, q1) * Np + max(r1, q1)] = y11;
     });
   } else if (vw) {
-    // V, identity at the round-0 positions.  Row-resident: lane l of V warp j holds row
-    // i = 32 j + l = vi0 + l, entry P in v[P].  Otherwise components vi0 .. vi0 + vrows - 1, entry
-    // u of positions 2 lane and 2 lane + 1 in v[u] and v[kBlVRows + u].
-    if constexpr (vrow) {
-      const int Pi = vi0 + lane < N ? bl_pos(vi0 + lane, Np) : -1;
+    // V, identity at the round-0 positions.
+    const int row = vr0 + lane;
+    const int Pi = row < N ? bl_pos(row, Np) : -1;
+    double* const up0 = &xup[0][vp][row];  // written by this part for the next one
+    double* const dn0 = &xdn[0][vp][row];
+    auto role = [&](auto np_, auto part_) {
+      constexpr int NP = decltype(np_)::value, PART = decltype(part_)::value;
+      constexpr int K0 = bl_first(NP, PART);
 #pragma unroll
-      for (int P = 0; P < VN; ++P) v[P] = (P == Pi) ? 1.0 : 0.0;
+      for (int e = 0; e < VL; ++e) v[e] = (2 * K0 + e == Pi) ? 1.0 : 0.0;
+      auto apply = [&](int r) {  // round r, after picking up what round r - 1 carried over
+        const int w = (r & 1) * PARTS * VR, o = ((r & 1) ^ 1) * PARTS * VR;
+        if (r > 0) bl_vpart_take<NP, PART, VL>(v, up0 + o - VR, dn0 + o + VR);
+        bl_vpart_round<NP, PART, VL>(v, pcd[r & 1], dn0 + w, up0 + w);
+      };
       rounds([&](int) {
-        if (R > 0) bl_vrow_apply<VN>(Np, v, pcd[(R & 1) ^ 1]);  // the previous round's rotations
+        if (R > 0) apply(R - 1);
       });
-      if (R > 0) bl_vrow_apply<VN>(Np, v, pcd[(R - 1) & 1]);  // and the last round's
-    } else {
-#pragma unroll
-      for (int u = 0; u < kBlVRows; ++u) {
-        const int i = vi0 + u;
-        const int P = (u < vrows && i < N) ? bl_pos(i, Np) : -1;
-        v[u] = (P == 2 * lane) ? 1.0 : 0.0;
-        v[kBlVRows + u] = (P == 2 * lane + 1) ? 1.0 : 0.0;
-      }
-      rounds([&](int) {
-        const float2* cs_ = pcs[R & 1];
-        double c = 1.0, sn = 0.0;
-        if (lane < H) rot_from_cs32(cs_[lane], c, sn);
-#pragma unroll
-        for (int u = 0; u < kBlVRows; ++u) {
-          if (u >= vrows) break;  // uniform across the warp
-          const double n0 = v[u] * c - v[kBlVRows + u] * sn;
-          const double n1 = v[u] * sn + v[kBlVRows + u] * c;
-          const double dn = __shfl_down_sync(0xffffffffu, n0, 1);  // lane k+1's even entry
-          const double up = __shfl_up_sync(0xffffffffu, n1, 1);    // lane k-1's odd entry
-          v[u] = lane == 0 ? n0 : (lane == H - 1 ? n1 : dn);
-          v[kBlVRows + u] = lane == 0 ? dn : up;
-        }
-      });
-    }
+      if (R > 0) apply(R - 1);
+    };
+    bl_dispatch<VN>(Np, vp, role);
   } else if (warp == PW) {
     // Rotation of pair `lane` in the next round.  Its two indices sit at the current positions
     // P = imv[2 lane], Q = imv[2 lane + 1]; the three entries of J^T W J it needs come from the
@@ -353,23 +373,19 @@ __device__ __forceinline__ int bl_solve(const double* __restrict__ w_in, int N, 
     evals[rank] = dg[a];
   }
   __syncthreads();
-  if constexpr (vrow) {
-    if (vw && vi0 + lane < N) {
+  if (vw && vr0 + lane < N) {
+    const int row = vr0 + lane, o = ((R - 1) & 1) * PARTS * VR;
+    auto out = [&](auto np_, auto part_) {
+      constexpr int NP = decltype(np_)::value, PART = decltype(part_)::value;
+      constexpr int K0 = bl_first(NP, PART), K1 = bl_first(NP, PART + 1);
+      if (R > 0) bl_vpart_take<NP, PART, VL>(v, &xup[0][vp][row] + o - VR, &xdn[0][vp][row] + o + VR);
 #pragma unroll
-      for (int P = 0; P < VN; ++P) {
-        const int a = P < Np ? pidx[P] : -1;  // index at position P
-        if (a >= 0) evecs[vi0 + lane + (long long)N * rk[a]] = v[P];
+      for (int e = 0; e < 2 * (K1 - K0); ++e) {
+        const int a = pidx[2 * K0 + e];  // index at this position
+        if (a >= 0) evecs[row + (long long)N * rk[a]] = v[e];
       }
-    }
-  } else if (vw && lane < H) {
-    const int a0 = pidx[2 * lane], a1 = pidx[2 * lane + 1];  // indices at this lane's positions
-#pragma unroll
-    for (int u = 0; u < kBlVRows; ++u) {
-      const int i = vi0 + u;
-      if (u >= vrows || i >= N) break;
-      if (a0 >= 0) evecs[i + (long long)N * rk[a0]] = v[u];
-      if (a1 >= 0) evecs[i + (long long)N * rk[a1]] = v[kBlVRows + u];
-    }
+    };
+    bl_dispatch<VN>(Np, vp, out);
   }
   __syncthreads();
   return converged ? sweep : max_sweeps + 1;

@@ -23,14 +23,21 @@ __device__ __forceinline__ bool jacobi_needed(double app, double aqq, double apq
 // so two reciprocal square roots (h = x rsqrt(x)) give (c, s) with no division.  Both factors of s
 // carry small relative errors, so the rotation leaves ~1e-7 |a_pq| behind however small the
 // angle.  (1, 0) when the pair is not rotated.  The skip test runs in FP64 beside the FP32 path.
+// The hardware's approximate rsqrt gives the bits of rsqrtf for normal arguments (a rotated pair has
+// x >= 4e-28) without its handling of subnormal ones, which lengthened the chain by 60 cycles.
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
 __device__ __forceinline__ float2 jacobi_cs32(double app, double aqq, double apq, double inv_s) {
   const double ps = app * inv_s, qs = aqq * inv_s, as = apq * inv_s;
   const bool need = fabs(as) > 1e-14 && as * as > 1e-24 * fabs(ps * qs);
   const float d = (float)(qs - ps), e = 2.0f * (float)as;
   const float x = fmaf(d, d, e * e);
-  const float h = need ? x * rsqrtf(x) : 1.0f;
+  const float h = need ? x * rsqrt_approx(x) : 1.0f;
   const float u = h + fabsf(d);
-  const float w = rsqrtf(2.0f * h * u);
+  const float w = rsqrt_approx(2.0f * h * u);
   const float c = u * w, s = (d >= 0.0f ? e : -e) * w;
   return need ? make_float2(c, s) : make_float2(1.0f, 0.0f);
 }
@@ -45,13 +52,6 @@ __device__ __forceinline__ void rot_from_cs32(float2 r, double& c, double& s) {
   const double g = fma(dl, fma(dl, 0.375, -0.5), 1.0);
   c = c0 * g;
   s = s0 * g;
-}
-
-__device__ __forceinline__ bool jacobi_rotation(double app, double aqq, double apq, double inv_s, double& c,
-                                                double& s) {
-  const float2 r = jacobi_cs32(app, aqq, apq, inv_s);
-  rot_from_cs32(r, c, s);
-  return r.y != 0.0f;
 }
 
 }  // namespace ttr

@@ -135,3 +135,35 @@ def test_project_fp32_edges(gpu, m, n, N):
     ref = q.astype(np.float64).T @ a.astype(np.float64)
     bound = 8 * np.sqrt(m) * U32 * (np.linalg.norm(q, axis=0)[:, None] * np.linalg.norm(a, axis=0)[None, :])
     assert np.all(np.abs(y - ref) <= bound)
+
+
+@pytest.mark.parametrize("rank", [1, 4, 9, 20, 32])
+def test_batched_edges(gpu, rank):
+    """Tensors of that rank without noise come back up to the rounding of FP32 chains: a step of a tensor with
+    sides m x c multiplies along m or c, relative errors of that length u, taken as 8x."""
+    shapes = [(32, 200), (33, 33), (31, 1000), (700, 32), (1, 9), (9, 1), (5, 3, 2), (200, 3),  # exact steps' limits
+              (192, 40), (193, 40), (384, 37), (385, 37), (512, 33),                          # rows per pass of a sketch
+              (7, 70, 33), (34, 16, 36), (13, 11, 17, 5), (2, 3, 2, 3, 2, 3)]
+    for order in sorted({len(n) for n in shapes}):
+        xs = []
+        for k, n in enumerate(shapes):
+            r = [1] + [min(rank, int(np.prod(n[:j])), int(np.prod(n[j:]))) for j in range(1, len(n))] + [1]
+            if len(n) == order:
+                xs.append(oracle.make_tt_tensor(list(n), r, 0.0, seed=100 * rank + k))
+        for x, (cores, ranks, _) in zip(xs, _ttr().tt_svd_batched(xs, eps=0.0, rmax=rank)):
+            err = oracle.rel_error(x, oracle.tt_full([c.double().cpu().numpy() for c in cores]))
+            assert err <= 8 * (x.ndim - 1) * max(max(x.shape), 64) * U32, (x.shape, ranks, err)
+
+
+@pytest.mark.parametrize("N", [3, 4, 6, 7, 8, 9, 13, 30, 34, 48, 62])
+def test_syev_row_parts(gpu, N):
+    """Rows of eigenvectors split over four warps: uneven splits, one pair per warp, fewer pairs than warps."""
+    import torch
+    rng = np.random.default_rng(N)
+    q = np.linalg.qr(rng.standard_normal((N, N)))[0]
+    w = (q * np.logspace(0, -4, N)) @ q.T
+    ev, vec, _ = _ttr().syev(torch.from_numpy(w).to(gpu))
+    ev, vec = ev.cpu().numpy(), vec.cpu().numpy()
+    assert np.max(np.abs(ev - np.logspace(0, -4, N))) < 1e-11
+    assert np.linalg.norm(w @ vec - vec * ev) < 1e-10 * N
+    assert np.linalg.norm(vec.T @ vec - np.eye(N)) < 1e-12 * N
