@@ -187,6 +187,10 @@ __global__ void __launch_bounds__(1024) k_syev_blw(const double* __restrict__ w_
   __syncthreads();
   const int NWB = H * (H + 1) / 2;
   constexpr int MAXIT = (64 * 65 / 2 + NE - 1) / NE;
+  // With at most a block per thread (N <= 86) the rotation warps are the longer part, and their 12 loads
+  // would queue behind the other warps' for a third of the round: those wait until they are issued (a
+  // round at N = 72: 0.94 -> 0.77 us; at N = 128 the blocks are the longer part, and waiting costs 8 %).
+  const bool first = NWB <= NE;
   // per block of this thread: the pair indices (a | b << 8, -1 for none), the offsets of its two
   // rows in W and of its four entries' next-round upper positions (fixed over the rounds)
   int dsc[MAXIT], ldo[MAXIT], sto[MAXIT][4];
@@ -244,6 +248,7 @@ __global__ void __launch_bounds__(1024) k_syev_blw(const double* __restrict__ w_
       double* Wn = cb ? Wb0 : Wb1;
       const double2* cs_ = pcs[cb];
       if (warp < RW0) {
+        if (first) asm volatile("bar.sync 1, 1024;" ::: "memory");
 #pragma unroll
         for (int u = 0; u < MAXIT; ++u) {
           const int dd = dsc[u];
@@ -265,30 +270,37 @@ __global__ void __launch_bounds__(1024) k_syev_blw(const double* __restrict__ w_
           if (a != b) Wn[sto[u][2]] = y10;
           Wn[sto[u][3]] = y11;
         }
-      } else if (rl < H) {
+      } else {
+        const double2 csP = cs_[aP], csQ = cs_[aQ];
+        double we[10];
+#pragma unroll
+        for (int e = 0; e < 10; ++e) we[e] = W[wo[e]];
+        if (first) asm volatile("bar.arrive 1, 1024;" ::: "memory");
         const int rn = (rnd + 1 == NR) ? 0 : rnd + 1;
-        bool live = true;
+        bool live = rl < H;
         if (Np != N) {
           const int xs = bl_slot(Np - 1, rn, NR);
-          live = (xs != rl) && (xs != Np - 1 - rl);
+          live = live && (xs != rl) && (xs != Np - 1 - rl);
         }
         float2 r = make_float2(1.0f, 0.0f);
         if (live) {
-          const double cP = cs_[aP].x, sP = cs_[aP].y, cQ = cs_[aQ].x, sQ = cs_[aQ].y;
+          const double cP = csP.x, sP = csP.y, cQ = csQ.x, sQ = csQ.y;
           const double tP0 = xP ? sP : cP, tP1 = xP ? cP : -sP;
           const double tQ0 = xQ ? sQ : cQ, tQ1 = xQ ? cQ : -sQ;
-          const double p0 = tP0 * W[wo[0]] + tP1 * W[wo[1]];
-          const double p1 = tP0 * W[wo[1]] + tP1 * W[wo[2]];
-          const double q0 = tQ0 * W[wo[3]] + tQ1 * W[wo[4]];
-          const double q1 = tQ0 * W[wo[4]] + tQ1 * W[wo[5]];
-          const double m0 = tP0 * W[wo[6]] + tP1 * W[wo[7]];
-          const double m1 = tP0 * W[wo[8]] + tP1 * W[wo[9]];
+          const double p0 = tP0 * we[0] + tP1 * we[1];
+          const double p1 = tP0 * we[1] + tP1 * we[2];
+          const double q0 = tQ0 * we[3] + tQ1 * we[4];
+          const double q1 = tQ0 * we[4] + tQ1 * we[5];
+          const double m0 = tP0 * we[6] + tP1 * we[7];
+          const double m1 = tP0 * we[8] + tP1 * we[9];
           r = jacobi_cs32(p0 * tP0 + p1 * tP1, q0 * tQ0 + q1 * tQ1, m0 * tQ0 + m1 * tQ1, inv_s);
         }
-        double c, sn;
-        rot_from_cs32(r, c, sn);
-        pcs[cb ^ 1][rl] = make_double2(c, sn);
-        tlog[(size_t)(R + 1) * H + rl] = make_double2(c, sn);  // rotations of round R + 1
+        if (rl < H) {
+          double c, sn;
+          rot_from_cs32(r, c, sn);
+          pcs[cb ^ 1][rl] = make_double2(c, sn);
+          tlog[(size_t)(R + 1) * H + rl] = make_double2(c, sn);  // rotations of round R + 1
+        }
       }
       __syncthreads();
       if (rnd + 1 == NR) {
