@@ -167,3 +167,17 @@ def test_syev_row_parts(gpu, N):
     assert np.max(np.abs(ev - np.logspace(0, -4, N))) < 1e-11
     assert np.linalg.norm(w @ vec - vec * ev) < 1e-10 * N
     assert np.linalg.norm(vec.T @ vec - np.eye(N)) < 1e-12 * N
+
+
+@pytest.mark.parametrize("width", [65, 66, 71, 72, 73, 80, 101, 127, 128])
+def test_wide_sketch_singular_values(gpu, width):
+    """A sketch of 65 to 128 columns of which 16 are kept goes through the subspace eigen-solver (rows padded to a
+    multiple of 8).  FP32 chains along the 130 rows: 130 u of the largest singular value."""
+    n, r = (130, 12, 11), 4
+    rng = np.random.default_rng(width)
+    cores = [rng.standard_normal((r, k, r)) for k in n]
+    x = oracle.tr_full(cores)
+    x = (x + 1e-5 * np.linalg.norm(x) / np.sqrt(x.size) * rng.standard_normal(x.shape)).astype(np.float32)
+    res = _ttr().tr_svd(_dev(x, gpu), [r, r, 11, r], gemm="fp32", oversample=width - r * r, power_iters=1)
+    ref = np.linalg.svd(np.reshape(x, (130, -1), order="F").astype(np.float64), compute_uv=False)
+    assert np.all(np.abs(res.sigmas[0][:r * r] - ref[:r * r]) <= 130 * U32 * ref[0])
