@@ -1344,7 +1344,7 @@ extern "C" int tt_rel_error(tt_ctx* c, const float* x, int d, const int* n, cons
   // Left part of a split after core k (k cores): (r0, P_k, r_k); right part: (r_k, N_k, r_d).  Any
   // split gives the same product; its cost is the final contraction (r0 r_k FMAs per element, in whole
   // tiles) plus the merges of both sides, least where both sides are small.  Scratch (FP64): the
-  // last two merges of a side, at most what merging everything right of core 1 takes.
+  // last two merges of a side, within the largest merge of everything right of core 1 wherever a cut allows.
   std::vector<long long> P((size_t)d + 1, 1);
   for (int k = 0; k < d; ++k) P[(size_t)k + 1] = P[(size_t)k] * n[k];
   auto right_of = [&](int k) { return P[(size_t)d] / P[(size_t)k]; };  // n_k ... n_{d-1}
@@ -1372,14 +1372,14 @@ extern "C" int tt_rel_error(tt_ctx* c, const float* x, int d, const int* n, cons
     for (int j = 2; j <= k; ++j) cost += (double)left_elems(j) * r[j - 1];
     for (int j = d - 2; j >= k; --j) cost += (double)right_elems(j) * r[j + 1];
     const Bufs2 lb = left_bufs(k), rb = right_bufs(k);
-    if (k > 1 && lb.b[0] + lb.b[1] + rb.b[0] + rb.b[1] > all.b[0] + all.b[1]) continue;
+    if (lb.b[0] + lb.b[1] + rb.b[0] + rb.b[1] > std::max(all.b[0], all.b[1])) continue;
     if (best < 0.0 || cost < best) {
       best = cost;
       cut = k;
     }
   }
   const Bufs2 lb = left_bufs(cut), rb = right_bufs(cut);
-  TT_TRY(tt_ctx_reserve(c, sizeof(double) * (lb.b[0] + lb.b[1] + rb.b[0] + rb.b[1]) + 8192 + (1 << 20)));
+  TT_TRY(tt_ctx_reserve(c, sizeof(double) * (lb.b[0] + lb.b[1] + rb.b[0] + rb.b[1]) + 4096 + (1 << 20)));
   Arena a{c->arena, c->cap, 0};
   double* lbuf[2] = {a.take<double>(lb.b[0]), a.take<double>(lb.b[1])};
   double* rbuf[2] = {a.take<double>(rb.b[0]), a.take<double>(rb.b[1])};
