@@ -181,3 +181,14 @@ def test_wide_sketch_singular_values(gpu, width):
     res = _ttr().tr_svd(_dev(x, gpu), [r, r, 11, r], gemm="fp32", oversample=width - r * r, power_iters=1)
     ref = np.linalg.svd(np.reshape(x, (130, -1), order="F").astype(np.float64), compute_uv=False)
     assert np.all(np.abs(res.sigmas[0][:r * r] - ref[:r * r]) <= 130 * U32 * ref[0])
+
+
+def test_batched_two_per_sm_same_bits(gpu):
+    """A batch large enough for two tensors per SM (the kernel with fewer registers) gives the bits of a small one."""
+    import torch
+    rng = np.random.default_rng(11)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    xs = [rng.standard_normal(rng.integers(4, 40, size=3)).astype(np.float32) for _ in range(4 * sms + 8)]
+    few, many = (_ttr().tt_svd_batched(x, eps=0.3, rmax=12) for x in (xs[:40], xs))
+    for (c0, r0, e0), (c1, r1, e1) in zip(few, many):
+        assert r0 == r1 and e0 == e1 and all(torch.equal(a, b) for a, b in zip(c0, c1))
