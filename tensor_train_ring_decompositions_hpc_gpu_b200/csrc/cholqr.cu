@@ -14,6 +14,11 @@
 //    row itself in shared memory, so one code serves every N and stays in the instruction cache.
 //    Above 64 columns, and where the rows are too many for one launch, the rows are multiplied by R^-1
 //    (FP64, rounded once): no chain at all per row.
+//  * `exact` rows (the decompositions on the FP32 engine): the first pass divides in FP64 and rounds each entry
+//    once.  An FP32 reciprocal pivot makes a whole column of Q longer or shorter by up to 2^-24, which the second
+//    pass cannot mend (its factor 1 + 3e-8 rounds back), and close eigenvectors of B B^T tilt by that over their
+//    gap: interior bases of a 24^6 tensor at ranks 24 come out 3 to 5 times closer to their 64-bit values.
+//    The second pass then finds R = I to 1e-9 and has nothing to round.  256^3, ranks 16: 678 -> 680 us.
 // CholeskyQR2 of 384 x 24: 66 us before, 32 now; 1024 x 40: 79, 49; 256 x 80: 212, 132; 640 x 96 (then
 // seven launches): about 590, 187.  What is left is the chain: at 1024 x 40, per pass, 14k cycles of
 // Cholesky, 8.5k of Gram, 6k for the cluster's sum, 6k of row solves.
@@ -147,8 +152,36 @@ __device__ __forceinline__ void solve_row(float* row, int N, const float* Rf, in
   }
 }
 
-// q = y T for one row, in place, T upper triangular (FP32 rows of stride RS): panels of 8 columns from
-// the last one down, so that a panel overwrites what no later one reads.
+// The same with FP64 products, sums and reciprocals against R in FP64 (packed).
+__device__ __forceinline__ void solve_row64(float* row, int N, const double* W, const double* inv) {
+  for (int p = 0; p < N; p += CQ_P) {
+    double a[CQ_P];
+#pragma unroll
+    for (int c = 0; c < CQ_P; ++c) a[c] = p + c < N ? (double)row[p + c] : 0.0;
+    const int last = N - 1 - p;  // columns past the end repeat the last one
+#pragma unroll 2
+    for (int k = 0; k < p; ++k) {
+      const double q = -(double)row[k];
+      const double* R = W + cq_row(k, N) + p;
+#pragma unroll
+      for (int c = 0; c < CQ_P; ++c) a[c] = fma(q, R[min(c, last)], a[c]);
+    }
+#pragma unroll
+    for (int k = 0; k < CQ_P; ++k) {
+      if (p + k < N) {
+        const float qf = (float)(a[k] * inv[p + k]);
+        row[p + k] = qf;
+        const double q = -(double)qf;
+        const double* R = W + cq_row(p + k, N) + p;
+#pragma unroll
+        for (int c = k + 1; c < CQ_P; ++c) a[c] = fma(q, R[min(c, last)], a[c]);
+      }
+    }
+  }
+}
+
+// q = y T for one row, in place, T upper triangular (FP32 or FP64 rows of stride RS; products and sums in its
+// type): panels of 8 columns from the last one down, so that a panel overwrites what no later one reads.
 __device__ __forceinline__ void mul_row(float* row, int N, const float* Tf, int RS) {
   for (int p = ((N - 1) / CQ_P) * CQ_P; p >= 0; p -= CQ_P) {
     uint64_t acc[4] = {0ull, 0ull, 0ull, 0ull};
@@ -173,11 +206,35 @@ __device__ __forceinline__ void mul_row(float* row, int N, const float* Tf, int 
   }
 }
 
-// FP32 copy of the packed triangle W (rows of stride RS, zero outside it; `diag`: with its diagonal).
-__device__ void write_tri(const double* W, int N, bool diag, float* Rf, int RS) {
+__device__ __forceinline__ void mul_row(float* row, int N, const double* T, int RS) {
+  for (int p = ((N - 1) / CQ_P) * CQ_P; p >= 0; p -= CQ_P) {
+    double a[CQ_P];
+#pragma unroll
+    for (int c = 0; c < CQ_P; ++c) a[c] = 0.0;
+    const int kend = min(p + CQ_P, N);
+#pragma unroll 2
+    for (int k = 0; k < kend; ++k) {
+      const double q = (double)row[k];
+      const double2* t = reinterpret_cast<const double2*>(T + k * RS + p);
+#pragma unroll
+      for (int c = 0; c < CQ_P / 2; ++c) {
+        const double2 v = t[c];
+        a[2 * c] = fma(q, v.x, a[2 * c]);
+        a[2 * c + 1] = fma(q, v.y, a[2 * c + 1]);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < CQ_P; ++c)
+      if (p + c < N) row[p + c] = (float)a[c];
+  }
+}
+
+// Copy of the packed triangle W (FP32 or FP64 rows of stride RS, zero outside it; `diag`: with its diagonal).
+template <typename T>
+__device__ void write_tri(const double* W, int N, bool diag, T* Rf, int RS) {
   for (int k = threadIdx.x >> 5; k < N; k += CQ_T / 32)
     for (int c = threadIdx.x & 31; c < RS; c += 32)
-      Rf[k * RS + c] = (c > k - (diag ? 1 : 0) && c < N) ? (float)W[cq_row(k, N) + c] : 0.f;
+      Rf[k * RS + c] = (c > k - (diag ? 1 : 0) && c < N) ? (T)W[cq_row(k, N) + c] : T(0);
 }
 
 // Columns up to which k_cholqr_cluster solves against R; above, the chain of pivots per row is longer
@@ -208,12 +265,12 @@ CqSmem cq_smem(int N, int rpc, int cl) {
 // shared memory.  Per pass: partial Gram of the CTA's rows, summed over the cluster through
 // distributed shared memory (each rank sums one slice in rank order, then all gather the slices: the
 // same bits everywhere, so the redundant factorisations agree), Cholesky, row solves.  y64 (or null):
-// Y in FP64, rounded on the way in.  r (or null): R2 R1 (r1: N x N scratch).
+// Y in FP64, rounded on the way in.  r (or null): R2 R1 (r1: N x N scratch).  exact: see above.
 template <int TS>
 __global__ void __launch_bounds__(CQ_T, 1) k_cholqr_cluster(const double* __restrict__ y64, float* __restrict__ y,
                                                             int n, int N, long long ld, int rpc, CqSmem lay,
                                                             double* __restrict__ r, double* __restrict__ r1,
-                                                            double rel_tol) {
+                                                            double rel_tol, bool exact) {
   extern __shared__ __align__(16) unsigned char sm_cq[];
   float* const Ys = reinterpret_cast<float*>(sm_cq);                       // rpc x SN
   double* const Yd = reinterpret_cast<double*>(sm_cq + lay.ys);            // FP64 rows / group sums / panel
@@ -344,7 +401,9 @@ __global__ void __launch_bounds__(CQ_T, 1) k_cholqr_cluster(const double* __rest
         }
       }
     }
-    if (N <= CQ_SOLVE) {
+    if (exact && pass == 0) {
+      for (int i = tid; i < nl; i += CQ_T) solve_row64(Ys + i * SN, N, W, inv);
+    } else if (N <= CQ_SOLVE) {
       write_tri(W, N, false, Rf, RS);
       for (int k = tid; k < N; k += CQ_T) invf[k] = (float)inv[k];
       __syncthreads();
@@ -363,9 +422,10 @@ __global__ void __launch_bounds__(CQ_T, 1) k_cholqr_cluster(const double* __rest
   if (csize > 1) cl_sync();  // peers may still be gathering this CTA's slice
 }
 
-// W (N x N, column-major) -> R^-1 in FP32 (rows of stride RS) for k_apply_t; R in FP64 (or null).
+// W (N x N, column-major) -> R^-1 (rows of stride RS) for k_apply_t; R in FP64 (or null).
+template <typename T>
 __global__ void __launch_bounds__(CQ_T, 1) k_chol_inv(const double* __restrict__ w, int N, double rel_tol,
-                                                      float* __restrict__ tf, double* __restrict__ r_out) {
+                                                      T* __restrict__ tf, double* __restrict__ r_out) {
   extern __shared__ __align__(16) double sm_ch[];
   double* const work = sm_ch;  // panel, then the inversion's scratch
   double* const W = work + cq_inv(N);
@@ -389,16 +449,20 @@ __global__ void __launch_bounds__(CQ_T, 1) k_chol_inv(const double* __restrict__
 // Y (n x N, column-major) <- Y T, T = R^-1.  A thread owns a row: the loads and stores of a warp are
 // runs of 32 rows of a column, the row waits in the thread's own line of shared memory (odd stride),
 // so nothing but T is shared and tiles need no barrier.  HBM / FP32 FMA bound: N (N + 1) / 2 FMAs per
-// 8 N bytes (262144 x 80: 609 us before, 128 now).
+// 8 N bytes (262144 x 80: 609 us before, 128 now).  An FP64 T takes twice the shared memory, so half the rows.
+template <typename T>
+constexpr int cq_apply_rows() { return sizeof(T) == 8 ? CQ_T / 2 : CQ_T; }
+template <typename T>
 __global__ void __launch_bounds__(CQ_T) k_apply_t(float* __restrict__ y, long long n, int N, long long ld,
-                                                  const float* __restrict__ tf) {
-  extern __shared__ __align__(16) float sm_ar[];
+                                                  const T* __restrict__ tf) {
+  constexpr int ROWS = cq_apply_rows<T>();
+  extern __shared__ __align__(16) unsigned char sm_ar[];
   const int RS = (N + 7) & ~7, SN = N | 1, tid = threadIdx.x;
-  float* const Ts = sm_ar;
-  float* const row = Ts + N * RS + tid * SN;
-  for (int idx = tid; idx < N * RS; idx += CQ_T) Ts[idx] = tf[idx];
+  T* const Ts = reinterpret_cast<T*>(sm_ar);
+  float* const row = reinterpret_cast<float*>(Ts + N * RS) + tid * SN;
+  for (int idx = tid; idx < N * RS; idx += ROWS) Ts[idx] = tf[idx];
   __syncthreads();
-  for (long long j = (long long)blockIdx.x * CQ_T + tid; j < n; j += (long long)gridDim.x * CQ_T) {
+  for (long long j = (long long)blockIdx.x * ROWS + tid; j < n; j += (long long)gridDim.x * ROWS) {
     float* src = y + j;
 #pragma unroll 16
     for (int c = 0; c < N; ++c) row[c] = src[ld * c];
@@ -421,8 +485,28 @@ __global__ void k_mul_upper(const double* __restrict__ r2, const double* __restr
 
 constexpr double kCqTol = 1e-12;  // pivots below this share of the largest diagonal: dependent columns
 
+// The pass Y <- Y R^-1 of the Gram w, R^-1 through `tf` (N rows of stride RS), R to r (or null).
+template <typename T>
+int apply_inverse(float* y, long long n, int N, long long ld, const double* w, T* tf, double* r, cudaStream_t s) {
+  constexpr int ROWS = cq_apply_rows<T>();
+  const size_t csm = ((size_t)cq_inv(N) + cq_packed(N) + N) * sizeof(double);
+  const size_t asm_ = (size_t)N * cq_rstride(N) * sizeof(T) + (size_t)ROWS * (N | 1) * sizeof(float);
+  TT_TRY(smem_optin_k(k_chol_inv<T>, csm));
+  TT_TRY(smem_optin_k(k_apply_t<T>, asm_));
+  // persistent blocks (T staged once per block), as many as fit on the SMs
+  const int per_sm = std::max(1, std::min(8, (int)((size_t)dev_smem_max() / (asm_ + 1024))));
+  const int grid = (int)std::min<long long>(ceil_div_ll(n, ROWS), (long long)per_sm * dev_sms());
+  k_chol_inv<T><<<1, CQ_T, csm, s>>>(w, N, kCqTol, tf, r);
+  count_launch();
+  TT_LAUNCH_CHECK();
+  k_apply_t<T><<<grid, ROWS, asm_, s>>>(y, n, N, ld, tf);
+  count_launch();
+  TT_LAUNCH_CHECK();
+  return TT_OK;
+}
+
 int cholqr_passes(const double* y64, float* y, long long n, int N, long long ld, double* r, Arena& ws,
-                  cudaStream_t s, int passes) {
+                  cudaStream_t s, int passes, bool exact) {
   if (N <= 0 || n <= 0) return TT_OK;
   if (N > TT_MAX_SMALL) {
     set_error(TT_ERR_UNSUPPORTED, "cholqr2 width %d > %d", N, TT_MAX_SMALL);
@@ -456,8 +540,8 @@ int cholqr_passes(const double* y64, float* y, long long n, int N, long long ld,
       cfg.attrs = at;
       cfg.numAttrs = 1;
       const cudaError_t e =
-          cq_tile(N) == 4 ? cudaLaunchKernelEx(&cfg, k_cholqr_cluster<4>, y64, y, (int)n, N, ld, rpc, lay, r, r1, kCqTol)
-                          : cudaLaunchKernelEx(&cfg, k_cholqr_cluster<8>, y64, y, (int)n, N, ld, rpc, lay, r, r1, kCqTol);
+          cq_tile(N) == 4 ? cudaLaunchKernelEx(&cfg, k_cholqr_cluster<4>, y64, y, (int)n, N, ld, rpc, lay, r, r1, kCqTol, exact)
+                          : cudaLaunchKernelEx(&cfg, k_cholqr_cluster<8>, y64, y, (int)n, N, ld, rpc, lay, r, r1, kCqTol, exact);
       if (e == cudaSuccess) {
         count_launch();
         TT_LAUNCH_CHECK();
@@ -472,26 +556,16 @@ int cholqr_passes(const double* y64, float* y, long long n, int N, long long ld,
   if (y64) TT_TRY(launch_f64_to_f32_cols(y64, n, n, N, y, ld, N, s));
   double* w = ws.take<double>((size_t)N * N);
   double* r2 = ws.take<double>((size_t)N * N);
-  float* tf = ws.take<float>((size_t)N * cq_rstride(N));
+  double* tf = ws.take<double>((size_t)N * cq_rstride(N));
   if (!w || !r2 || !tf) {
     set_error(TT_ERR_NOMEM, "cholqr2 workspace");
     return TT_ERR_NOMEM;
   }
-  const size_t csm = ((size_t)cq_inv(N) + cq_packed(N) + N) * sizeof(double);
-  const size_t asm_ = ((size_t)N * cq_rstride(N) + (size_t)CQ_T * (N | 1)) * sizeof(float);
-  TT_TRY(smem_optin_k(k_chol_inv, csm));
-  TT_TRY(smem_optin_k(k_apply_t, asm_));
-  // persistent blocks (T staged once per block), as many as fit on the SMs
-  const int per_sm = std::max(1, std::min(8, (int)((size_t)dev_smem_max() / (asm_ + 1024))));
-  const int grid = (int)std::min<long long>(ceil_div_ll(n, CQ_T), (long long)per_sm * dev_sms());
   for (int pass = 0; pass < passes; ++pass) {
     TT_TRY(launch_gram(y, n, N, 1, ld, w, ws, s));
-    k_chol_inv<<<1, CQ_T, csm, s>>>(w, N, kCqTol, tf, !r ? nullptr : pass == 0 ? r1 : r2);
-    count_launch();
-    TT_LAUNCH_CHECK();
-    k_apply_t<<<grid, CQ_T, asm_, s>>>(y, n, N, ld, tf);
-    count_launch();
-    TT_LAUNCH_CHECK();
+    double* rp = !r ? nullptr : pass == 0 ? r1 : r2;
+    if (exact && pass == 0) TT_TRY(apply_inverse(y, n, N, ld, w, tf, rp, s));
+    else TT_TRY(apply_inverse(y, n, N, ld, w, reinterpret_cast<float*>(tf), rp, s));
   }
   if (r && passes == 2) {
     k_mul_upper<<<ceil_div(N * N, 256), 256, 0, s>>>(r2, r1, N, r);
@@ -505,8 +579,8 @@ int cholqr_passes(const double* y64, float* y, long long n, int N, long long ld,
 }  // namespace
 
 int launch_cholqr2(const double* y64, float* y, long long n, int N, long long ld, double* r, Arena& ws,
-                   cudaStream_t s) {
-  return cholqr_passes(y64, y, n, N, ld, r, ws, s, 2);
+                   cudaStream_t s, bool exact) {
+  return cholqr_passes(y64, y, n, N, ld, r, ws, s, 2, exact);
 }
 
 // One CholeskyQR pass: the orthonormalisation between power iterations, which only has to keep
@@ -514,7 +588,7 @@ int launch_cholqr2(const double* y64, float* y, long long n, int N, long long ld
 // columns span a graded spectrum (condition kappa) comes out with orthogonality ~kappa * 2^-24.  A
 // basis that fits one launch gets both passes there.
 int launch_orth_power(float* y, long long n, int N, long long ld, Arena& ws, cudaStream_t s) {
-  return cholqr_passes(nullptr, y, n, N, ld, nullptr, ws, s, 1);
+  return cholqr_passes(nullptr, y, n, N, ld, nullptr, ws, s, 1, false);
 }
 
 }  // namespace ttr

@@ -980,7 +980,10 @@ int run_chain(tt_ctx* c, const float* x_in, Plan P, const tt_opts& o, float* con
         TT_TRY(pass.run(TT_PASS_SKETCH, fl_pass, by_pass, [&] {
           return launch_sketch(cur, m, cols, B.omega, ksa, 1, cols, B.yd, engine, ws, c->dstat, s);
         }));
-        TT_TRY(launch_cholqr2(B.yd, B.yf, m, ksa, m, nullptr, ws, s));
+        // FP32 products and fixed ranks: Q as orthonormal as FP32 entries can be.  Beside TF32 products its rounding
+        // is nothing; adaptive ranks compare energies and not vectors.
+        const bool exact_q = !adaptive && engine == TT_GEMM_FP32;
+        TT_TRY(launch_cholqr2(B.yd, B.yf, m, ksa, m, nullptr, ws, s, exact_q && pwa == 0));
         for (int it = 0; it < pwa; ++it) {
           // Z = A^T Q written column-major (cols x ksa), the layout the sketch reads W in
           TT_TRY(pass.run(TT_PASS_PROJECT, fl_pass, by_pass, [&] {
@@ -993,7 +996,7 @@ int run_chain(tt_ctx* c, const float* x_in, Plan P, const tt_opts& o, float* con
           TT_TRY(pass.run(TT_PASS_SKETCH, fl_pass, by_pass, [&] {
             return launch_sketch(cur, m, cols, B.bt, ksa, 1, cols, B.yd, engine, ws, c->dstat, s);
           }));
-          TT_TRY(launch_cholqr2(B.yd, B.yf, m, ksa, m, nullptr, ws, s));
+          TT_TRY(launch_cholqr2(B.yd, B.yf, m, ksa, m, nullptr, ws, s, exact_q && it + 1 == pwa));
         }
         // B^T = A^T Q (cols x ksa, row-major) = B (ksa x cols, column-major).  Adaptive ranks
         // take ||B||^2 as the captured energy, which must hold ~1e-8 relative.  Tensor-core

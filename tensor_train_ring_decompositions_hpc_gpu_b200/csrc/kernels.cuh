@@ -59,8 +59,9 @@ int launch_gram32_reduce(const double* part, int nblk, int M, double* w, cudaStr
 
 // CholeskyQR2 on a tall FP32 matrix (n x N, column-major, ld), in place; y64 (or null): the matrix
 // in FP64 (ld = n), taken instead of y's contents.  Writes R (N x N, FP64, upper) when r != nullptr.
+// exact: Q's entries are rounded once in the first pass, so that Q^T Q = I to about 1e-9 instead of 1e-7.
 int launch_cholqr2(const double* y64, float* y, long long n, int N, long long ld, double* r, Arena& ws,
-                   cudaStream_t s);
+                   cudaStream_t s, bool exact = false);
 // One CholeskyQR pass (between power iterations).
 int launch_orth_power(float* y, long long n, int N, long long ld, Arena& ws, cudaStream_t s);
 
