@@ -365,9 +365,10 @@ __global__ void k_project_reduce(const float* __restrict__ part, long long n, in
   const long long total = n * N;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
-    float v = 0.f;
+    double vd = 0.0;
 #pragma unroll 8
-    for (int z = 0; z < nsplit; ++z) v += part[(long long)z * total + idx];
+    for (int z = 0; z < nsplit; ++z) vd += (double)part[(long long)z * total + idx];
+    const float v = (float)vd;
     const long long j = idx / N;
     const int c = (int)(idx - j * N);
     if (mode == OUT_ROWMAJOR) {
