@@ -64,14 +64,17 @@ __device__ __forceinline__ double ld_peer_f64(const double* p, unsigned rank) {
 // W (packed R) <- R^-1, in place, by the whole block: 8 rows at a time from the bottom.  A thread
 // pair holds a column j of those rows (the pair splits the sum over k), T[i][j] = -(sum_{k > i} R[i][k]
 // T[k][j]) / R[i][i], T[j][j] = 1 / R[j][j]; a dependent column (inv 0) comes out zero.  rt: the rows'
-// R staged k-major (N x 8), red: 8 x 128 partial sums.  Ends with a block barrier.
+// R staged k-major (N x 8, at least 8 x 8: the bottom rows' triangle is read whole, zero past N), red: 8 x 128
+// partial sums.  Ends with a block barrier.
+constexpr int cq_rt(int N) { return (N > CQ_P ? N : CQ_P) * CQ_P; }
+constexpr int cq_inv(int N) { return cq_rt(N) + CQ_P * 128; }  // doubles of both
 __device__ void invert_upper(double* W, int N, const double* inv, double* rt, double* red) {
   const int tid = threadIdx.x, j = tid & 127, h = tid >> 7;
   for (int k0 = ((N - 1) / CQ_P) * CQ_P; k0 >= 0; k0 -= CQ_P) {
     const int k1 = min(k0 + CQ_P, N);
-    for (int idx = tid; idx < (N - k0) * CQ_P; idx += CQ_T) {
+    for (int idx = tid; idx < max(N - k0, CQ_P) * CQ_P; idx += CQ_T) {
       const int k = k0 + idx / CQ_P, i = k0 + idx % CQ_P;
-      rt[(k - k0) * CQ_P + (i - k0)] = (i < N && k > i) ? W[cq_row(i, N) + k] : 0.0;
+      rt[(k - k0) * CQ_P + (i - k0)] = (k < N && k > i) ? W[cq_row(i, N) + k] : 0.0;
     }
     __syncthreads();
     double a[CQ_P];
@@ -240,7 +243,6 @@ __device__ void write_tri(const double* W, int N, bool diag, T* Rf, int RS) {
 // Columns up to which k_cholqr_cluster solves against R; above, the chain of pivots per row is longer
 // than the inversion.
 constexpr int CQ_SOLVE = 64;
-constexpr int cq_inv(int N) { return N * CQ_P + CQ_P * 128; }  // doubles of invert_upper's scratch
 constexpr int cq_tile(int N) { return N <= 56 ? 4 : 8; }  // Gram tile: 4 x 4 keeps the threads busy (N = 56: 69 against 83 us)
 
 // Shared memory of k_cholqr_cluster (bytes), `rpc` rows per CTA.
@@ -410,7 +412,7 @@ __global__ void __launch_bounds__(CQ_T, 1) k_cholqr_cluster(const double* __rest
       for (int i = tid; i < nl; i += CQ_T) solve_row(Ys + i * SN, N, Rf, RS, invf);
     } else {
       __syncthreads();  // R is out
-      invert_upper(W, N, inv, Yd, Yd + N * CQ_P);
+      invert_upper(W, N, inv, Yd, Yd + cq_rt(N));
       write_tri(W, N, true, Rf, RS);
       __syncthreads();
       for (int i = tid; i < nl; i += CQ_T) mul_row(Ys + i * SN, N, Rf, RS);
@@ -442,7 +444,7 @@ __global__ void __launch_bounds__(CQ_T, 1) k_chol_inv(const double* __restrict__
     }
     __syncthreads();
   }
-  invert_upper(W, N, inv, work, work + N * CQ_P);
+  invert_upper(W, N, inv, work, work + cq_rt(N));
   write_tri(W, N, true, tf, (N + 7) & ~7);
 }
 

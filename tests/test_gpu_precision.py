@@ -37,3 +37,32 @@ def test_fp32_bases_are_orthonormal(gpu, shape, ranks, power):
         if u.shape[0] > 4 * u.shape[1] and u.shape[0] > 130:  # sketched steps
             defect = np.abs(u.T @ u - np.eye(u.shape[1])).max()
             assert defect <= 12 * U32 * np.sqrt(3.0 / u.shape[0]), (k, u.shape, defect)
+
+
+def _fill_shared_memory_with_nan(dev):
+    """Grams of NaN in either layout: what a later kernel finds in shared memory that it does not write is NaN."""
+    import ctypes as C
+    import torch
+    ttr = _ttr()
+    z = torch.full((200000, 128), float("nan"), device=dev)
+    w = torch.empty((128, 128), dtype=torch.float64, device=dev)
+    for rs, cs in ((128, 1), (1, 200000)):
+        ttr._lib.check(ttr.lib().tt_k_gram_tall(ttr._ctx_for(0), C.c_void_p(z.data_ptr()), 200000, 128, rs, cs,
+                                                C.c_void_p(w.data_ptr())))
+
+
+@pytest.mark.parametrize("n,N", [(200000, 3), (100000, 7), (60000, 10), (60000, 27), (60001, 54), (60000, 101)])
+def test_cholqr2_tall_ragged(gpu, n, N):
+    """More rows than one launch holds and widths that are no multiple of 8, after a kernel that left NaN in shared
+    memory.  Bounds as in test_cholqr2_edges."""
+    import torch
+    g = torch.Generator(device="cpu").manual_seed(n + N)
+    y = torch.randn((N, n), generator=g).to(gpu).t()
+    yd = y.double()
+    _fill_shared_memory_with_nan(gpu)
+    q, r = _ttr().cholqr2(y)
+    qd = q.double()
+    tol = 4 * U32 * N * max(1.0, np.sqrt(N))
+    eye = torch.eye(N, dtype=torch.float64, device=gpu)
+    assert float(torch.linalg.norm(qd.t() @ qd - eye)) <= tol
+    assert float(torch.linalg.norm(qd @ r - yd)) <= tol * float(torch.linalg.norm(yd))
