@@ -12,8 +12,8 @@
 //    loads of a warp are consecutive words; row groups are summed from shared memory.
 //  * Rows are solved in panels of 8 columns: 32 independent sums per row instead of 4 per column, the
 //    row itself in shared memory, so one code serves every N and stays in the instruction cache.
-//    Above 64 columns, and where the rows are too many for one launch, the rows are multiplied by R^-1
-//    (FP64, rounded once): no chain at all per row.
+//    Above 64 columns (80 for few rows), and where the rows are too many for one launch, the rows are
+//    multiplied by R^-1 (FP64, rounded once): no chain at all per row.
 //  * `exact` rows (the decompositions on the FP32 engine): the first pass divides in FP64 and rounds each entry
 //    once.  An FP32 reciprocal pivot makes a whole column of Q longer or shorter by up to 2^-24, which the second
 //    pass cannot mend (its factor 1 + 3e-8 rounds back), and close eigenvectors of B B^T tilt by that over their
@@ -240,22 +240,28 @@ __device__ void write_tri(const double* W, int N, bool diag, T* Rf, int RS) {
       Rf[k * RS + c] = (c > k - (diag ? 1 : 0) && c < N) ? (T)W[cq_row(k, N) + c] : T(0);
 }
 
-// Columns up to which k_cholqr_cluster solves against R; above, the chain of pivots per row is longer
-// than the inversion.
-constexpr int CQ_SOLVE = 64;
+// Whether k_cholqr_cluster solves its rows against R (four partial sums an entry) or multiplies them by R^-1 (one
+// chain of FP32 products with a rounded inverse).  Solving is the more exact form and, up to 80 columns, the faster
+// one (CholeskyQR2 of 256 x 80: 118 us, 151 with the inverse; 448 x 72: 107, 135; 1024 x 80: 132, 170).  Above 64
+// columns it ends all the same where the rows (odd multiples of 16 bytes) and W no longer fit 206,528 bytes of one
+// CTA: a TF32 decomposition without power iterations follows the rounding of its noise columns (3e-5 of a core when
+// the form changes), so the sizes keep the form that they have always had.
+__host__ __device__ constexpr bool cq_solves(long long n, int N) {
+  return N <= 64 || (N <= 80 && 16 * n * (((N + 3) / 4) | 1) + 8 * ((N * N + 1) & ~1) <= 206528);
+}
 constexpr int cq_tile(int N) { return N <= 56 ? 4 : 8; }  // Gram tile: 4 x 4 keeps the threads busy (N = 56: 69 against 83 us)
 
 // Shared memory of k_cholqr_cluster (bytes), `rpc` rows per CTA.
 struct CqSmem {
   size_t ys, work, part, w, slice, total;
 };
-CqSmem cq_smem(int N, int rpc, int cl) {
+CqSmem cq_smem(long long n, int N, int rpc, int cl) {
   auto up = [](size_t b) { return (b + 15) & ~size_t(15); };
   CqSmem s;
   const size_t E = (size_t)cq_packed(N), rf = (size_t)N * cq_rstride(N) * 4;
   const int ts = cq_tile(N), tt = (N + ts - 1) / ts;
   s.ys = up((size_t)rpc * (N | 1) * 4);
-  s.work = up(8 * (size_t)std::max({CQ_RC * tt * ts, CQ_T * 16, cq_pan(N), N > CQ_SOLVE ? cq_inv(N) : 0}));
+  s.work = up(8 * (size_t)std::max({CQ_RC * tt * ts, CQ_T * 16, cq_pan(N), cq_solves(n, N) ? 0 : cq_inv(N)}));
   s.part = up(std::max(E * 8, rf));
   s.w = up(E * 8);
   s.slice = up((E + cl - 1) / cl * 8);
@@ -405,7 +411,7 @@ __global__ void __launch_bounds__(CQ_T, 1) k_cholqr_cluster(const double* __rest
     }
     if (exact && pass == 0) {
       for (int i = tid; i < nl; i += CQ_T) solve_row64(Ys + i * SN, N, W, inv);
-    } else if (N <= CQ_SOLVE) {
+    } else if (cq_solves(n, N)) {
       write_tri(W, N, false, Rf, RS);
       for (int k = tid; k < N; k += CQ_T) invf[k] = (float)inv[k];
       __syncthreads();
@@ -525,7 +531,7 @@ int cholqr_passes(const double* y64, float* y, long long n, int N, long long ld,
   if (n <= (1LL << 20)) {
     for (int cl = (int)std::min<long long>(8, ceil_div_ll(n, 64)); cl <= 8; ++cl) {
       const int rpc = (int)ceil_div_ll(n, cl);
-      const CqSmem lay = cq_smem(N, rpc, cl);
+      const CqSmem lay = cq_smem(n, N, rpc, cl);
       if (lay.total > (size_t)dev_smem_max()) continue;
       TT_TRY(smem_optin_k(k_cholqr_cluster<4>, dev_smem_max()));
       TT_TRY(smem_optin_k(k_cholqr_cluster<8>, dev_smem_max()));

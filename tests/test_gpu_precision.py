@@ -66,3 +66,23 @@ def test_cholqr2_tall_ragged(gpu, n, N):
     eye = torch.eye(N, dtype=torch.float64, device=gpu)
     assert float(torch.linalg.norm(qd.t() @ qd - eye)) <= tol
     assert float(torch.linalg.norm(qd @ r - yd)) <= tol * float(torch.linalg.norm(yd))
+
+
+@pytest.mark.parametrize("n,N", [(256, 65), (400, 72), (300, 77), (462, 80)])
+def test_cholqr2_wide_rows_are_solved(gpu, n, N):
+    """65 to 80 columns of few rows: q R = y is solved row by row, like the narrower ones, and not multiplied by an
+    inverse rounded to FP32.  R = 1 / 2 x normal above a unit diagonal has a condition of 1e4 and more.  Solving leaves
+    Q (Q^T Y) - Y at the rounding of two passes' sums of N / 4 terms, 2 u sqrt(N / 4) of |Y|, of which 2x is allowed; a
+    rounded inverse leaves u |Y R^-1| |R|, several times that bound."""
+    import ctypes as C
+    import torch
+    ttr = _ttr()
+    rng = np.random.default_rng(N)
+    r = np.triu(rng.standard_normal((N, N)), 1) * 0.5 + np.diag(np.ones(N))
+    q0 = np.linalg.qr(rng.standard_normal((n, N)))[0]
+    y = (q0 @ r).astype(np.float32)
+    yt = torch.from_numpy(np.ascontiguousarray(y.T)).to(gpu)
+    ttr._lib.check(ttr.lib().tt_k_cholqr2(ttr._ctx_for(0), C.c_void_p(yt.data_ptr()), n, N, n, None))
+    q = yt.t().double().cpu().numpy()
+    yd = y.astype(np.float64)
+    assert np.linalg.norm(q @ (q.T @ yd) - yd) <= 4 * U32 * np.sqrt(N / 4) * np.linalg.norm(yd)
