@@ -706,12 +706,14 @@ int run_chain(tt_ctx* c, const float* x_in, Plan P, const tt_opts& o, float* con
   // CUDA-core kernels in every form (FP32 products, FP64 sums), whose result
   // resolves eigenvalues down to ~1e-9 of the largest; the tensor cores' truncating FP32 accumulation
   // would bias the small ones.  `precise` (adaptive ranks: energies to ~1e-8 relative) keeps short
-  // unfoldings, whose few partial sums do not average the FP32 rounding out, on FP64 products.  Wider:
+  // unfoldings, whose few partial sums do not average the FP32 rounding out, on FP64 products: below 2^16
+  // columns where the TMA can address the rows (m a multiple of 4), below 2^22 where it cannot.  Wider:
   // tensor cores when allowed, else FP64 products.
   auto gram_rows = [&](const float* a, long long mm, long long nc, double* w, int eng, bool precise) -> int {
     if (mm <= 32 && (!precise || nc >= (1LL << 16))) {
       int rc = launch_gram32x(a, nc, (int)mm, w, ws, c->dstat, s);
-      if (rc == TT_ERR_UNSUPPORTED) rc = launch_gram32u(a, nc, (int)mm, w, ws, s);
+      if (rc == TT_ERR_UNSUPPORTED && (!precise || nc >= (1LL << 22)))
+        rc = launch_gram32u(a, nc, (int)mm, w, ws, s);
       if (rc != TT_ERR_UNSUPPORTED) return rc;
     }
     if (eng == TT_GEMM_TC && !precise && mm > 32) {

@@ -86,3 +86,17 @@ def test_cholqr2_wide_rows_are_solved(gpu, n, N):
     q = yt.t().double().cpu().numpy()
     yd = y.astype(np.float64)
     assert np.linalg.norm(q @ (q.T @ yd) - yd) <= 4 * U32 * np.sqrt(N / 4) * np.linalg.norm(yd)
+
+
+@pytest.mark.parametrize("m", [17, 30, 31])
+def test_adaptive_gram_of_unaligned_rows(gpu, m):
+    """A tolerance run reads the discarded energy off the Gram of its first unfolding: 1e-8 of the whole here, of rows
+    that are almost constant, so that FP32 products and sums would all round the same way (1e-7).  FP64 ones leave
+    2^-53 of the whole per term, n m^2 terms at the worst: 1e-4 of the discarded energy at most."""
+    n = 70000
+    rng = np.random.default_rng(m)
+    x = ((1.1 + 0.01 * np.arange(m))[:, None] * 0.9 * np.ones(n) + 1e-4 * rng.standard_normal((m, n))).astype(np.float32)
+    res = _ttr().tt_svd(_dev(x, gpu), [1, 1, 1], eps=1e-3)
+    lam = np.linalg.eigvalsh(x.astype(np.float64) @ x.T.astype(np.float64))
+    want = np.sqrt(lam[:-1].sum() / lam.sum())
+    assert abs(res.est_rel_err - want) <= 1e-4 * want
