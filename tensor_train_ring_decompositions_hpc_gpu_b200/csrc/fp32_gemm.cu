@@ -200,14 +200,22 @@ int sk_width(int N, int* blocks) {
 }
 
 // Splits of the long dimension: as many blocks as fill the SMs twice, each a whole chunk per warp at
-// least (8 warps x 8 columns; a 384 x 320 unfolding then takes 30 blocks and 7 us instead of 2 and 39).
+// least (8 warps x 8 columns; a 384 x 320 unfolding then takes 30 blocks and 7 us instead of 2 and 39).  More
+// often than twice where a warp's FP32 chain, an eighth of a split, would be longer than that of splits that fill
+// the SMs four times with blocks of 256 rows (and 256 columns): sketches above 64 columns, which take two blocks of
+// columns (600 x 950k, 96 columns: chains of 8,488 -> 4,096 columns in the same 2.5 ms).
 void sketch_split_plan(long long m, long long n, int N, long long* jchunk, int* nsplit) {
   int cb;
   const int NT = sk_width(N, &cb);
   const long long tiles = ceil_div_ll(m, SK_ROWS) * cb;
-  const long long splits = std::max<long long>(1, 2LL * sk_blocks(NT) * dev_sms() / tiles);
   constexpr long long unit = SK_W * SK_JC;
-  const long long jc = ceil_div_ll(ceil_div_ll(n, splits), unit) * unit;
+  const long long chain = std::max(256LL, ceil_div_ll(n, std::max(1LL, 4LL * dev_sms() / ceil_div_ll(m, 256))));
+  long long jc = unit;
+  for (int waves = 2;; ++waves) {
+    const long long splits = std::max<long long>(1, (long long)waves * sk_blocks(NT) * dev_sms() / tiles);
+    jc = ceil_div_ll(ceil_div_ll(n, splits), unit) * unit;
+    if (jc <= SK_W * chain) break;
+  }
   *jchunk = jc;
   *nsplit = (int)ceil_div_ll(n, jc);
 }

@@ -100,3 +100,15 @@ def test_adaptive_gram_of_unaligned_rows(gpu, m):
     lam = np.linalg.eigvalsh(x.astype(np.float64) @ x.T.astype(np.float64))
     want = np.sqrt(lam[:-1].sum() / lam.sum())
     assert abs(res.est_rel_err - want) <= 1e-4 * want
+
+
+@pytest.mark.parametrize("m,n,N", [(600, 200000, 96), (256, 600000, 80), (4096, 37000, 64), (600, 200000, 24),
+                                   (130, 600000, 128)])
+def test_sketch_fp32_chain_length(gpu, m, n, N):
+    """FP32 sums of a sketch run over at most 1024 of these columns.  Products of 1 + 2^-14 add up exactly as long as
+    the sum is below 1024 and lose 2^-14 each from there on; everything after the chains is FP64."""
+    import torch
+    a = torch.ones((n, m), device=gpu).t()
+    w = torch.full((N, n), 1.0 + 2.0 ** -14, device=gpu).t()
+    y = _ttr().sketch(a, w, "fp32")
+    assert torch.all(y.double() == n * (1.0 + 2.0 ** -14))
