@@ -37,6 +37,8 @@ struct tt_ctx {
   cudaStream_t stream = nullptr;
   char* arena = nullptr;
   size_t cap = 0;
+  char* extra = nullptr;  // scratch of replanned steps that the arena's is too small for (grow_scratch)
+  size_t extra_cap = 0;
   DevStatus* dstat = nullptr;
   DevStatus* hstat = nullptr;
   double* dsig = nullptr;  // TT_MAX_ORDER x TT_STATS_MAX_SIGMA
@@ -109,6 +111,7 @@ extern "C" int tt_ctx_destroy(tt_ctx* c) {
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   if (c->arena) cudaFree(c->arena);
+  if (c->extra) cudaFree(c->extra);
   if (c->dstat) cudaFree(c->dstat);
   if (c->hstat) cudaFreeHost(c->hstat);
   if (c->dsig) cudaFree(c->dsig);
@@ -509,6 +512,30 @@ int carve(tt_ctx* c, const Plan& P, bool host_io, Bufs& B, Arena& ws) {
   return TT_OK;
 }
 
+// Scratch of at least `bytes` for the steps to come.  Fewer rows than planned can take more of it (other splits, an
+// exact Gram and its eigen-solve instead of a sketch), and the arena, whose other buffers hold data, cannot grow in
+// the middle of a run: a second buffer of the context takes its place.  Where it cannot be had `ws` stays as it is.
+void grow_scratch(tt_ctx* c, size_t bytes, Arena& ws) {
+  if (bytes <= ws.cap) return;
+  if (bytes > c->extra_cap) {
+    bytes = (bytes + (1u << 20) - 1) & ~size_t((1u << 20) - 1);
+    if (c->alloc_limit && c->cap + bytes > c->alloc_limit) return;
+    if (c->extra) {
+      cudaStreamSynchronize(c->stream);
+      cudaFree(c->extra);
+      c->extra = nullptr;
+      c->extra_cap = 0;
+    }
+    if (cudaMalloc(&c->extra, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      c->extra = nullptr;
+      return;
+    }
+    c->extra_cap = bytes;
+  }
+  ws = Arena{c->extra, c->extra_cap, 0};
+}
+
 // Store sqrt(evals[0:cnt]) of step k for the stats (device-side copy; read back at the end).
 __global__ void k_store_sigma(const double* evals, int cnt, double* dst) {
   const int i = threadIdx.x;
@@ -777,6 +804,7 @@ int run_chain(tt_ctx* c, const float* x_in, Plan P, const tt_opts& o, float* con
       TT_TRY(make_plan(P.d, nn.data(), P.r.data(), P.ring, oplan, P2));
       for (size_t j = (size_t)k + 1; j < P.steps.size(); ++j) P.steps[j] = P2.steps[j];
       P.last_rows = P2.last_rows;
+      grow_scratch(c, P2.max_ws, ws);
       return TT_OK;
     };
     const int pr1 = st.perm231 ? st.r1_out : 1;     // TR bond r1 carried after step 1

@@ -220,6 +220,20 @@ void sketch_split_plan(long long m, long long n, int N, long long* jchunk, int* 
   *nsplit = (int)ceil_div_ll(n, jc);
 }
 
+// Lowers the split count until the partial sums fit `cap` doubles.
+int sketch_split_fit(long long m, long long n, int N, size_t cap, long long* jchunk, int* nsplit) {
+  const long long max_ns = (long long)(cap / ((size_t)N * (size_t)m));
+  if (max_ns < 1) {
+    set_error(TT_ERR_NOMEM, "sketch workspace");
+    return TT_ERR_NOMEM;
+  }
+  if (*nsplit > max_ns) {
+    *jchunk = (ceil_div_ll(n, max_ns) + 31) / 32 * 32;
+    *nsplit = (int)ceil_div_ll(n, *jchunk);
+  }
+  return TT_OK;
+}
+
 template <int RC>
 int run_sketch32(const float* a, long long m, long long n, const float* w, int N, long long wj, long long wc,
                  long long jchunk, int nsplit, int cb, double* part, cudaStream_t s) {
@@ -618,6 +632,8 @@ int launch_sketch(const float* a, long long m, long long n, const float* w, int 
   int nsplit;
   sketch_split_plan(m, n, N, &jchunk, &nsplit);
   const size_t mk = ws.mark();
+  const size_t left = (ws.cap - std::min(ws.cap, (mk + 255) & ~size_t(255))) & ~size_t(255);
+  TT_TRY(sketch_split_fit(m, n, N, left / sizeof(double), &jchunk, &nsplit));
   double* part = ws.take<double>((size_t)nsplit * N * m);
   if (!part) {
     set_error(TT_ERR_NOMEM, "sketch workspace");
@@ -638,16 +654,10 @@ int launch_sketch_simt_static(const float* a, long long m, long long n, const fl
   long long jchunk;
   int nsplit;
   sketch_split_plan(m, n, N, &jchunk, &nsplit);
-  const long long max_ns = (long long)(part_cap / ((size_t)N * (size_t)m));
-  if (max_ns < 1) {
+  if (sketch_split_fit(m, n, N, part_cap, &jchunk, &nsplit) != TT_OK) {
     set_error(TT_ERR_SHAPE, "sketch partials of %lld x %d doubles exceed the scratch of %zu doubles", m, N,
               part_cap);
     return TT_ERR_SHAPE;
-  }
-  if (nsplit > max_ns) {
-    jchunk = (n + max_ns - 1) / max_ns;
-    jchunk = (jchunk + 31) / 32 * 32;
-    nsplit = (int)((n + jchunk - 1) / jchunk);
   }
   TT_TRY(sketch32(a, m, n, w, N, wj, wc, jchunk, nsplit, part, s));
   return launch_reduce_splits(part, (long long)N * m, nsplit, y, s);

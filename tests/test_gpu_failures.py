@@ -71,3 +71,49 @@ def test_wait_limit_runs_out_and_context_survives(gpu):
     res = ttr.tt_svd(xd, [1, 4, 4, 4, 1])
     g = [c.double().cpu().numpy() for c in res.cores]
     assert oracle.rel_error(x, oracle.tt_full(g)) < 1e-3
+
+
+@pytest.mark.parametrize("shape,rank,bounds,gemm", [
+    ((17, 8, 75776), 16, (17, 24), "fp32"),   # 128 rows instead of 136: more splits of the sketch
+    ((33, 32, 20000), 32, (33, 24), "tc"),    # 1024 rows instead of 1056, the same on the tensor cores
+    ((17, 8, 200), 12, (17, 40), "fp32"),     # 96 rows instead of 136: an exact step and its eigen-solve
+])
+def test_tolerance_run_whose_ranks_shrink(gpu, monkeypatch, shape, rank, bounds, gemm):
+    """The first rank comes out below its bound, and the step after it needs more scratch than it was planned with: a
+    fresh context has it."""
+    import torch
+    ttr = _ttr()
+    monkeypatch.setattr(ttr, "_CTX", {})
+    g = torch.Generator(device=gpu).manual_seed(sum(shape))
+    a = torch.randn(shape[0], rank, generator=g, device=gpu)
+    b = torch.randn(rank * shape[1], 12, generator=g, device=gpu)
+    c = torch.randn(12, shape[2], generator=g, device=gpu)
+    x = torch.einsum("ir,rjs,sk->ijk", a, b.view(rank, shape[1], 12), c)
+    res = ttr.tt_svd(x, [1, *bounds, 1], eps=1e-3, gemm=gemm)
+    assert res.ranks == [1, rank, 12, 1]
+    assert ttr.rel_error(x, res.cores) < 1e-3
+
+
+def test_tolerance_run_at_its_allocation_limit(gpu, monkeypatch):
+    """The same where nothing may be allocated beyond what the plan takes: the sketch makes do with fewer splits."""
+    import torch
+    ttr = _ttr()
+    g = torch.Generator(device=gpu).manual_seed(4)
+    a = torch.randn(17, 16, generator=g, device=gpu)
+    b = torch.randn(16 * 8, 12, generator=g, device=gpu)
+    c = torch.randn(12, 75776, generator=g, device=gpu)
+    x = torch.einsum("ir,rjs,sk->ijk", a, b.view(16, 8, 12), c)
+    low, high = 1 << 20, 1 << 30
+    while high - low > 1 << 20:  # the least limit, to 1 MiB, that a run which keeps its ranks needs
+        mid = (low + high) // 2
+        monkeypatch.setattr(ttr, "_CTX", {})
+        assert ttr.lib().tt_ctx_set_alloc_limit(ttr._ctx_for(0), mid) == 0
+        try:
+            ttr.tt_svd(x, [1, 17, 24, 1], eps=1e-9)
+            high = mid
+        except ttr._lib.TTError:
+            low = mid
+    monkeypatch.setattr(ttr, "_CTX", {})
+    assert ttr.lib().tt_ctx_set_alloc_limit(ttr._ctx_for(0), high) == 0
+    res = ttr.tt_svd(x, [1, 17, 24, 1], eps=1e-3, gemm="fp32")
+    assert res.ranks == [1, 16, 12, 1]
