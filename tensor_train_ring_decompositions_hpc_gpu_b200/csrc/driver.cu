@@ -1436,11 +1436,14 @@ extern "C" int tt_rel_error(tt_ctx* c, const float* x, int d, const int* n, cons
                         rbuf[k & 1], s));
     rf = rbuf[k & 1];
   }
-  TT_CUDA(cudaMemsetAsync(acc, 0, 2 * sizeof(double), s));
-  TT_TRY(launch_recon_err(x, P[(size_t)cut], right_of(cut), lf, cut > 1, rf, cut < d - 1, (int)rr0, r[cut], acc, s));
   double h[2] = {0, 0};
-  TT_CUDA(cudaMemcpyAsync(h, acc, sizeof(h), cudaMemcpyDeviceToHost, s));
-  TT_CUDA(cudaStreamSynchronize(s));
+  for (int ends = 0; ends == 0 || (ends == 1 && h[0] != h[0]); ++ends) {  // NaN: see k_recon_err
+    TT_CUDA(cudaMemsetAsync(acc, 0, 2 * sizeof(double), s));
+    TT_TRY(launch_recon_err(x, P[(size_t)cut], right_of(cut), lf, cut > 1, rf, cut < d - 1, (int)rr0, r[cut], ends == 1,
+                            acc, s));
+    TT_CUDA(cudaMemcpyAsync(h, acc, sizeof(h), cudaMemcpyDeviceToHost, s));
+    TT_CUDA(cudaStreamSynchronize(s));
+  }
   *rel_err = h[1] > 0 ? sqrt(h[0] / h[1]) : 0.0;
   return TT_OK;
 }

@@ -126,10 +126,11 @@ int launch_merge(const void* a, bool a64, long long M, int K, const void* b, boo
 
 // Fused reconstruction check of a ring/train: acc += ||X - X^||^2 and ||X||^2, X (P x N) and
 // X^[i, J] = sum_{a,b} L[a, i, b] R[b, J, a] with the merged left cores L (r0, P, rk) and the merged
-// right cores R (rk, N, r0), each FP64 (merged) or FP32 (a core as it is); recon_tiles: its tile count.
+// right cores R (rk, N, r0), each FP64 (merged) or FP32 (a core as it is); recon_tiles: its tile count.  ends: also
+// right where a core is infinite (without it the sum may be NaN then), and a little slower.
 long long recon_tiles(long long P, long long N);
 int launch_recon_err(const float* x, long long P, long long N, const void* lf, bool l64, const void* rf, bool r64,
-                     int r0, int rk, double* acc, cudaStream_t s);
+                     int r0, int rk, bool ends, double* acc, cudaStream_t s);
 
 // Learned predictor (mlp.cu).  Features from the descending probe eigenvalues mu
 // (TT_PROBE_COLS of them); network inference; training (mode 0: Adam steps on Philox-drawn

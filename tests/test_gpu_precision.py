@@ -112,3 +112,17 @@ def test_sketch_fp32_chain_length(gpu, m, n, N):
     w = torch.full((N, n), 1.0 + 2.0 ** -14, device=gpu).t()
     y = _ttr().sketch(a, w, "fp32")
     assert torch.all(y.double() == n * (1.0 + 2.0 ** -14))
+
+
+@pytest.mark.parametrize("ring,n", [(False, (5, 3)), (False, (130, 70)), (False, (128, 64)), (False, (9, 15, 33, 7)),
+                                    (True, (130, 3, 131)), (True, (16, 9, 17))])
+def test_rel_error_of_an_infinite_core(gpu, ring, n):
+    """Positive cores of rank 1 of which one entry is infinite: the reconstruction is infinite there and nowhere NaN,
+    and so is the error, whatever the sizes leave of the last tiles."""
+    rng = np.random.default_rng(sum(n))
+    cores = [rng.uniform(0.5, 1.0, (1, k, 1)).astype(np.float32) for k in n]
+    x = (oracle.tr_full if ring else oracle.tt_full)([c.astype(np.float64) for c in cores]).astype(np.float32)
+    for k in (0, len(n) - 1):
+        bad = [c.copy() for c in cores]
+        bad[k][0, 1, 0] = np.inf
+        assert _ttr().rel_error(_dev(x, gpu), [_dev(c, gpu) for c in bad], ring=ring) == np.inf
