@@ -1377,7 +1377,8 @@ extern "C" int tt_rel_error(tt_ctx* c, const float* x, int d, const int* n, cons
   // Left part of a split after core k (k cores): (r0, P_k, r_k); right part: (r_k, N_k, r_d).  Any
   // split gives the same product; its cost is the final contraction (r0 r_k FMAs per element, in whole
   // tiles) plus the merges of both sides, least where both sides are small.  Scratch (FP64): the
-  // last two merges of a side, within the largest merge of everything right of core 1 wherever a cut allows.
+  // last two merges of a side, within the largest merge of everything right of core 1 (`most`); where no cut
+  // allows that, core 1 against the rest, the last mode a part at a time.
   std::vector<long long> P((size_t)d + 1, 1);
   for (int k = 0; k < d; ++k) P[(size_t)k + 1] = P[(size_t)k] * n[k];
   auto right_of = [&](int k) { return P[(size_t)d] / P[(size_t)k]; };  // n_k ... n_{d-1}
@@ -1398,6 +1399,7 @@ extern "C" int tt_rel_error(tt_ctx* c, const float* x, int d, const int* n, cons
     return q;
   };
   const Bufs2 all = right_bufs(1);
+  const size_t most = std::max({all.b[0], all.b[1], right_elems(d - 1)});
   int cut = 1;
   double best = -1.0;
   for (int k = 1; k < d; ++k) {
@@ -1411,7 +1413,14 @@ extern "C" int tt_rel_error(tt_ctx* c, const float* x, int d, const int* n, cons
       cut = k;
     }
   }
-  const Bufs2 lb = left_bufs(cut), rb = right_bufs(cut);
+  const Bufs2 lb = left_bufs(cut);
+  Bufs2 rb = right_bufs(cut);
+  const long long nl = n[d - 1];  // the last mode, `part` of it at a time
+  long long part = nl;
+  if (best < 0.0 && rb.b[0] + rb.b[1] > most) {
+    part = std::max<long long>(1, (long long)((double)nl * (double)most / (double)(rb.b[0] + rb.b[1])));
+    for (size_t& b : rb.b) b = b / (size_t)nl * (size_t)part;
+  }
   TT_TRY(tt_ctx_reserve(c, sizeof(double) * (lb.b[0] + lb.b[1] + rb.b[0] + rb.b[1]) + 4096 + (1 << 20)));
   Arena a{c->arena, c->cap, 0};
   double* lbuf[2] = {a.take<double>(lb.b[0]), a.take<double>(lb.b[1])};
@@ -1425,22 +1434,28 @@ extern "C" int tt_rel_error(tt_ctx* c, const float* x, int d, const int* n, cons
   const void* lf = cores[0];
   for (int k = 2; k <= cut; ++k) {
     // (r0, P_k, r_k) = (r0 P_{k-1} x r_{k-1}) * (r_{k-1} x n_{k-1} r_k)
-    TT_TRY(launch_merge(lf, k > 2, rr0 * P[(size_t)k - 1], r[k - 1], cores[k - 1], false, (long long)n[k - 1] * r[k],
-                        lbuf[k & 1], s));
+    const long long cols = (long long)n[k - 1] * r[k];
+    TT_TRY(launch_merge(lf, k > 2, rr0 * P[(size_t)k - 1], r[k - 1], cores[k - 1], false, cols, cols, 0, lbuf[k & 1],
+                        s));
     lf = lbuf[k & 1];
-  }
-  const void* rf = cores[d - 1];
-  for (int k = d - 2; k >= cut; --k) {
-    // (r_k, N_k, r_d) = (r_k n_k x r_{k+1}) * (r_{k+1} x N_{k+1} r_d)
-    TT_TRY(launch_merge(cores[k], false, (long long)r[k] * n[k], r[k + 1], rf, k < d - 2, right_of(k + 1) * r[d],
-                        rbuf[k & 1], s));
-    rf = rbuf[k & 1];
   }
   double h[2] = {0, 0};
   for (int ends = 0; ends == 0 || (ends == 1 && h[0] != h[0]); ++ends) {  // NaN: see k_recon_err
     TT_CUDA(cudaMemsetAsync(acc, 0, 2 * sizeof(double), s));
-    TT_TRY(launch_recon_err(x, P[(size_t)cut], right_of(cut), lf, cut > 1, rf, cut < d - 1, (int)rr0, r[cut], ends == 1,
-                            acc, s));
+    for (long long i0 = 0; i0 < nl; i0 += part) {
+      const long long np = std::min(part, nl - i0);
+      const void* rf = cores[d - 1] + r[d - 1] * i0;
+      for (int k = d - 2; k >= cut; --k) {
+        // (r_k, N_k, r_d) = (r_k n_k x r_{k+1}) * (r_{k+1} x N_{k+1} r_d)
+        const bool last = k == d - 2;
+        const long long cols = right_of(k + 1) / nl * np * r[d];
+        TT_TRY(launch_merge(cores[k], false, (long long)r[k] * n[k], r[k + 1], rf, !last, cols, last ? np : cols,
+                            last ? nl - np : 0, rbuf[k & 1], s));
+        rf = rbuf[k & 1];
+      }
+      TT_TRY(launch_recon_err(x + P[(size_t)d - 1] * i0, P[(size_t)cut], right_of(cut) / nl * np, lf, cut > 1, rf,
+                              cut < d - 1, (int)rr0, r[cut], ends == 1, acc, s));
+    }
     TT_CUDA(cudaMemcpyAsync(h, acc, sizeof(h), cudaMemcpyDeviceToHost, s));
     TT_CUDA(cudaStreamSynchronize(s));
   }

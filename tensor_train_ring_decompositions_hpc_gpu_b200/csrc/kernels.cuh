@@ -120,9 +120,10 @@ int launch_check_finite(const float* x, long long count, int* flag, cudaStream_t
 // Sum of squares (FP64) of (x - y) and of x, accumulated into acc[0], acc[1].
 int launch_diff_norm(const float* x, const float* y, long long count, double* acc, cudaStream_t s);
 
-// C (M x N, FP64) = A (M x K) * B (K x N), column-major, each FP32 or FP64 (a64, b64): core merging.
-int launch_merge(const void* a, bool a64, long long M, int K, const void* b, bool b64, long long N, double* c,
-                 cudaStream_t s);
+// C (M x N, FP64) = A (M x K) * B (K x N), column-major, each FP32 or FP64 (a64, b64): core merging.  Runs of bn
+// columns of B are bgap columns apart.
+int launch_merge(const void* a, bool a64, long long M, int K, const void* b, bool b64, long long N, long long bn,
+                 long long bgap, double* c, cudaStream_t s);
 
 // Fused reconstruction check of a ring/train: acc += ||X - X^||^2 and ||X||^2, X (P x N) and
 // X^[i, J] = sum_{a,b} L[a, i, b] R[b, J, a] with the merged left cores L (r0, P, rk) and the merged

@@ -185,10 +185,12 @@ __global__ void __launch_bounds__(256, 2) k_recon_err(const float* __restrict__ 
   }
 }
 
-// C (M x N, FP64) = A (M x K) * B (K x N), column-major, K small: the merge of two cores.
+// C (M x N, FP64) = A (M x K) * B (K x N), column-major, K small: the merge of two cores.  Column n of B lies at
+// b + K (n + n / bn * bgap): a part of the last mode of a ring's core.
 template <typename TA, typename TB>
 __global__ void __launch_bounds__(128) k_merge(const TA* __restrict__ a, long long M, int K, const TB* __restrict__ b,
-                                               long long N, double* __restrict__ c) {
+                                               long long N, long long bn, long long bgap,
+                                               double* __restrict__ c) {
   constexpr int NC = 8;
   __shared__ double bs[64][NC];
   const long long nblk = (M + 127) / 128, tiles = nblk * ((N + NC - 1) / NC);
@@ -201,7 +203,8 @@ __global__ void __launch_bounds__(128) k_merge(const TA* __restrict__ a, long lo
       __syncthreads();
       for (int f = threadIdx.x; f < 64 * NC; f += 128) {
         const int kk = f & 63, u = f >> 6;
-        bs[kk][u] = (n0 + u < N && k0 + kk < K) ? (double)b[(k0 + kk) + (long long)K * (n0 + u)] : 0.0;
+        const long long n = n0 + u;
+        bs[kk][u] = (n < N && k0 + kk < K) ? (double)b[(k0 + kk) + (long long)K * (n + (bgap ? n / bn * bgap : 0))] : 0.0;
       }
       __syncthreads();
       if (i < M) {
@@ -255,18 +258,18 @@ int launch_recon_err(const float* x, long long P, long long N, const void* lf, b
              : run_recon<float, float>(x, P, N, lf, rf, r0, rk, ends, acc, s);
 }
 
-int launch_merge(const void* a, bool a64, long long M, int K, const void* b, bool b64, long long N, double* c,
-                 cudaStream_t s) {
+int launch_merge(const void* a, bool a64, long long M, int K, const void* b, bool b64, long long N, long long bn,
+                 long long bgap, double* c, cudaStream_t s) {
   if (M <= 0 || N <= 0) return TT_OK;
   const int grid = (int)std::min<long long>(ceil_div_ll(M, 128) * ceil_div_ll(N, 8), 64LL * dev_sms());
   const double* a8 = static_cast<const double*>(a);
   const float* a4 = static_cast<const float*>(a);
   const double* b8 = static_cast<const double*>(b);
   const float* b4 = static_cast<const float*>(b);
-  if (a64 && b64) k_merge<<<grid, 128, 0, s>>>(a8, M, K, b8, N, c);
-  else if (a64) k_merge<<<grid, 128, 0, s>>>(a8, M, K, b4, N, c);
-  else if (b64) k_merge<<<grid, 128, 0, s>>>(a4, M, K, b8, N, c);
-  else k_merge<<<grid, 128, 0, s>>>(a4, M, K, b4, N, c);
+  if (a64 && b64) k_merge<<<grid, 128, 0, s>>>(a8, M, K, b8, N, bn, bgap, c);
+  else if (a64) k_merge<<<grid, 128, 0, s>>>(a8, M, K, b4, N, bn, bgap, c);
+  else if (b64) k_merge<<<grid, 128, 0, s>>>(a4, M, K, b8, N, bn, bgap, c);
+  else k_merge<<<grid, 128, 0, s>>>(a4, M, K, b4, N, bn, bgap, c);
   count_launch();
   TT_LAUNCH_CHECK();
   return TT_OK;

@@ -126,3 +126,26 @@ def test_rel_error_of_an_infinite_core(gpu, ring, n):
         bad = [c.copy() for c in cores]
         bad[k][0, 1, 0] = np.inf
         assert _ttr().rel_error(_dev(x, gpu), [_dev(c, gpu) for c in bad], ring=ring) == np.inf
+
+
+@pytest.mark.parametrize("ring,n,ranks", [
+    (False, (2000, 10, 12, 14), (1, 5, 7, 4, 1)),
+    (True, (700, 20, 30, 13), (3, 5, 7, 4, 3)),
+    (True, (900, 10, 60, 2), (2, 5, 7, 4, 2)),
+    (False, (1500, 12, 10, 8, 9), (1, 4, 8, 30, 9, 1)),
+])
+def test_rel_error_within_its_scratch(gpu, monkeypatch, ring, n, ranks):
+    """A long first mode, so that every cut but the first would merge a larger left side than the cores right of it.
+    The check takes two FP32 buffers of the largest of those, 1 MiB and 4 KiB of alignment, as its context allows here."""
+    ttr = _ttr()
+    rng = np.random.default_rng(sum(n))
+    d = len(n)
+    cores = [rng.standard_normal((ranks[k], n[k], ranks[k + 1])).astype(np.float32) for k in range(d)]
+    full = (oracle.tr_full if ring else oracle.tt_full)([c.astype(np.float64) for c in cores])
+    x = (full + 1e-2 * np.linalg.norm(full) / np.sqrt(full.size) * rng.standard_normal(n)).astype(np.float32)
+    most = max(ranks[k] * int(np.prod(n[k:])) * ranks[d] for k in range(1, d))
+    xd, cd = _dev(x, gpu), [_dev(c, gpu) for c in cores]
+    want = oracle.rel_error(x, full)
+    monkeypatch.setattr(ttr, "_CTX", {})
+    assert ttr.lib().tt_ctx_set_alloc_limit(ttr._ctx_for(0), 8 * most + 4096 + (1 << 20)) == 0
+    assert abs(ttr.rel_error(xd, cd, ring=ring) - want) <= 1e-9 * want
