@@ -149,3 +149,23 @@ def test_rel_error_within_its_scratch(gpu, monkeypatch, ring, n, ranks):
     monkeypatch.setattr(ttr, "_CTX", {})
     assert ttr.lib().tt_ctx_set_alloc_limit(ttr._ctx_for(0), 8 * most + 4096 + (1 << 20)) == 0
     assert abs(ttr.rel_error(xd, cd, ring=ring) - want) <= 1e-9 * want
+
+
+@pytest.mark.parametrize("ring,n,ranks,noise", [
+    (False, (5, 3), (1, 3, 1), 1e-4),
+    (False, (12, 12, 12, 12, 12), (1, 7, 40, 65, 9, 1), 1e-4),
+    (False, (37, 29, 41, 23), (1, 19, 45, 13, 1), 1e-3),
+    (True, (16, 9, 17, 8), (4, 3, 11, 2, 4), 1e-4),
+    (True, (130, 3, 131), (2, 5, 6, 2), 1e-2),
+])
+def test_rel_error_is_fp64(gpu, ring, n, ranks, noise):
+    """FP64 from the FP32 cores and X to the sums: at an error of `noise` the difference X - X^ holds 2^-53 x the sum of
+    magnitudes / noise, 1e-9 of the result with room to spare; an FP32 X^ would move it by u / noise and more."""
+    rng = np.random.default_rng(sum(n))
+    d = len(n)
+    cores = [rng.standard_normal((ranks[k], n[k], ranks[k + 1])).astype(np.float32) for k in range(d)]
+    full = (oracle.tr_full if ring else oracle.tt_full)([c.astype(np.float64) for c in cores])
+    x = (full + noise * np.linalg.norm(full) / np.sqrt(full.size) * rng.standard_normal(n)).astype(np.float32)
+    want = oracle.rel_error(x, full)
+    got = _ttr().rel_error(_dev(x, gpu), [_dev(c, gpu) for c in cores], ring=ring)
+    assert abs(got - want) <= 1e-9 * want
