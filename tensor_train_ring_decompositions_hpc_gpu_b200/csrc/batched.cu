@@ -912,10 +912,10 @@ int launch_batched(int bch, int grid, cudaStream_t s, const BatchArgs& a) {
 }
 
 // CTAs of a batch, `per_sm` (1 or 2) to an SM.  Up to kOneWave tensors per SM one is better: the batch is then
-// about as long as its slowest tensors, and those run faster alone.  Order 4, 8-32 per mode: 310 tensors 1443 us
-// against 2325 with two, 580 2081 against 2728, 800 the same; of nearly equal sizes (12-20) 580 take 1223 against
-// 1065.
-constexpr int kOneWave = 4;
+// about as long as its slowest tensors, and those run faster alone.  One against two, us: order 4 of 8-32 per mode,
+// 310 tensors 1168 / 1708, 440 1542 / 1740, 580 1933 / 1848; of 12-20, 200 tensors 566 / 645, 310 821 / 775, 440 994 /
+// 994, 580 1284 / 1119; order 3 of 20-28, 440 728 / 702, 580 925 / 773.
+constexpr int kOneWave = 3;
 int best_per_sm(int count) { return count <= kOneWave * dev_sms() ? 1 : 2; }
 int persistent_grid(int count, int per_sm) { return std::max(1, std::min(count, per_sm * dev_sms())); }
 
