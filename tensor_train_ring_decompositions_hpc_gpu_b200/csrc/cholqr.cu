@@ -526,7 +526,7 @@ int cholqr_passes(const double* y64, float* y, long long n, int N, long long ld,
     set_error(TT_ERR_NOMEM, "cholqr2 workspace");
     return TT_ERR_NOMEM;
   }
-  // One launch whenever the rows fit the shared memory of 8 CTAs (at N = 40 that is 6,800 rows each):
+  // One launch whenever the rows fit the shared memory of 8 CTAs (at N = 40 1,130 rows each, 9,000 in all):
   // CTAs of at least 64 rows, as few as fit.
   if (n <= (1LL << 20)) {
     for (int cl = (int)std::min<long long>(8, ceil_div_ll(n, 64)); cl <= 8; ++cl) {

@@ -1370,6 +1370,8 @@ extern "C" int tt_rel_error(tt_ctx* c, const float* x, int d, const int* n, cons
   }
   TT_CUDA(cudaSetDevice(c->device));
   const long long rr0 = ring ? r[0] : 1;
+  // Nothing below needs this bound (either side streams through a fixed share of shared memory).  It is part of what
+  // the call answers: a first core above it has been TT_ERR_UNSUPPORTED in every version.
   if (((double)rr0 * n[0] * r[1] + 32.0 * rr0 * r[1]) * sizeof(float) > 200.0 * 1024) {
     set_error(TT_ERR_UNSUPPORTED, "reconstruction check: first core too large");
     return TT_ERR_UNSUPPORTED;
