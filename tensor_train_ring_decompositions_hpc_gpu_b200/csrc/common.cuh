@@ -85,6 +85,13 @@ __device__ __forceinline__ void ffma2(uint64_t& d, uint64_t a, uint64_t b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
 }
 
+// c += a (8 x 4) * b (4 x 8): lane holds a[lane / 4][lane % 4], b[lane % 4][lane / 4], c[lane / 4][2 (lane % 4) ..].
+__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
 // Launch-count accounting (kernels launched by the current library call).
 extern thread_local int g_kernel_launches;
 inline void count_launch(int n = 1) { g_kernel_launches += n; }

@@ -62,12 +62,6 @@ GramJobs gr_jobs(long long nvec, int M) {
   return J;
 }
 
-__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
-}
-
 // One warp's share of a job: NG = 1, one group against itself (upper tiles); NG = 2, two groups against
 // each other; MULTI: M has more than one group.  Ends with the block's sum of the tiles, rows of 8 GS, in
 // dst.

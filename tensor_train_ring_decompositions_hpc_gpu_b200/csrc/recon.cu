@@ -20,11 +20,6 @@ constexpr int RE_LI = RE_I + 4, RE_LJ = RE_J + 4;    // row strides: 4 k x 4 col
 constexpr int RE_LX = 32 + 8;                        // X: a warp's 32 x 32 entries, 4 rows x 4 pairs in distinct banks
 constexpr size_t RE_SMEM = (size_t)2 * RE_K * (RE_LI + RE_LJ) * sizeof(double) + 8 * 32 * RE_LX * sizeof(float);
 
-__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
-}
 __device__ __forceinline__ void cp_async8(double* dst, const double* src, bool valid) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
                "l"(src), "r"(valid ? 8 : 0)

@@ -27,13 +27,6 @@ constexpr int su_rows(int N) { return (N + 7) & ~7; }
 constexpr int su_ld(int N) { return su_rows(N) + 4; }
 constexpr int kSubPacked = kSubDim * (kSubDim + 1) / 2;
 
-// c += a (8 x 4) * b (4 x 8): lane holds a[lane / 4][lane % 4], b[lane % 4][lane / 4], c[lane / 4][2 (lane % 4) ..].
-__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
-}
-
 // Upper tile (p, q) of the kSubDim / 8 x kSubDim / 8 tiles, in rows.
 __device__ __forceinline__ void su_tile(int e, int& p, int& q) {
   constexpr int T = kSubDim / 8;
