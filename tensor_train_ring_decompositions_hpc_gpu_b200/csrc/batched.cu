@@ -325,7 +325,7 @@ __device__ int pick_rank(const double* lam, int nev, int cap, double delta2, boo
 }
 
 // The phases of a step, each a call of its own width with its own registers.  4096 tensors of order 4 (8-32 per
-// mode, 2.6 GB read, floor 0.41 ms): 18.9 ms -> 13.0.  It is bound by chains, not by memory: 39 % of the time are
+// mode, 2.6 GB read, floor 0.41 ms): 13.0 ms.  It is bound by chains, not by memory: 39 % of the time are
 // the eigen-solves (8 sweeps of one barrier per round), 15 % the Gram matrices of exact steps, 22 % the products
 // with the bases.  The order of every FP32 sum is fixed per tensor, whatever the batch and the schedule.
 
@@ -890,7 +890,7 @@ template <int BCH>
 int launch_bch(int grid, cudaStream_t s, const BatchArgs& a) {
   TT_TRY(set_smem_attr<BCH>());
   // Alone on its SM a CTA may have 168 registers a thread instead of 80: a round of the eigen-solver is shorter
-  // and the Gram matrices do not spill (69 tensors of order 3: 410 -> 326 us).
+  // and the Gram matrices do not spill (69 tensors of order 3: 326 us, 410 at 80 registers).
   auto* kernel = grid <= dev_sms() ? k_tt_batched<BCH, 1> : k_tt_batched<BCH, 2>;
   kernel<<<grid, BT, sm_total(a.mrows), s>>>(a.shp, a.order, a.count, a.x, a.cores, a.ranks, a.err, a.scratch,
                                              a.per_cta, a.half, a.eps, a.rmax, a.oversample, a.seed, 40, a.counter,

@@ -18,10 +18,9 @@
 //    once.  An FP32 reciprocal pivot makes a whole column of Q longer or shorter by up to 2^-24, which the second
 //    pass cannot mend (its factor 1 + 3e-8 rounds back), and close eigenvectors of B B^T tilt by that over their
 //    gap: interior bases of a 24^6 tensor at ranks 24 come out 3 to 5 times closer to their 64-bit values.
-//    The second pass then finds R = I to 1e-9 and has nothing to round.  256^3, ranks 16: 678 -> 680 us.
-// CholeskyQR2 of 384 x 24: 66 us before, 32 now; 1024 x 40: 79, 49; 256 x 80: 212, 132; 640 x 96 (then
-// seven launches): about 590, 187.  What is left is the chain: at 1024 x 40, per pass, 14k cycles of
-// Cholesky, 8.5k of Gram, 6k for the cluster's sum, 6k of row solves.
+//    The second pass then finds R = I to 1e-9 and has nothing to round.  256^3, ranks 16: 680 us (678 without).
+// CholeskyQR2 of 384 x 24: 32 us; 1024 x 40: 49; 256 x 80: 118; 640 x 96: 187.  What is left is the chain: at
+// 1024 x 40, per pass, 14k cycles of Cholesky, 8.5k of Gram, 6k for the cluster's sum, 6k of row solves.
 // Small matrices take one launch, a cluster of up to 8 CTAs (launch_cholqr2 below has the rule).
 #include <algorithm>
 
@@ -457,7 +456,7 @@ __global__ void __launch_bounds__(CQ_T, 1) k_chol_inv(const double* __restrict__
 // Y (n x N, column-major) <- Y T, T = R^-1.  A thread owns a row: the loads and stores of a warp are
 // runs of 32 rows of a column, the row waits in the thread's own line of shared memory (odd stride),
 // so nothing but T is shared and tiles need no barrier.  HBM / FP32 FMA bound: N (N + 1) / 2 FMAs per
-// 8 N bytes (262144 x 80: 609 us before, 128 now).  An FP64 T takes twice the shared memory, so half the rows.
+// 8 N bytes (262144 x 80: 128 us).  An FP64 T takes twice the shared memory, so half the rows.
 template <typename T>
 constexpr int cq_apply_rows() { return sizeof(T) == 8 ? CQ_T / 2 : CQ_T; }
 template <typename T>

@@ -3,11 +3,10 @@
 // Replaces the GemmEx calls of TT3O:601-708.
 //
 // Bound by the FP32 FMAs from about 24 output columns on (128 per clock and SM, issued as pairs by
-// fma.rn.f32x2), by HBM below.  What held the kernels these replace at 35-49 % of the FMA rate was the
-// tile of a thread (8 x 4 or 8 x 5: as many issue slots for loads and operand copies as for FMAs) and row
-// tiles of 256 or 512 that hung over the end of the unfolding.  576 x 331776 at 32 columns (floor 164 us
-// of FMAs): sketch 467 -> 328 us, projection 415 -> 330; 600 x 950k: 16 columns 1125 -> 409, 96 columns
-// 3732 -> 1743; 384 x 320: 39 -> 7 and 16 -> 7.
+// fma.rn.f32x2), by HBM below.  Hence wide tiles per thread (at 8 x 4 or 8 x 5, loads and operand copies take as
+// many issue slots as the FMAs: 35-49 % of their rate) and row tiles of 64, which hang little over the end of an
+// unfolding.  576 x 331776 at 32 columns (floor 164 us of FMAs): sketch 328 us, projection 330.  Sketches of
+// 600 x 950k: 565 us at 16 columns, 2480 at 96 (59 % of the FMA rate).  384 x 320: 6 us each.
 #include <algorithm>
 
 #include "kernels.cuh"
@@ -410,7 +409,7 @@ __global__ void k_project_reduce(const float* __restrict__ part, long long n, in
 // computes NPT outputs of CT columns, so a row of Q is loaded once for CT columns; G groups of threads
 // share a column.  Products in one chain over k per output.  Row-major outputs and the TR bond permute
 // leave through shared memory as contiguous runs.  HBM / FP32 FMA bound: 30 -> 20 rows of 19M columns
-// 1885 us with one column per thread, 960 now.
+// 960 us (1885 with one column per thread).
 template <int NP, int G, int CT>
 __global__ void __launch_bounds__(256) k_proj_smallk(const float* __restrict__ a, int m, long long n,
                                                      const float* __restrict__ q, int N, long long ldq,

@@ -9,8 +9,7 @@
 // own vectors through its own cp.async ring (no block barrier until the end) and keeps all 8 x 8 tiles of
 // its part of W's upper triangle in registers: blocks of up to 6 x 6 tiles, larger M being split into
 // jobs (pairs of component groups) with blocks in proportion to their tiles.  One kernel for either layout,
-// any M and any alignment; it took the place of five.  Before -> now, us: 24 x 8.4M 656 -> 246,
-// 85 x 950k 1614 -> 372, 45 x 850k 403 -> 60, 80 x 262k (column-major, FP32 products before) 353 -> 76.
+// any M and any alignment.  24 x 8.4M: 249 us; 85 x 950k: 329; 45 x 850k: 77; 80 x 262k (column-major): 75.
 #include <algorithm>
 
 #include "kernels.cuh"
@@ -243,7 +242,7 @@ int run_gram64(const float* x, long long nvec, int M, long long vs, long long es
 // t takes 8 x 8 tile t of vector 3 it + u) for vectors whose length is not a multiple of 4, which the
 // TMA cannot address as rows: a box of 48 vectors is one contiguous run, copied as it lies by 16-byte
 // cp.async (48 M floats are always a multiple of 16 bytes), and read by 8-byte (EVEN: M even) or 4-byte
-// loads.  FP32 FMA and shared-memory issue bound; 30 x 19M: 4834 us before, 667 now.
+// loads.  FP32 FMA and shared-memory issue bound; 30 x 19M: 667 us.
 constexpr int G32U_VPS = 48, G32U_ST = 4, G32U_WARPS = 8;
 constexpr int g32u_stage(int M) { return G32U_VPS * M + 32; }  // floats; the last vector is read 32 wide
 constexpr size_t g32u_smem(int M) {

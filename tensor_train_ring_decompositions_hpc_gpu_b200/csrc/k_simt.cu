@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(1024) k_syev_blw(const double* __restrict__ w_
   constexpr int MAXIT = (64 * 65 / 2 + NE - 1) / NE;
   // With at most a block per thread (N <= 86) the rotation warps are the longer part, and their 12 loads
   // would queue behind the other warps' for a third of the round: those wait until they are issued (a
-  // round at N = 72: 0.94 -> 0.77 us; at N = 128 the blocks are the longer part, and waiting costs 8 %).
+  // round at N = 72: 0.77 us, 0.94 without; at N = 128 the blocks are the longer part, and waiting costs 8 %).
   const bool first = NWB <= NE;
   // per block of this thread: the pair indices (a | b << 8, -1 for none), the offsets of its two
   // rows in W and of its four entries' next-round upper positions (fixed over the rounds)

@@ -2,12 +2,10 @@
 //
 // X^[i, J] = sum_{a,b} L[a, i, b] R[b, J, a] over q = r0 rk products, L (r0, P, rk) the merged left cores and
 // R (rk, N, r0) the merged right ones.  Everything between the FP32 cores and the two sums is FP64: at a
-// relative error of 1e-4 an FP32 X^ moves the result by 3e-6 (an FP32 tile loop took 2.4 ms for a 32^6 tensor
-// at ranks 32, but was less exact than the kernel before it on small tensors).  Bound by the FP64 matrix
-// instructions (mma.m8n8k4.f64, 64 FMAs per clock and SM without a register-tiled loop's loads): q FMAs per
-// element of X, 1.85 ms at q = 32, next to one read of X (0.66 ms).  18.0 ms before (two shared-memory loads
-// per FMA, and a merged factor as large as X written and read), 3.5 ms now (3.7 with X read by the lanes
-// that need it instead of copied behind the products), and exact where the old one was 2.6e-6 off.
+// relative error of 1e-4 an FP32 X^ moves the result by 3e-6 (its tile loop takes 2.4 ms for a 32^6 tensor at
+// ranks 32, this one 3.5).  Bound by the FP64 matrix instructions (mma.m8n8k4.f64, 64 FMAs per clock and SM
+// without a register-tiled loop's loads): q FMAs per element of X, 1.85 ms at q = 32, next to one read of X
+// (0.66 ms).  X is copied behind the products; read by the lanes that need it the check takes 3.7 ms.
 #include <algorithm>
 
 #include "kernels.cuh"

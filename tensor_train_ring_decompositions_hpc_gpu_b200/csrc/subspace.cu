@@ -10,8 +10,7 @@
 // Bound by latency and the FP64 rate of one SM: 17 products W Y (N^2 x 32 FMAs, 1.7 us each at N = 80), 10 Gram
 // matrices, Cholesky factors and row solves.  All products are on the FP64 matrix instructions, fragments straight
 // from shared memory: a leading dimension of 4 or 12 modulo 16 puts the 4 x 4 values of a half warp in distinct
-// banks.  N = 80: 461 us with a warp per Gram entry, a barrier and a division per pivot and a fifth of the threads
-// in the products; 165 us now.
+// banks.  N = 80: 165 us.
 #include "chol.cuh"
 #include "kernels.cuh"
 #include "philox.cuh"
