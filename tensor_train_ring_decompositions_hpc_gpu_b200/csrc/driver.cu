@@ -730,16 +730,17 @@ int run_chain(tt_ctx* c, const float* x_in, Plan P, const tt_opts& o, float* con
     return TT_OK;
   };
   // Gram of the rows of an unfolding with m <= 128 rows (the exact step).  Up to 32 rows: the exact
-  // CUDA-core kernels in every form (FP32 products, FP64 sums), whose result
-  // resolves eigenvalues down to ~1e-9 of the largest; the tensor cores' truncating FP32 accumulation
-  // would bias the small ones.  `precise` (adaptive ranks: energies to ~1e-8 relative) keeps short
-  // unfoldings, whose few partial sums do not average the FP32 rounding out, on FP64 products: below 2^16
-  // columns where the TMA can address the rows (m a multiple of 4), below 2^22 where it cannot.  Wider:
-  // tensor cores when allowed, else FP64 products.
+  // CUDA-core kernels in every form, whose result resolves eigenvalues down to ~1e-9 of the largest; the
+  // tensor cores' truncating FP32 accumulation would bias the small ones.  Where the TMA can address the rows
+  // (m a multiple of 4): FP32 products summed in FP64, but FP64 products for `precise` (adaptive ranks:
+  // energies to ~1e-8 relative) below 2^16 columns, whose few partial sums do not average the FP32 rounding
+  // out.  Elsewhere FP64 products, which are also faster there (15 x 8.4M: 124 us against 354; 23 x 8.4M: 214,
+  // 358; 30 x 90,000: 8.5, 9.4), except for 25 to 31 rows of 2^22 columns or more (30 x 8.4M: 375, 309).
+  // Wider: tensor cores when allowed, else FP64 products.
   auto gram_rows = [&](const float* a, long long mm, long long nc, double* w, int eng, bool precise) -> int {
     if (mm <= 32 && (!precise || nc >= (1LL << 16))) {
       int rc = launch_gram32x(a, nc, (int)mm, w, ws, c->dstat, s);
-      if (rc == TT_ERR_UNSUPPORTED && (!precise || nc >= (1LL << 22)))
+      if (rc == TT_ERR_UNSUPPORTED && mm > 24 && nc >= (1LL << 22))
         rc = launch_gram32u(a, nc, (int)mm, w, ws, s);
       if (rc != TT_ERR_UNSUPPORTED) return rc;
     }

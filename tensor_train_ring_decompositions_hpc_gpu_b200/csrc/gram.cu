@@ -242,7 +242,8 @@ int run_gram64(const float* x, long long nvec, int M, long long vs, long long es
 // t takes 8 x 8 tile t of vector 3 it + u) for vectors whose length is not a multiple of 4, which the
 // TMA cannot address as rows: a box of 48 vectors is one contiguous run, copied as it lies by 16-byte
 // cp.async (48 M floats are always a multiple of 16 bytes), and read by 8-byte (EVEN: M even) or 4-byte
-// loads.  FP32 FMA and shared-memory issue bound; 30 x 19M: 667 us.
+// loads.  FP32 FMA and shared-memory issue bound; 30 x 19M: 667 us.  Used where the FP64 form has 4 x 4 blocks and
+// many vectors (25 to 31 components; the rule and both times are at gram_rows in driver.cu).
 constexpr int G32U_VPS = 48, G32U_ST = 4, G32U_WARPS = 8;
 constexpr int g32u_stage(int M) { return G32U_VPS * M + 32; }  // floats; the last vector is read 32 wide
 constexpr size_t g32u_smem(int M) {

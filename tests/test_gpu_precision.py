@@ -102,6 +102,36 @@ def test_adaptive_gram_of_unaligned_rows(gpu, m):
     assert abs(res.est_rel_err - want) <= 1e-4 * want
 
 
+@pytest.mark.parametrize("shape,rank", [((9, 5, 9, 4), 2), ((7, 11, 5), 3), ((18, 10, 23, 6), 5), ((30, 7, 31), 6)])
+def test_grams_of_odd_rows_do_not_overflow(gpu, shape, rank):
+    """Rows that are no multiple of 4: values of about 2^62, sixteen of whose squares add up beyond FP32.  Scaling by a
+    power of two changes no rounding, so the singular values are those of the tensor as it is, times that."""
+    import torch
+    ranks = [1] + [rank] * (len(shape) - 1) + [1]
+    x = _dev(oracle.make_tt_tensor(list(shape), ranks, 1e-2, seed=sum(shape)), gpu)
+    x = 1.0 + 0.25 * x / x.abs().max()
+    one = _ttr().tt_svd(x, ranks, gemm="fp32")
+    big = _ttr().tt_svd(x * 2.0 ** 62, ranks, gemm="fp32")
+    for k, (a, b) in enumerate(zip(one.sigmas, big.sigmas)):
+        a, b = np.asarray(a)[:ranks[k + 1]], np.asarray(b)[:ranks[k + 1]] / 2.0 ** 62
+        assert np.abs(a - b).max() <= 1e-6 * a.max(), (k, a, b)
+    assert all(torch.isfinite(c).all() for c in big.cores)
+
+
+@pytest.mark.parametrize("m,n2,n3", [(25, 2048, 2048), (26, 2048, 2049), (30, 2049, 2048), (31, 2047, 2050)])
+def test_gram_of_long_odd_rows(gpu, m, n2, n3):
+    """25 to 31 rows on both sides of 2^22 columns.  FP32 products in chains of 64 are off by 65 u of the sum of their
+    magnitudes at most, FP64 ones by nothing that shows: eigenvalues to 65 u of the trace."""
+    import torch
+    g = torch.Generator(device=gpu).manual_seed(m)
+    x = torch.randn((n3, n2, m), generator=g, device=gpu) * torch.logspace(0, -2, m, device=gpu)
+    a = x.reshape(-1, m)
+    lam = sum(p.double().t() @ p.double() for p in a.split(1 << 20))
+    want = torch.linalg.eigvalsh(lam).flip(0).cpu().numpy()
+    got = np.asarray(_ttr().tt_svd(x.permute(2, 1, 0), [1, 4, 4, 1], gemm="fp32").sigmas[0][:m]) ** 2
+    assert np.abs(got - want).max() <= 65 * U32 * want.sum()
+
+
 @pytest.mark.parametrize("m,n,N", [(600, 200000, 96), (256, 600000, 80), (4096, 37000, 64), (600, 200000, 24),
                                    (130, 600000, 128)])
 def test_sketch_fp32_chain_length(gpu, m, n, N):
