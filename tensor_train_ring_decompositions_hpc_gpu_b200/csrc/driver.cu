@@ -241,11 +241,17 @@ struct Plan {
   std::vector<int> r;
   std::vector<Step> steps;
   long long total = 0;
-  size_t max_data = 0, max_omega = 0, max_y = 0, max_y0 = 0, max_bt = 0, max_core = 0, max_ws = 0;
+  size_t max_data = 0, max_omega = 0, max_y = 0, max_y0 = 0, max_bt = 0, max_core = 0;
+  size_t max_ws = 0, least_ws = 0;  // scratch of the steps: wanted, and what they can do with (reserve_between)
   size_t max_ef = (size_t)TT_MAX_SMALL * TT_MAX_SMALL;  // FP32 basis (m x r or ks x r)
   int max_small = 0;
   int last_rows = 1;  // rows per mode index of the data left for the last core
   long long stream_cols = 0;  // host streaming: columns of the first unfolding per chunk (0: off)
+  void need(size_t most, size_t least) {
+    max_ws = std::max(max_ws, most);
+    least_ws = std::max(least_ws, least);
+  }
+  void need(size_t bytes) { need(bytes, bytes); }
 };
 
 // An exact step whose Gram comes from the tensor cores (more than 32 rows) and that truncates
@@ -370,9 +376,9 @@ int make_plan(int d, const int* n, const int* r, bool ring, const tt_opts& o, Pl
       const int b = refine_width(st);
       P.max_y = std::max<size_t>(P.max_y, (size_t)st.m * b);
       P.max_bt = std::max<size_t>(P.max_bt, (size_t)st.cols * b);
-      P.max_ws = std::max(P.max_ws, project_ws_bytes(st.m, st.cols, b));
-      P.max_ws = std::max(P.max_ws, project_ws_bytes(b, st.cols, st.r_req));
-      P.max_ws = std::max(P.max_ws, gram_ws_bytes(st.cols, b));
+      P.need(project_ws_bytes(st.m, st.cols, b), project_ws_least(st.m, st.cols, b));
+      P.need(project_ws_bytes(b, st.cols, st.r_req), project_ws_least(b, st.cols, st.r_req));
+      P.need(gram_ws_bytes(st.cols, b));
     }
     P.max_core = std::max<size_t>(P.max_core, (size_t)st.m * std::max(st.r_req, st.ks));
     P.max_ef = std::max<size_t>(P.max_ef, (size_t)std::max<long long>(st.m, st.ks) * st.r_req);
@@ -385,25 +391,26 @@ int make_plan(int d, const int* n, const int* r, bool ring, const tt_opts& o, Pl
       // the adaptive modes run narrower sketches (and the probe) within the same buffers
       const bool narrow = (o.flags & (TT_FLAG_ADAPTIVE_KS | TT_FLAG_LEARNED)) != 0;
       for (int w = narrow ? 1 : st.ks; w <= st.ks; ++w) {
-        P.max_ws = std::max(P.max_ws, sketch_ws_bytes(st.m, st.cols, w));
-        P.max_ws = std::max(P.max_ws, gram_ws_bytes(st.cols, w));
-        P.max_ws = std::max(P.max_ws, gram_ws_bytes(st.m, w));
-        P.max_ws = std::max(P.max_ws, gram_tc_ws_bytes(w, st.cols));
-        P.max_ws = std::max(P.max_ws, gram32x_ws_bytes());
-        P.max_ws = std::max(P.max_ws, project_ws_bytes(st.m, st.cols, w));
-        P.max_ws = std::max(P.max_ws, project_ws_bytes(w, st.cols, std::min(w, st.r_req)));
+        P.need(sketch_ws_bytes(st.m, st.cols, w), sketch_ws_least(st.m, st.cols, w));
+        P.need(gram_ws_bytes(st.cols, w));
+        P.need(gram_ws_bytes(st.m, w));
+        P.need(gram_tc_ws_bytes(w, st.cols));
+        P.need(gram32x_ws_bytes());
+        P.need(project_ws_bytes(st.m, st.cols, w), project_ws_least(st.m, st.cols, w));
+        P.need(project_ws_bytes(w, st.cols, std::min(w, st.r_req)), project_ws_least(w, st.cols, std::min(w, st.r_req)));
       }
-      P.max_ws = std::max(P.max_ws, project_ws_bytes(st.ks, st.cols, st.r_req));
-      P.max_ws = std::max(P.max_ws, syev_ws_bytes(st.ks, o.max_sweeps));
+      P.need(project_ws_bytes(st.ks, st.cols, st.r_req), project_ws_least(st.ks, st.cols, st.r_req));
+      P.need(syev_ws_bytes(st.ks, o.max_sweeps));
     } else {
-      P.max_ws = std::max(P.max_ws, project_ws_bytes(st.m, st.cols, st.r_req));
-      P.max_ws = std::max(P.max_ws, gram_ws_bytes(std::max(st.m, st.cols), (int)mn));
-      P.max_ws = std::max(P.max_ws, gram_tc_ws_bytes(st.m, st.cols));
-      P.max_ws = std::max(P.max_ws, gram32x_ws_bytes());
-      P.max_ws = std::max(P.max_ws, syev_ws_bytes((int)mn, o.max_sweeps));
+      P.need(project_ws_bytes(st.m, st.cols, st.r_req), project_ws_least(st.m, st.cols, st.r_req));
+      P.need(gram_ws_bytes(std::max(st.m, st.cols), (int)mn));
+      P.need(gram_tc_ws_bytes(st.m, st.cols));
+      P.need(gram32x_ws_bytes());
+      P.need(syev_ws_bytes((int)mn, o.max_sweeps));
     }
   }
   P.max_ws += (size_t)TT_MAX_SMALL * TT_MAX_SMALL * sizeof(double) * 8;
+  P.least_ws += (size_t)TT_MAX_SMALL * TT_MAX_SMALL * sizeof(double) * 8;
   return TT_OK;
 }
 
@@ -435,7 +442,7 @@ struct Bufs {
   float* ef2 = nullptr;
 };
 
-size_t plan_bytes(const Plan& P, bool host_io) {
+size_t plan_bytes(const Plan& P, bool host_io, size_t ws) {
   const size_t S = TT_MAX_SMALL;
   size_t b = 0;
   auto add = [&](size_t bytes) { b += (bytes + 255) & ~size_t(255); };
@@ -462,8 +469,15 @@ size_t plan_bytes(const Plan& P, bool host_io) {
   add(P.max_ef * sizeof(float));
   if (host_io)
     for (int k = 0; k < P.d; ++k) add(core_elems(P, k) * sizeof(float));
-  add(P.max_ws);
+  add(ws);
   return b + (1 << 20);
+}
+
+// Reserves `most` bytes, or all that the context's allocation limit leaves where that is at least `least`: sketches
+// and projections then take fewer splits of their long side.
+int reserve_between(tt_ctx* c, size_t most, size_t least) {
+  if (c->alloc_limit && most > c->alloc_limit && least <= c->alloc_limit) most = c->alloc_limit;
+  return tt_ctx_reserve(c, most);
 }
 
 int carve(tt_ctx* c, const Plan& P, bool host_io, Bufs& B, Arena& ws) {
@@ -610,7 +624,7 @@ int run_chain(tt_ctx* c, const float* x_in, Plan P, const tt_opts& o, float* con
   TT_CUDA(cudaSetDevice(c->device));
   // a side-stream job of an earlier call that failed midway must not outlive its buffers
   if (c->side_stream) TT_CUDA(cudaStreamSynchronize(c->side_stream));
-  TT_TRY(tt_ctx_reserve(c, plan_bytes(P, host_io)));
+  TT_TRY(reserve_between(c, plan_bytes(P, host_io, P.max_ws), plan_bytes(P, host_io, P.least_ws)));
   Bufs B;
   Arena ws;
   TT_TRY(carve(c, P, host_io, B, ws));
@@ -1334,10 +1348,10 @@ int run_entry(tt_ctx* c, const float* x, int d, const int* n, const int* r, cons
     }
     P.stream_cols = std::max<long long>(1, std::min<long long>(s0.cols, (long long)(c->chunk_bytes / (4 * s0.m))));
     // the Gram and projection kernels see one chunk at a time
-    P.max_ws = std::max(P.max_ws, gram_ws_bytes(P.stream_cols, (int)s0.m));
-    P.max_ws = std::max(P.max_ws, gram_tc_ws_bytes(s0.m, P.stream_cols));
-    P.max_ws = std::max(P.max_ws, gram32x_ws_bytes());
-    P.max_ws = std::max(P.max_ws, project_ws_bytes(s0.m, P.stream_cols, s0.r_req));
+    P.need(gram_ws_bytes(P.stream_cols, (int)s0.m));
+    P.need(gram_tc_ws_bytes(s0.m, P.stream_cols));
+    P.need(gram32x_ws_bytes());
+    P.need(project_ws_bytes(s0.m, P.stream_cols, s0.r_req), project_ws_least(s0.m, P.stream_cols, s0.r_req));
   }
   for (int k = 0; k < d; ++k)
     if (!cores[k]) {
@@ -1468,8 +1482,8 @@ extern "C" int tt_rel_error(tt_ctx* c, const float* x, int d, const int* n, cons
 
 // ---- building blocks ----
 namespace {
-int ws_for(tt_ctx* c, size_t bytes, Arena& ws) {
-  TT_TRY(tt_ctx_reserve(c, bytes + (1 << 20)));
+int ws_for(tt_ctx* c, size_t bytes, Arena& ws, size_t least = 0) {
+  TT_TRY(reserve_between(c, bytes + (1 << 20), (least ? least : bytes) + (1 << 20)));
   ws = Arena{c->arena, c->cap, 0};
   return TT_OK;
 }
@@ -1555,7 +1569,7 @@ extern "C" int tt_k_sketch(tt_ctx* c, const float* a, long long m, long long n, 
   }
   TT_CUDA(cudaSetDevice(c->device));
   Arena ws;
-  TT_TRY(ws_for(c, sketch_ws_bytes(m, n, N) * 2, ws));
+  TT_TRY(ws_for(c, sketch_ws_bytes(m, n, N) * 2, ws, sketch_ws_least(m, n, N)));
   const int eng = (gemm == TT_GEMM_FP32 || !tc_available()) ? TT_GEMM_FP32 : TT_GEMM_TC;
   TT_CUDA(cudaMemsetAsync(c->dstat, 0, sizeof(DevStatus), c->stream));
   TT_TRY(launch_sketch(a, m, n, w, N, 1, ldw, y, eng, ws, c->dstat, c->stream));
@@ -1590,10 +1604,10 @@ extern "C" int tt_probe_features(tt_ctx* c, const float* a, long long m, long lo
   tt_default_opts(&o);
   const int engine = engine_for(o, m, n);
   const size_t bytes = sizeof(float) * (size_t)n * P + sizeof(double) * (size_t)m * P + sizeof(float) * (size_t)m * P +
-                       sizeof(double) * (2 * P * P + P + 2) + sketch_ws_bytes(m, n, P) + gram_ws_bytes(m, P) +
+                       sizeof(double) * (2 * P * P + P + 2) + gram_ws_bytes(m, P) +
                        (size_t)TT_MAX_SMALL * TT_MAX_SMALL * sizeof(double) * 8 + 16 * 4096;
   Arena ws;
-  TT_TRY(ws_for(c, bytes, ws));
+  TT_TRY(ws_for(c, bytes + sketch_ws_bytes(m, n, P), ws, bytes + sketch_ws_least(m, n, P)));
   float* om = ws.take<float>((size_t)n * P);
   double* yd = ws.take<double>((size_t)m * P);
   float* yf = ws.take<float>((size_t)m * P);
@@ -1687,7 +1701,8 @@ extern "C" int tt_k_project(tt_ctx* c, const float* a, long long m, long long n,
   }
   TT_CUDA(cudaSetDevice(c->device));
   Arena ws;
-  TT_TRY(ws_for(c, std::max<size_t>(1 << 20, project_ws_bytes(m, n, N)), ws));
+  TT_TRY(ws_for(c, std::max<size_t>(1 << 20, project_ws_bytes(m, n, N)), ws,
+                std::max<size_t>(1 << 20, project_ws_least(m, n, N))));
   const int eng = (gemm == TT_GEMM_FP32 || !tc_available()) ? TT_GEMM_FP32 : TT_GEMM_TC;
   TT_CUDA(cudaMemsetAsync(c->dstat, 0, sizeof(DevStatus), c->stream));
   TT_TRY(launch_project(a, m, n, q, N, ldq, out, ldo, OUT_ROWMAJOR, 1, 1, eng, ws, c->dstat, c->stream));

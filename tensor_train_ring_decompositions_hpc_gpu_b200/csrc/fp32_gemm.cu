@@ -203,12 +203,15 @@ int sk_width(int N, int* blocks) {
 // often than twice where a warp's FP32 chain, an eighth of a split, would be longer than that of splits that fill
 // the SMs four times with blocks of 256 rows (and 256 columns): sketches above 64 columns, which take two blocks of
 // columns (600 x 950k, 96 columns: chains of 8,488 -> 4,096 columns in the same 2.5 ms).
+long long sketch_chain(long long m, long long n) {
+  return std::max(256LL, ceil_div_ll(n, std::max(1LL, 4LL * dev_sms() / ceil_div_ll(m, 256))));
+}
 void sketch_split_plan(long long m, long long n, int N, long long* jchunk, int* nsplit) {
   int cb;
   const int NT = sk_width(N, &cb);
   const long long tiles = ceil_div_ll(m, SK_ROWS) * cb;
   constexpr long long unit = SK_W * SK_JC;
-  const long long chain = std::max(256LL, ceil_div_ll(n, std::max(1LL, 4LL * dev_sms() / ceil_div_ll(m, 256))));
+  const long long chain = sketch_chain(m, n);
   long long jc = unit;
   for (int waves = 2;; ++waves) {
     const long long splits = std::max<long long>(1, (long long)waves * sk_blocks(NT) * dev_sms() / tiles);
@@ -590,6 +593,13 @@ int project_ksplit(long long m, long long n, int N, long long* kchunk) {
   return (int)ceil_div_ll(m, kc);
 }
 
+// Lowers the split count to `fit` where it is above.
+int project_split_fit(long long m, long long fit, int ks, long long* kchunk) {
+  if (ks <= fit) return ks;
+  *kchunk = ceil_div_ll(ceil_div_ll(m, std::max(1LL, fit)), PJ_KC) * PJ_KC;
+  return (int)ceil_div_ll(m, *kchunk);
+}
+
 template <int RC>
 int run_project32(const float* a, long long m, long long n, const float* q, int N, long long ldq, float* out,
                   long long ldo, int mode, int r0, int r1, int cb, int ks, long long kc, cudaStream_t s) {
@@ -609,6 +619,12 @@ size_t sketch_ws_bytes(long long m, long long n, int N) {
   sketch_split_plan(m, n, N, &jchunk, &nsplit);
   const size_t simt = (size_t)nsplit * (size_t)N * (size_t)m * sizeof(double) + 4096;
   return std::max(simt, sketch_tc_ws_bytes(m, n, N));
+}
+
+size_t sketch_ws_least(long long m, long long n, int N) {
+  const long long jc = ceil_div_ll(sketch_chain(m, n), 32) * 32;
+  const size_t simt = (size_t)ceil_div_ll(n, jc) * (size_t)N * (size_t)m * sizeof(double) + 4096;
+  return std::min(sketch_ws_bytes(m, n, N), std::max(simt, sketch_tc_ws_bytes(m, n, N)));
 }
 
 int launch_reduce_splits(const double* part, long long count, int nsplit, double* y, cudaStream_t s) {
@@ -669,6 +685,17 @@ size_t project_ws_bytes(long long m, long long n, int N) {
   return split + 2 * (size_t)m * N * sizeof(float) + 4096;
 }
 
+size_t project_ws_least(long long m, long long n, int N) {
+  const int nt = N <= 16 ? 16 : N <= 32 ? 32 : N <= 48 ? 48 : 64;
+  const long long blocks = ceil_div_ll(n, 256) * ceil_div(N, nt);
+  long long kc, least = 1;
+  int ks = project_ksplit(m, n, N, &kc);
+  if (m >= 256 && blocks < 2LL * dev_sms()) least = std::min(ceil_div_ll(2LL * dev_sms(), blocks), m / 64);
+  ks = project_split_fit(m, least, ks, &kc);
+  const size_t split = ks > 1 ? (size_t)ks * n * N * sizeof(float) : 0;
+  return split + 2 * (size_t)m * N * sizeof(float) + 4096;
+}
+
 int launch_project(const float* a, long long m, long long n, const float* q, int N, long long ldq,
                    float* out, long long ldo, int mode, int r0, int r1, int engine, Arena& ws,
                    DevStatus* st, cudaStream_t s) {
@@ -682,6 +709,8 @@ int launch_project(const float* a, long long m, long long n, const float* q, int
   int ks = project_ksplit(m, n, N, &kc);
   float* part = nullptr;
   const size_t mk = ws.mark();
+  const size_t left = (ws.cap - std::min(ws.cap, (mk + 255) & ~size_t(255))) & ~size_t(255);
+  ks = project_split_fit(m, (long long)(left / (sizeof(float) * (size_t)n * N)), ks, &kc);
   if (ks > 1) part = ws.take<float>((size_t)ks * n * N);
   if (!part) {
     ks = 1;

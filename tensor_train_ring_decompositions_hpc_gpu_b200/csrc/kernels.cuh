@@ -25,6 +25,10 @@ struct Arena {
 size_t sketch_ws_bytes(long long m, long long n, int N);
 size_t gram_ws_bytes(long long nvec, int M);
 size_t project_ws_bytes(long long m, long long n, int N);
+// What they can do with: fewer splits, FP32 chains as long as those of splits that fill the SMs four times with
+// blocks of 256 rows (sketch) or twice with blocks of 256 columns (projection).
+size_t sketch_ws_least(long long m, long long n, int N);
+size_t project_ws_least(long long m, long long n, int N);
 
 // Philox Gaussian fill (column-major rows x cols, ld).
 int launch_gaussian(float* out, long long rows, int cols, long long ld, unsigned long long seed,

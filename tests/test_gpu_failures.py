@@ -117,3 +117,38 @@ def test_tolerance_run_at_its_allocation_limit(gpu, monkeypatch):
     assert ttr.lib().tt_ctx_set_alloc_limit(ttr._ctx_for(0), high) == 0
     res = ttr.tt_svd(x, [1, 17, 24, 1], eps=1e-3, gemm="fp32")
     assert res.ranks == [1, 16, 12, 1]
+
+
+@pytest.mark.parametrize("call", ["tt", "tr", "eps", "sketch", "project"])
+def test_fewer_splits_under_an_allocation_limit(gpu, monkeypatch, call):
+    """Sketches and projections split their long side for speed.  Limits between the scratch of all these splits and
+    that of fewer: the call runs, and to the same result."""
+    import torch
+    ttr = _ttr()
+    g = torch.Generator(device=gpu).manual_seed(3)
+    def rand(*shape):
+        return torch.randn(*shape, generator=g, device=gpu)
+    if call in ("sketch", "project"):
+        m, n, N, limit = (50, 9469, 111, 7_650_000) if call == "sketch" else (225, 21602, 53, 2_100_000)
+        a, w = rand(n, m).t(), rand(N, n if call == "sketch" else m).t()
+        def run():
+            return [getattr(ttr, call)(a, w, "fp32")]
+    else:
+        n, limit = {"tt": ((137, 110, 312), 20_100_000), "tr": ((140, 153, 251), 13_700_000),
+                    "eps": ((144, 303, 132), 18_050_000)}[call]
+        x = torch.einsum("ir,rjs,sk->kji", rand(n[0], 5), rand(5, n[1], 5), rand(5, n[2])).permute(2, 1, 0)
+        x = x + 1e-4 * rand(n[2], n[1], n[0]).permute(2, 1, 0)
+        def run():
+            if call == "tr":
+                res = ttr.tr_svd(x, [1, 1, 1, 1], gemm="fp32", power_iters=1, oversample=20)
+            elif call == "tt":
+                res = ttr.tt_svd(x, [1, 17, 17, 1], gemm="fp32", power_iters=1)
+            else:
+                res = ttr.tt_svd(x, [1, 5, 5, 1], eps=1e-2, oversample=20)
+            return [torch.as_tensor(np.asarray(s)[:r]) for s, r in zip(res.sigmas, res.ranks[1:])]
+    monkeypatch.setattr(ttr, "_CTX", {})
+    want = run()
+    monkeypatch.setattr(ttr, "_CTX", {})
+    assert ttr.lib().tt_ctx_set_alloc_limit(ttr._ctx_for(0), limit) == 0
+    for u, v in zip(want, run()):  # FP32 sums in another order
+        assert float((u - v).abs().max()) <= 1e-5 * float(u.abs().max())
