@@ -247,11 +247,21 @@ struct Plan {
   int max_small = 0;
   int last_rows = 1;  // rows per mode index of the data left for the last core
   long long stream_cols = 0;  // host streaming: columns of the first unfolding per chunk (0: off)
-  void need(size_t most, size_t least) {
-    max_ws = std::max(max_ws, most);
-    least_ws = std::max(least_ws, least);
+  bool limited = false;  // least_ws is wanted too (it costs as much as the rest of the plan); else it is max_ws
+  void need(size_t bytes) {
+    max_ws = std::max(max_ws, bytes);
+    least_ws = std::max(least_ws, bytes);
   }
-  void need(size_t bytes) { need(bytes, bytes); }
+  void need_sketch(long long m, long long n, int N) {
+    const size_t most = sketch_ws_bytes(m, n, N);
+    max_ws = std::max(max_ws, most);
+    least_ws = std::max(least_ws, limited ? sketch_ws_least(m, n, N) : most);
+  }
+  void need_project(long long m, long long n, int N) {
+    const size_t most = project_ws_bytes(m, n, N);
+    max_ws = std::max(max_ws, most);
+    least_ws = std::max(least_ws, limited ? project_ws_least(m, n, N) : most);
+  }
 };
 
 // An exact step whose Gram comes from the tensor cores (more than 32 rows) and that truncates
@@ -376,8 +386,8 @@ int make_plan(int d, const int* n, const int* r, bool ring, const tt_opts& o, Pl
       const int b = refine_width(st);
       P.max_y = std::max<size_t>(P.max_y, (size_t)st.m * b);
       P.max_bt = std::max<size_t>(P.max_bt, (size_t)st.cols * b);
-      P.need(project_ws_bytes(st.m, st.cols, b), project_ws_least(st.m, st.cols, b));
-      P.need(project_ws_bytes(b, st.cols, st.r_req), project_ws_least(b, st.cols, st.r_req));
+      P.need_project(st.m, st.cols, b);
+      P.need_project(b, st.cols, st.r_req);
       P.need(gram_ws_bytes(st.cols, b));
     }
     P.max_core = std::max<size_t>(P.max_core, (size_t)st.m * std::max(st.r_req, st.ks));
@@ -391,18 +401,18 @@ int make_plan(int d, const int* n, const int* r, bool ring, const tt_opts& o, Pl
       // the adaptive modes run narrower sketches (and the probe) within the same buffers
       const bool narrow = (o.flags & (TT_FLAG_ADAPTIVE_KS | TT_FLAG_LEARNED)) != 0;
       for (int w = narrow ? 1 : st.ks; w <= st.ks; ++w) {
-        P.need(sketch_ws_bytes(st.m, st.cols, w), sketch_ws_least(st.m, st.cols, w));
+        P.need_sketch(st.m, st.cols, w);
         P.need(gram_ws_bytes(st.cols, w));
         P.need(gram_ws_bytes(st.m, w));
         P.need(gram_tc_ws_bytes(w, st.cols));
         P.need(gram32x_ws_bytes());
-        P.need(project_ws_bytes(st.m, st.cols, w), project_ws_least(st.m, st.cols, w));
-        P.need(project_ws_bytes(w, st.cols, std::min(w, st.r_req)), project_ws_least(w, st.cols, std::min(w, st.r_req)));
+        P.need_project(st.m, st.cols, w);
+        P.need_project(w, st.cols, std::min(w, st.r_req));
       }
-      P.need(project_ws_bytes(st.ks, st.cols, st.r_req), project_ws_least(st.ks, st.cols, st.r_req));
+      P.need_project(st.ks, st.cols, st.r_req);
       P.need(syev_ws_bytes(st.ks, o.max_sweeps));
     } else {
-      P.need(project_ws_bytes(st.m, st.cols, st.r_req), project_ws_least(st.m, st.cols, st.r_req));
+      P.need_project(st.m, st.cols, st.r_req);
       P.need(gram_ws_bytes(std::max(st.m, st.cols), (int)mn));
       P.need(gram_tc_ws_bytes(st.m, st.cols));
       P.need(gram32x_ws_bytes());
@@ -1338,6 +1348,7 @@ int run_entry(tt_ctx* c, const float* x, int d, const int* n, const int* r, cons
     o.flags |= TT_FLAG_NO_FOLD;
   }
   Plan P;
+  P.limited = c->alloc_limit != 0;
   TT_TRY(make_plan(d, n, r, ring, o, P));
   if (o.flags & TT_FLAG_HOST_STREAM) {
     const Step& s0 = P.steps[0];
@@ -1351,7 +1362,7 @@ int run_entry(tt_ctx* c, const float* x, int d, const int* n, const int* r, cons
     P.need(gram_ws_bytes(P.stream_cols, (int)s0.m));
     P.need(gram_tc_ws_bytes(s0.m, P.stream_cols));
     P.need(gram32x_ws_bytes());
-    P.need(project_ws_bytes(s0.m, P.stream_cols, s0.r_req), project_ws_least(s0.m, P.stream_cols, s0.r_req));
+    P.need_project(s0.m, P.stream_cols, s0.r_req);
   }
   for (int k = 0; k < d; ++k)
     if (!cores[k]) {
