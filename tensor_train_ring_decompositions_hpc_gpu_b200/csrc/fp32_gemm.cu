@@ -8,6 +8,7 @@
 // unfolding.  576 x 331776 at 32 columns (floor 164 us of FMAs): sketch 328 us, projection 330.  Sketches of
 // 600 x 950k: 565 us at 16 columns, 2480 at 96 (59 % of the FMA rate).  384 x 320: 6 us each.
 #include <algorithm>
+#include <type_traits>
 
 #include "kernels.cuh"
 
@@ -288,17 +289,23 @@ __global__ void __launch_bounds__(PJ_T) k_project32(const float* __restrict__ a,
   const bool va = (m & 3) == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0;
   const bool vq = (ldq & 3) == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0;
   // chunk of 32 k: rows of A and Q into rows of PJ_LD floats, zero past the ends.  The aligned copy of a
-  // thread is k 4 (tid & 7) .. + 3 of rows tid / 8 + 16 u: addresses are set up once.
+  // thread is k 4 (tid & 7) .. + 3 of rows tid / 8 + 16 u, the other one (m no multiple of 4, the last chunk) k
+  // tid & 31 of rows tid / 32 + 4 u: addresses are set up once (97 x 700k, 24 outputs: 243 us with an index
+  // calculation per copy, 170 so).
   const int cr = tid >> 3, ck = 4 * (tid & 7);
   const float* const asrc = a + (j0 + cr) * m + kb + ck;
   const float* const qsrc = q + (c0 + cr) * ldq + kb + ck;
   const long long astep = 16 * m, qstep = 16 * ldq;
   const int arows = (int)min((long long)PJ_T, n - j0) - cr, qrows = N - c0 - cr;  // rows left for this thread
-  auto copy4 = [&](float* dst, const float* src, long long ld, long long row0, long long rows, int count, long long k0) {
-    for (int f = tid; f < count * PJ_KC; f += PJ_T) {
-      const int r = f >> 5, k = f & 31;
-      const bool ok = row0 + r < rows && k0 + k < ke;
-      cp_async4(dst + r * PJ_LD + k, ok ? src + ld * (row0 + r) + k0 + k : src, ok);
+  const float* const asrc1 = a + (j0 + warp) * m + kb + lane;
+  const float* const qsrc1 = q + (c0 + warp) * ldq + kb + lane;
+  const int arows1 = (int)min((long long)PJ_T, n - j0) - warp, qrows1 = N - c0 - warp;
+  auto copy1 = [&](auto count, float* dst, const float* src, long long step, int rows, const float* safe) {
+#pragma unroll 16
+    for (int u = 0; u < decltype(count)::value / 4; ++u) {
+      const bool ok = 4 * u < rows;
+      cp_async4(dst + 4 * u * PJ_LD, ok ? src : safe, ok);
+      src += step;
     }
   };
   auto load = [&](int ch) {
@@ -315,7 +322,8 @@ __global__ void __launch_bounds__(PJ_T) k_project32(const float* __restrict__ a,
           src += astep;
         }
       } else {
-        copy4(as, a, m, j0, n, PJ_T, k0);
+        copy1(std::integral_constant<int, PJ_T>{}, as + warp * PJ_LD + lane, asrc1 + ch * PJ_KC, 4 * m,
+              k0 + lane < ke ? arows1 : 0, a);
       }
       if (vq && whole) {
         const float* src = qsrc + ch * PJ_KC;
@@ -326,7 +334,8 @@ __global__ void __launch_bounds__(PJ_T) k_project32(const float* __restrict__ a,
           src += qstep;
         }
       } else {
-        copy4(as + PJ_T * PJ_LD, q, ldq, c0, N, NT, k0);
+        copy1(std::integral_constant<int, NT>{}, as + (PJ_T + warp) * PJ_LD + lane, qsrc1 + ch * PJ_KC, 4 * ldq,
+              k0 + lane < ke ? qrows1 : 0, q);
       }
     }
     cp_async_commit();
