@@ -490,6 +490,10 @@ __global__ void k_mul_upper(const double* __restrict__ r2, const double* __restr
   r[idx] = (j >= i) ? acc : 0.0;
 }
 
+// Rows up to which the eight SMs of a cluster are as fast as the whole GPU in seven launches.  One launch against
+// several, us: 7,000 x 2 61 / 63, 10,000 x 2 72 / 63, 100,000 x 2 334 / 62; 7,000 x 16 87 / 75, 15,000 x 16 123 / 75;
+// 15,000 x 24 144 / 87.
+constexpr long long kCqRows = 8192;
 constexpr double kCqTol = 1e-12;  // pivots below this share of the largest diagonal: dependent columns
 
 // The pass Y <- Y R^-1 of the Gram w, R^-1 through `tf` (N rows of stride RS), R to r (or null).
@@ -525,13 +529,17 @@ int cholqr_passes(const double* y64, float* y, long long n, int N, long long ld,
     set_error(TT_ERR_NOMEM, "cholqr2 workspace");
     return TT_ERR_NOMEM;
   }
-  // One launch whenever the rows fit the shared memory of 8 CTAs (at N = 40 1,130 rows each, 9,000 in all):
+  // One launch up to kCqRows rows whenever they fit the shared memory of 8 CTAs (at N = 40 1,130 rows each, 9,000 in all):
   // CTAs of at least 64 rows, as few as fit.
   if (n <= (1LL << 20)) {
     for (int cl = (int)std::min<long long>(8, ceil_div_ll(n, 64)); cl <= 8; ++cl) {
       const int rpc = (int)ceil_div_ll(n, cl);
       const CqSmem lay = cq_smem(n, N, rpc, cl);
       if (lay.total > (size_t)dev_smem_max()) continue;
+      if (n > kCqRows) {
+        passes = 2;  // as in one launch
+        break;
+      }
       TT_TRY(smem_optin_k(k_cholqr_cluster<4>, dev_smem_max()));
       TT_TRY(smem_optin_k(k_cholqr_cluster<8>, dev_smem_max()));
       cudaLaunchConfig_t cfg = {};

@@ -68,6 +68,12 @@ def test_cholqr2_tall_ragged(gpu, n, N):
     assert float(torch.linalg.norm(qd @ r - yd)) <= tol * float(torch.linalg.norm(yd))
 
 
+@pytest.mark.parametrize("n,N", [(8192, 1), (8193, 1), (8192, 12), (8193, 12), (16411, 2), (12001, 40)])
+def test_cholqr2_around_the_rows_of_one_launch(gpu, n, N):
+    """Both sides of the row count above which several launches are taken although one would hold the rows."""
+    test_cholqr2_tall_ragged(gpu, n, N)
+
+
 @pytest.mark.parametrize("n,N", [(256, 65), (400, 72), (300, 77), (462, 80)])
 def test_cholqr2_wide_rows_are_solved(gpu, n, N):
     """65 to 80 columns of few rows: q R = y is solved row by row, like the narrower ones, and not multiplied by an
