@@ -21,7 +21,7 @@
 //    The second pass then finds R = I to 1e-9 and has nothing to round.  256^3, ranks 16: 680 us (678 without).
 // CholeskyQR2 of 384 x 24: 32 us; 1024 x 40: 49; 256 x 80: 118; 640 x 96: 187.  What is left is the chain: at
 // 1024 x 40, per pass, 14k cycles of Cholesky, 8.5k of Gram, 6k for the cluster's sum, 6k of row solves.
-// Small matrices take one launch, a cluster of up to 8 CTAs (launch_cholqr2 below has the rule).
+// Small matrices take one launch, a cluster of up to 8 CTAs (kCqRows and cholqr_passes below have the rule).
 #include <algorithm>
 
 #include "chol.cuh"
@@ -529,8 +529,8 @@ int cholqr_passes(const double* y64, float* y, long long n, int N, long long ld,
     set_error(TT_ERR_NOMEM, "cholqr2 workspace");
     return TT_ERR_NOMEM;
   }
-  // One launch up to kCqRows rows whenever they fit the shared memory of 8 CTAs (at N = 40 1,130 rows each, 9,000 in all):
-  // CTAs of at least 64 rows, as few as fit.
+  // One launch up to kCqRows rows where they fit the shared memory of 8 CTAs (at N = 40 1,130 rows each): CTAs of
+  // at least 64 rows, as few as fit.
   if (n <= (1LL << 20)) {
     for (int cl = (int)std::min<long long>(8, ceil_div_ll(n, 64)); cl <= 8; ++cl) {
       const int rpc = (int)ceil_div_ll(n, cl);
